@@ -375,8 +375,8 @@ class Graph:
 
     def set_clean_split(self, min_seeds: int, max_mean_list: float = 8.0):
         """Clean units with at least `min_seeds` seeds and triangle lists of at
-        most `max_mean_list` entries on average replay in parallel rounds (one
-        thread block each), the others one warp per unit (same bits)."""
+        most `max_mean_list` entries on average replay a window of pops at a
+        time (one thread block each), the others one warp per unit (same bits)."""
         _check(lib().rtr_set_clean_split(self._h, int(min_seeds), float(max_mean_list)))
 
     def nucleus(self) -> int:

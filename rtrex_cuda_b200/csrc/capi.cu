@@ -348,6 +348,7 @@ int rtr_graph_destroy(rtr_graph* g)
         if (g->kev[k]) cudaEventDestroy(g->kev[k]);
     if (g->own_stream && g->stream) cudaStreamDestroy(g->stream);
     if (g->side) cudaStreamDestroy(g->side);
+    if (g->side2) cudaStreamDestroy(g->side2);
     delete[] g->batch_vbase;
     delete g;
     return RTR_OK;
@@ -417,6 +418,7 @@ int rtr_set_clean_split(rtr_graph* g, int64_t min_seeds, double max_mean_list)
     }
     g->clean_round_min = min_seeds;
     g->clean_round_list = max_mean_list;
+    g->clean_auto = false;
     return RTR_OK;
 }
 

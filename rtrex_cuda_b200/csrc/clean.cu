@@ -201,26 +201,60 @@ __global__ void k_unit_desc(const uint64_t* __restrict__ keys, int64_t ns, int r
     }
 }
 
-// Unit bounds and the schedule: the units replayed in parallel rounds (many
-// seeds, short lists: those are where disjoint pops are common) first, then
-// the others; within each group the units with the most seeds first.
-__global__ void k_unit_finish(UnitDesc* __restrict__ units, const int64_t* __restrict__ cap,
-                              const int64_t* __restrict__ capoff, int64_t nu, int64_t ns,
-                              const uint32_t* __restrict__ ecount, const unsigned long long* __restrict__ tsum,
-                              int64_t round_min, double round_max_list, uint64_t* __restrict__ order_keys,
-                              unsigned* __restrict__ nbig, int64_t stack_limit)
+// How a unit is replayed.
+enum UnitClass : uint32_t { UNIT_WIDE = 0, UNIT_NARROW = 1, UNIT_WARP = 2 };
+
+struct UnitRule {
+    int64_t min_seeds;  // window replay from this many seeds ...
+    double max_list;    // ... and up to this mean triangle-list length
+    double wide_list;   // mean list length above which a window's lists are packed
+};
+// Without a rule from the caller (rtr_set_clean_split), units of at least 512
+// seeds take the window replay, of any list length: on 14 graphs of 1,000 to
+// 926,000 edges (G(n,p) with cliques, SBM, Chung-Lu, R-MAT, e-mail and
+// co-authorship networks, eps 0.3 and 0.1) it took 0.45 to 0.96 of the warp
+// replay's time from there on (0.57 against 1.10 ms on a 10,000-edge
+// Chung-Lu graph, 97 against 132 ms on the e-mail network); below it the log's
+// fold costs what the replay gains (0.40 against 0.32 ms, a 5,000-edge SBM).
+constexpr int64_t kAutoSeeds = 512;
+// Up to a mean list of 8 entries a window is 16 items of 16 threads each, above
+// it 8 items packed into 256 threads: 15.4 against 20.4 ms on the co-purchase
+// graph (mean list 3), 150 against 116 ms on the 203,311-edge R-MAT (mean 31).
+constexpr double kNarrowList = 8.0;
+
+// Unit bounds and classes, and the triangles of the window-replayed units.
+__global__ void k_unit_class(UnitDesc* __restrict__ units, int64_t nu, int64_t ns, const uint32_t* __restrict__ ecount,
+                             const unsigned long long* __restrict__ tsum, UnitRule rule, uint32_t* __restrict__ cls,
+                             unsigned long long* __restrict__ ntri, unsigned* __restrict__ ncls)
 {
     for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < nu; u += (int64_t)gridDim.x * blockDim.x) {
-        units[u].seed_end = (u + 1 < nu) ? units[u + 1].seed_begin : ns;
+        const int64_t end = (u + 1 < nu) ? units[u + 1].seed_begin : ns;
+        units[u].seed_end = end;
+        const int64_t r = units[u].root;
+        const double lists = (double)tsum[r], edges = (double)ecount[r];
+        const bool rounds = end - units[u].seed_begin >= rule.min_seeds && lists <= rule.max_list * edges;
+        const uint32_t c = !rounds ? UNIT_WARP : lists > rule.wide_list * edges ? UNIT_WIDE : UNIT_NARROW;
+        cls[u] = c;
+        if (rounds) {
+            atomicAdd(&ncls[c], 1u);
+            atomicAdd(ntri, tsum[r] / 3);  // each triangle is in three edges' lists
+        }
+    }
+}
+
+// The schedule: the units' classes in turn, within each the units with the
+// most seeds first.
+__global__ void k_unit_finish(UnitDesc* __restrict__ units, const int64_t* __restrict__ cap,
+                              const int64_t* __restrict__ capoff, int64_t nu,
+                              const uint32_t* __restrict__ cls, uint64_t* __restrict__ order_keys, int64_t stack_limit)
+{
+    for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < nu; u += (int64_t)gridDim.x * blockDim.x) {
         units[u].stack_base = capoff[u];
+        units[u].edges = cap[u];
         units[u].stack_cap = (stack_limit >= 0 && cap[u] > stack_limit) ? stack_limit : cap[u];
         const uint64_t work = (uint64_t)(units[u].seed_end - units[u].seed_begin);
-        const int64_t r = units[u].root;
-        const bool rounds = (int64_t)work >= round_min && (double)tsum[r] <= round_max_list * (double)ecount[r];
-        if (rounds) atomicAdd(nbig, 1u);
-        order_keys[u] = ((uint64_t)(rounds ? 0u : 1u) << 63) |
-                        ((uint64_t)(0x7fffffffu - (uint32_t)(work < 0x7fffffffull ? work : 0x7fffffffull)) << 32) |
-                        (uint64_t)u;
+        const uint64_t w = work < 0x3fffffffull ? work : 0x3fffffffull;
+        order_keys[u] = ((uint64_t)cls[u] << 62) | ((0x3fffffffull - w) << 32) | (uint64_t)u;
     }
 }
 
@@ -747,66 +781,79 @@ int initial_clean(rtr_graph* g, double eps)
         UnitDesc* units = (UnitDesc*)sc.get(sizeof(UnitDesc) * (nu + 1));
         int64_t* cap = (int64_t*)sc.get(sizeof(int64_t) * (nu + 1));
         int64_t* capoff = (int64_t*)sc.get(sizeof(int64_t) * (nu + 1));
+        uint32_t* cls = (uint32_t*)sc.get(sizeof(uint32_t) * (nu + 1));
         int64_t* ctmp = (int64_t*)sc.get(sizeof(int64_t) * scan_temp_elems(nu + 1));
-        int64_t* d_cap_total = (int64_t*)sc.get(sizeof(int64_t));
+        int64_t* d_tot = (int64_t*)sc.get(sizeof(int64_t) * 4);  // stack entries, triangles, wide and narrow units
         uint64_t* okeys = (uint64_t*)sc.get(sizeof(uint64_t) * (nu + 1));
         uint64_t* oalt = (uint64_t*)sc.get(sizeof(uint64_t) * (nu + 1));
         void* otmp = sc.get(radix_temp_bytes(nu));
-        unsigned* next_unit = (unsigned*)sc.get(sizeof(unsigned) * 4);
-        if (!units || !cap || !capoff || !ctmp || !d_cap_total || !okeys || !oalt || !otmp || !next_unit) {
+        unsigned* next_unit = (unsigned*)sc.get(sizeof(unsigned));
+        if (!units || !cap || !capoff || !cls || !ctmp || !d_tot || !okeys || !oalt || !otmp ||
+            !next_unit) {
             set_error("device allocation failed (clean units)");
             return RTR_ERR_CUDA;
         }
-        RTR_CUDA_TRY(cudaMemsetAsync(next_unit, 0, sizeof(unsigned) * 4, s));
+        RTR_CUDA_TRY(cudaMemsetAsync(next_unit, 0, sizeof(unsigned), s));
+        RTR_CUDA_TRY(cudaMemsetAsync(d_tot, 0, sizeof(int64_t) * 4, s));
+        UnitRule rule{g->clean_round_min, g->clean_round_list, kNarrowList};
+        if (g->clean_auto) rule = UnitRule{kAutoSeeds, 1e300, kNarrowList};
         k_unit_desc<<<gs, kBlock, 0, s>>>(sorted, ns, rbits, head, hpos, ecount, units, cap);
-        exclusive_scan_i64(cap, capoff, nu, d_cap_total, ctmp, s);
-        k_unit_finish<<<grid_for(nu, kBlock), kBlock, 0, s>>>(units, cap, capoff, nu, ns, ecount, tsum,
-                                                              g->clean_round_min, g->clean_round_list, okeys,
-                                                              next_unit + 1, g->clean_stack_limit);
-        uint64_t* order = radix_sort_u64(okeys, oalt, nu, 64, otmp, s);
-        g->launches += 5 + 24;
-        int64_t cap_total = 0;
-        unsigned nbig = 0;
-        RTR_CUDA_TRY(cudaMemcpyAsync(&cap_total, d_cap_total, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        RTR_CUDA_TRY(cudaMemcpyAsync(&nbig, next_unit + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+        k_unit_class<<<grid_for(nu, kBlock), kBlock, 0, s>>>(units, nu, ns, ecount, tsum, rule, cls,
+                                                             (unsigned long long*)(d_tot + 1),
+                                                             (unsigned*)(d_tot + 2));
+        exclusive_scan_i64(cap, capoff, nu, d_tot, ctmp, s);
+        k_unit_finish<<<grid_for(nu, kBlock), kBlock, 0, s>>>(units, cap, capoff, nu, cls, okeys,
+                                                              g->clean_stack_limit);
+        // units ascend in the keys' low half already
+        uint64_t* order = radix_sort_bits_u64(okeys, oalt, nu, 32, 64, otmp, s);
+        g->launches += 9 + 20;
+        int64_t tot[4] = {0, 0, 0, 0};
+        RTR_CUDA_TRY(cudaMemcpyAsync(tot, d_tot, sizeof tot, cudaMemcpyDeviceToHost, s));
         RTR_CUDA_TRY(cudaStreamSynchronize(s));
-        StackEntry* stacks = (StackEntry*)sc.get(sizeof(StackEntry) * (cap_total + 1));
+        const unsigned* nc = (const unsigned*)(tot + 2);
+        const int64_t nwide = nc[UNIT_WIDE], nnarrow = nc[UNIT_NARROW], nbig = nwide + nnarrow;
+        StackEntry* stacks = (StackEntry*)sc.get(sizeof(StackEntry) * (tot[0] + 1));
         if (!stacks) {
             set_error("device allocation failed (clean stacks)");
             return RTR_ERR_CUDA;
         }
         ktime_begin(g, KT_CLEAN_UNITS);
-        // the largest units (order[0, nbig)) replay in parallel rounds on the
-        // side stream while the others replay one warp per unit here
+        // the units order[0, nbig) take the window replay on the side streams
+        // while the others replay one warp per unit here
         RoundReplay rr;
-        cudaEvent_t joined = nullptr;
-        SideWait side_wait;  // an early return waits for the side stream before scratch is freed
+        SideWait side_wait, side_wait2;  // an early return waits for the side streams before scratch is freed
         if (nbig > 0) {
             if (!g->side) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking));
+            if (!g->side2) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&g->side2, cudaStreamNonBlocking));
             side_wait.st = g->side;
-            const int rc = clean_rounds_launch(g, sc, g->side, rec, seeds, units, order, nbig, stacks, &rr);
+            side_wait2.st = g->side2;
+            const int rc = clean_rounds_launch(g, sc, g->side, g->side2, rec, seeds, units, order, nwide, nnarrow,
+                                               tot[0], tot[1], stacks, &rr);
             if (rc) return rc;
-            RTR_CUDA_TRY(cudaEventCreateWithFlags(&joined, cudaEventDisableTiming));
-            RTR_CUDA_TRY(cudaEventRecord(joined, g->side));
         }
-        if ((int64_t)nbig < (int64_t)nu) {
+        if (nbig < (int64_t)nu) {
             CleanArgs ca{g->tl, rec, g->pv, 1 / (double)n, seeds,
                          g->clean_wait_first > 0 ? (long)g->clean_wait_first : kWaitLimit, g->clean_stack_limit};
             // one warp per unit, persistent over the unit list (largest units first)
-            const int64_t nsmall = (int64_t)nu - (int64_t)nbig;
+            const int64_t nsmall = (int64_t)nu - nbig;
             int blocks = (int)std::min<int64_t>((nsmall + kCleanWarps - 1) / kCleanWarps,
                                                 (int64_t)grid_for(1 << 30, kCleanBlock, 8));
             blocks = std::max(blocks, 1);
             const size_t smem = sizeof(WarpSmem) * kCleanWarps;
             RTR_CUDA_TRY(cudaFuncSetAttribute(k_clean_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            k_clean_units<<<blocks, kCleanBlock, smem, s>>>(ca, units, order, (int64_t)nbig, nu, stacks, next_unit,
+            k_clean_units<<<blocks, kCleanBlock, smem, s>>>(ca, units, order, nbig, nu, stacks, next_unit,
                                                             (unsigned*)(g->ctr + 1), g->ctr, g->ctr + 2);
             g->launches += 1;
             RTR_CUDA_TRY(cudaGetLastError());
         }
         if (nbig > 0) {
-            RTR_CUDA_TRY(cudaStreamWaitEvent(s, joined, 0));
-            cudaEventDestroy(joined);
+            for (cudaStream_t st : {g->side, g->side2}) {
+                cudaEvent_t joined;
+                RTR_CUDA_TRY(cudaEventCreateWithFlags(&joined, cudaEventDisableTiming));
+                cudaEventRecord(joined, st);
+                cudaStreamWaitEvent(s, joined, 0);
+                cudaEventDestroy(joined);
+            }
             const int rc = clean_rounds_finish(g, sc, &rr);
             if (rc) return rc;
         }

@@ -15,6 +15,7 @@ struct UnitDesc {
     int64_t stack_base;
     int64_t stack_cap;
     int64_t root;  // the unit's union-find root (smallest vertex id)
+    int64_t edges;  // its triangle-carrying edges
 };
 
 // One cascade-stack entry: the pair as deleteAndClean pushed it plus the
@@ -61,26 +62,28 @@ __device__ __forceinline__ PairSide pair_side(const StackEntry& c)
     return s;
 }
 
-// Round-parallel replay of the units order[0, nbig) (clean_rounds.cu): one
-// thread block per unit on the stream `side`, concurrently with whatever the
-// caller launches on the graph's stream; the per-vertex weights of those
-// units are folded in afterwards, in the reference's order, by
-// clean_rounds_finish on the graph's stream (after `side` is joined).
-struct RoundReplay {
-    int64_t nbig = 0;
-    EdgeRec* rec = nullptr;
-    const StackEntry* seeds = nullptr;
-    const UnitDesc* units = nullptr;
-    const uint64_t* order = nullptr;
-    int32_t *nx = nullptr, *nx2 = nullptr, *dd = nullptr, *dd2 = nullptr, *inv = nullptr;
-    int32_t* pop_wcnt = nullptr;
-    uint32_t *logcnt = nullptr, *logoff = nullptr, *logtmp = nullptr;
-    double* wbuf = nullptr;
-    int32_t* zbuf = nullptr;
-    int64_t *len = nullptr, *ubase = nullptr, *tmp = nullptr;
+// One pop of the window replay.
+struct alignas(16) PopLog {
+    int32_t e;   // forward rank of its edge (-1: unused)
+    int32_t n;   // live triangles it removed
+    int64_t at;  // its triangle list
 };
-int clean_rounds_launch(rtr_graph* g, Scratch& sc, cudaStream_t side, EdgeRec* rec, const StackEntry* seeds,
-                        const UnitDesc* units, const uint64_t* order, int64_t nbig, StackEntry* stacks,
+
+// Window replay (clean_rounds.cu) of the units order[0, nwide) (long triangle
+// lists) and order[nwide, nwide + nnarrow) (short ones): one thread block per
+// unit on the given streams, concurrently with whatever the caller launches on
+// the graph's stream; the popped edges' perEdge and the per-vertex weights of
+// those units are folded in afterwards, in the reference's order, by
+// clean_rounds_finish on the graph's stream (after both streams are joined).
+struct RoundReplay {
+    EdgeRec* rec = nullptr;
+    int64_t pops_cap = 0, logs_cap = 0;
+    PopLog* plog = nullptr;
+    uint8_t* live8 = nullptr;  // per list entry: its triangle was removed by the pop of its list's edge
+};
+int clean_rounds_launch(rtr_graph* g, Scratch& sc, cudaStream_t wide_st, cudaStream_t narrow_st, EdgeRec* rec,
+                        const StackEntry* seeds, const UnitDesc* units, const uint64_t* order, int64_t nwide,
+                        int64_t nnarrow, int64_t stack_entries, int64_t log_entries, StackEntry* stacks,
                         RoundReplay* rr);
 int clean_rounds_finish(rtr_graph* g, Scratch& sc, RoundReplay* rr);
 

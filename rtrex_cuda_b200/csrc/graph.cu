@@ -125,6 +125,7 @@ size_t free_device_bytes(rtr_graph* g, bool trim)
     if (trim) {
         cudaStreamSynchronize(g->stream);
         if (g->side) cudaStreamSynchronize(g->side);
+        if (g->side2) cudaStreamSynchronize(g->side2);
         cudaMemPool_t pool;
         if (cudaDeviceGetDefaultMemPool(&pool, g->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
     }

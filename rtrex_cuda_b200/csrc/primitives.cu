@@ -212,6 +212,12 @@ size_t radix_temp_bytes(int64_t n)
 
 uint64_t* radix_sort_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int nbits, void* temp, cudaStream_t s)
 {
+    return radix_sort_bits_u64(d_keys, d_alt, n, 0, nbits, temp, s);
+}
+
+uint64_t* radix_sort_bits_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int lo, int hi, void* temp,
+                              cudaStream_t s)
+{
     if (n <= 1) return d_keys;
     const int64_t ntiles = (n + kTile - 1) / kTile;
     const int64_t h = ntiles * kBins;
@@ -220,7 +226,7 @@ uint64_t* radix_sort_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int nbits
     uint32_t* stmp = offs + h;
     uint64_t* src = d_keys;
     uint64_t* dst = d_alt;
-    for (int shift = 0; shift < nbits; shift += kRadixBits) {
+    for (int shift = lo; shift < hi; shift += kRadixBits) {
         k_radix_hist<<<(unsigned)ntiles, kBlock, 0, s>>>(src, n, shift, hist, ntiles);
         scan_impl<uint32_t>(hist, offs, h, nullptr, stmp, s);
         k_radix_scatter<<<(unsigned)ntiles, kBlock, 0, s>>>(src, dst, n, shift, offs, ntiles);

@@ -22,6 +22,10 @@ size_t radix_temp_bytes(int64_t n);
 uint64_t* radix_sort_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int nbits, void* temp,
                          cudaStream_t s);
 
+// The same over bits [lo, hi) only.
+uint64_t* radix_sort_bits_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int lo, int hi, void* temp,
+                              cudaStream_t s);
+
 // Number of bits needed to represent values in [0, x].
 inline int bits_for(uint64_t x)
 {

@@ -48,11 +48,11 @@ static_assert(sizeof(TriEntry) == 32, "TriEntry must be two 16-byte vectors");
 // Clean-time state of one undirected edge, indexed by forward rank: everything
 // a pop reads or writes for the edge in one 32-byte record.
 struct alignas(16) EdgeRec {
-    double pe;     // perEdge
-    double thr;    // eps * 1/double(du*dv): the edge's cleaning threshold
-    int64_t t0;    // triangle-list start
+    double pe;     // perEdge; with cnt and ss one 16-byte vector, all that a pop writes
     uint32_t cnt;  // triangle-list length
     uint32_t ss;   // live support (low 30 bits) | status code (top 2 bits)
+    double thr;    // eps * 1/double(du*dv): the edge's cleaning threshold
+    int64_t t0;    // triangle-list start
 };
 static_assert(sizeof(EdgeRec) == 32, "EdgeRec is 32 bytes");
 constexpr uint32_t SS_SUP = (1u << 30) - 1u;

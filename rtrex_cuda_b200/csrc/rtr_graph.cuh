@@ -97,10 +97,12 @@ struct rtr_graph {
     int count_hub = 1024;
     bool lists = false;  // the last count kept the triangle lists (the clean needs them)
     // clean units with at least this many seeds and triangle lists of at most
-    // this mean length replay in parallel rounds (one thread block each); the
-    // others one warp per unit
+    // this mean length take the window replay (one thread block each); the
+    // others one warp per unit.  Until the caller sets them (clean_auto) the
+    // clean picks the window replay by its own rule, a superset of these.
     int64_t clean_round_min = 2048;
     double clean_round_list = 8.0;
+    bool clean_auto = true;
     // bounds of the clean's device-side checks, lowered only to test their reports:
     // try_wait rounds of a window's first wait (0: the full limit), unit stack entries (-1: as sized)
     int64_t clean_wait_first = 0;
@@ -108,7 +110,8 @@ struct rtr_graph {
     // extraction: components of at least this many vertices are replayed by a
     // whole thread block (the two-hop scan's pairs worked out ahead), the others by a warp
     int64_t extract_big = 512;
-    cudaStream_t side = nullptr;  // second stream of the graph (created on first use)
+    cudaStream_t side = nullptr;  // second and third streams of the graph (created on first use)
+    cudaStream_t side2 = nullptr;
 
     // stage timings from CUDA events (ms)
     float ms_build = 0, ms_count = 0, ms_clean = 0, ms_extract = 0, ms_decompose = 0, ms_expand = 0;
