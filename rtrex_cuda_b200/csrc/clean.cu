@@ -744,7 +744,7 @@ int initial_clean(rtr_graph* g, double eps)
     RTR_CUDA_TRY(cudaMemsetAsync(tsum, 0, sizeof(unsigned long long) * (n + 1), s));
     k_unit_edges<<<gm, kBlock, 0, s>>>(g->esrc, g->fwd, m, g->sup, root, ecount, tsum);
     exclusive_scan_u32(is_seed, spos, m, d_ns, stmp, s);
-    g->launches += 8;
+    g->launches += 5 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     uint32_t ns = 0;
     RTR_CUDA_TRY(cudaMemcpyAsync(&ns, d_ns, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -774,7 +774,7 @@ int initial_clean(rtr_graph* g, double eps)
         k_unit_heads<<<gs, kBlock, 0, s>>>(sorted, ns, rbits, head);
         exclusive_scan_u32(head, hpos, ns, d_ns + 1, htmp, s);
         k_seed_info<<<gs, kBlock, 0, s>>>(sorted, ns, rmask, g->fwd, g->esrc, g->nbors, g->deg, rec, seeds);
-        g->launches += 4 + 3 * ((rbits + bits_for((uint64_t)n) + 7) / 8);
+        g->launches += 3 + take_primitive_launches();
         uint32_t nu = 0;
         RTR_CUDA_TRY(cudaMemcpyAsync(&nu, d_ns + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         RTR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -806,7 +806,7 @@ int initial_clean(rtr_graph* g, double eps)
                                                               g->clean_stack_limit);
         // units ascend in the keys' low half already
         uint64_t* order = radix_sort_bits_u64(okeys, oalt, nu, 32, 64, otmp, s);
-        g->launches += 9 + 20;
+        g->launches += 3 + take_primitive_launches();
         int64_t tot[4] = {0, 0, 0, 0};
         RTR_CUDA_TRY(cudaMemcpyAsync(tot, d_tot, sizeof tot, cudaMemcpyDeviceToHost, s));
         RTR_CUDA_TRY(cudaStreamSynchronize(s));

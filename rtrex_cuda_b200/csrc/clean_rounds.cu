@@ -744,7 +744,7 @@ int clean_rounds_finish(rtr_graph* g, Scratch& sc, RoundReplay* rr)
     uint64_t* sorted = radix_sort_bits_u64(keys, alt, cnt, lb, lb + vb, rtmp, s);
     k_log_gather<<<grid_for(cnt, kBlock), kBlock, 0, s>>>(sorted, cnt, g->n, lb, wlog, ws, g->pv, runs, nruns);
     k_fold_long_runs<<<grid_for(1ll << 40, 128, 8), 128, 0, s>>>(runs, nruns, sorted, lb, ws, g->pv);
-    g->launches += 7 + 3 * ((vb + 7) / 8);
+    g->launches += 4 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     return RTR_OK;
 }

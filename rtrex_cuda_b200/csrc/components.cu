@@ -211,7 +211,7 @@ int connected_components(rtr_graph* g)
     k_cc_flatten<<<gn, kBlock, 0, s>>>(root, n, is_root);
     exclusive_scan_u32(is_root, pos, n, d_cnt, tmp, s);
     k_cc_roots<<<gn, kBlock, 0, s>>>(is_root, pos, n, fa, vis, seq);
-    g->launches += 7;
+    g->launches += 4 + take_primitive_launches();
     uint32_t ncomp = 0;
     RTR_CUDA_TRY(cudaMemcpyAsync(&ncomp, d_cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     RTR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -224,7 +224,7 @@ int connected_components(rtr_graph* g)
         k_cc_count<<<gf, kBlock, 0, s>>>(cur, nf, g->offsets, g->nbors, vis, key, cnt);
         exclusive_scan_u32(cnt, base, nf, d_cnt + 1, tmp, s);
         k_cc_write<<<gf, kBlock, 0, s>>>(cur, nf, g->offsets, g->nbors, vis, key, base, nxt);
-        g->launches += 6;
+        g->launches += 3 + take_primitive_launches();
         uint32_t nn = 0;
         RTR_CUDA_TRY(cudaMemcpyAsync(&nn, d_cnt + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         RTR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -265,7 +265,7 @@ int connected_components(rtr_graph* g)
     exclusive_scan_u32(is_root, pos, n, nullptr, tmp, s);
     k_cc_offsets<<<gn, kBlock, 0, s>>>(is_root, pos, n, g->cc_off);
     RTR_CUDA_TRY(cudaMemcpyAsync(g->cc_off + ncomp, &n, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-    g->launches += 7 + 3 * ((2 * B + 7) / 8);
+    g->launches += 4 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     RTR_CUDA_TRY(cudaStreamSynchronize(s));
     g->ncc = ncomp;

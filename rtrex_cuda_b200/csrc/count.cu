@@ -518,7 +518,7 @@ int count_triangles(rtr_graph* g)
             const uint64_t* sorted = radix_sort_u64(hkeys, halt, nh, bits_for((uint64_t)(n > 0 ? n - 1 : 0)),
                                                     htmp, s);
             k_heavy_order<<<grid_for(nh, 256), 256, 0, s>>>(sorted, nh, heavy_list);
-            g->launches += 2 + 3 * ((bits_for((uint64_t)(n > 0 ? n - 1 : 0)) + 7) / 8);
+            g->launches += 2 + take_primitive_launches();
         }
     }
     // Hit masks of the heavy edges (rows layout possible): the list fill then reads the masks
@@ -556,7 +556,7 @@ int count_triangles(rtr_graph* g)
             } else {
                 moff = nullptr;
             }
-            g->launches += 2;
+            g->launches += 1 + take_primitive_launches();
         }
     }
     ktime_begin(g, KT_EDGE_HEAVY);
@@ -566,7 +566,7 @@ int count_triangles(rtr_graph* g)
     ktime_end(g, KT_EDGE_HEAVY);
     ktime_end(g, KT_EDGE_FOLD);
     exclusive_scan_i64(cnt, g->tl_off, m2 + 1, nullptr, tmp, s);
-    g->launches += 6;
+    g->launches += 2 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     int64_t tl_len = 0;
     RTR_CUDA_TRY(cudaMemcpyAsync(&tl_len, g->tl_off + m2, sizeof(int64_t), cudaMemcpyDeviceToHost, s));

@@ -650,7 +650,7 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const int64_t* cgt,
         }
         uint64_t* sorted = radix_sort_u64(keys, alt, nbig, 64, rtmp, s);
         k_low_ids<<<grid_for(nbig, 256), 256, 0, s>>>(sorted, nbig, big);
-        g->launches += 1 + 3 * 8;
+        g->launches += 1 + take_primitive_launches();
     }
     // the block-folded vertices' segments and the slot each one starts in
     int64_t* segoff = nullptr;

@@ -541,7 +541,7 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
             const int nbits = sbits + bits_for((uint64_t)ncl);
             uint64_t* sorted = radix_sort_u64(mk, malt, nm, nbits, rtmp, s);
             k_apply_parallel<<<grid_for(nm, kBlock), kBlock, 0, s>>>(st, sorted, nm, sbits, s_vertex, err);
-            g->launches += 1 + 3 * ((nbits + 7) / 8);
+            g->launches += 1 + take_primitive_launches();
         }
         k_mark_moved<<<gs, kBlock, 0, s>>>(s_best, s_vertex, S, moved);
         g->launches += 2;

@@ -1003,7 +1003,7 @@ int extract_clusters(rtr_graph* g)
     uint64_t* csorted = radix_sort_u64(ck, calt, n, 2 * B, rtmp, s);
     k_comp_heads<<<gn, kBlock, 0, s>>>(csorted, n, B, by_rank, head, vlist);
     exclusive_scan_u32(head, hpos, n, d_nc, htmp, s);
-    g->launches += 12 + 3 * ((B + bits_for((uint64_t)m2) + 7) / 8) + 3 * ((2 * B + 7) / 8);
+    g->launches += 8 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     uint32_t nc = 0;
     RTR_CUDA_TRY(cudaMemcpyAsync(&nc, d_nc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -1029,8 +1029,9 @@ int extract_clusters(rtr_graph* g)
     exclusive_scan_i64(bneed, boff, nc, d_tot, ltmp, s);
     exclusive_scan_i64(sneed, soff, nc, d_tot + 1, ltmp, s);
     k_comp_finish<<<gc, kBlock, 0, s>>>(comps, nc, boff, soff, sneed, okeys, g->extract_big);
-    uint64_t* order = radix_sort_u64(okeys, oalt, nc, 64, otmp, s);
-    g->launches += 9 + 24;
+    // components ascend in the keys' low half already
+    uint64_t* order = radix_sort_bits_u64(okeys, oalt, nc, 32, 64, otmp, s);
+    g->launches += 3 + take_primitive_launches();
     int64_t tots[2] = {0, 0};
     RTR_CUDA_TRY(cudaMemcpyAsync(tots, d_tot, sizeof tots, cudaMemcpyDeviceToHost, s));
     RTR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1203,7 +1204,7 @@ int extract_clusters(rtr_graph* g)
     k_cluster_stats<<<gn, kBlock, 0, s>>>(g->offsets, g->nbors, n, g->cluster_of,
                                           (unsigned long long*)g->cl_ne, (unsigned long long*)g->cl_cut);
     k_halve<<<gk, kBlock, 0, s>>>(g->cl_ne, ncl);
-    g->launches += 8 + 3 * ((2 * B + 7) / 8);
+    g->launches += 6 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     cudaEventRecord(e1, s);
     RTR_CUDA_TRY(cudaEventSynchronize(e1));

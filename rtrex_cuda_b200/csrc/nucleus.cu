@@ -419,7 +419,7 @@ int nucleus_run(rtr_graph* g)
         uint64_t* sorted = radix_sort_u64(k1, k2, n, B + bits_for((uint64_t)g->m2), rtmp, s);
         k_nuc_rank<<<gn, kBlock, 0, s>>>(sorted, n, mask, inv, newid);
         k_nuc_pairs<<<grid_for(m, kBlock), kBlock, 0, s>>>(g->fwd, g->esrc, g->nbors, newid, m, du, dv);
-        g->launches += 3 + 3 * ((B + bits_for((uint64_t)g->m2) + 7) / 8);
+        g->launches += 3 + take_primitive_launches();
         RTR_CUDA_TRY(cudaGetLastError());
         RTR_CUDA_TRY(cudaStreamSynchronize(s));
         int rc = make_graph_handle(n, g->device, &rel.g);
@@ -562,7 +562,7 @@ int nucleus_run(rtr_graph* g)
         k_nuc_member_keys<<<grid_for(ncl, kBlock), kBlock, 0, rs>>>(ta.cl_voff, ncl, ta.cl_vert, B, mk);
         uint64_t* ms = radix_sort_u64(mk, ma, cnt, B + KB, mt, rs);
         k_nuc_members<<<grid_for(cnt, kBlock), kBlock, 0, rs>>>(ms, cnt, mask, inv, mv);
-        g->launches += 2 + 3 * ((B + KB + 7) / 8);
+        g->launches += 2 + take_primitive_launches();
         RTR_CUDA_TRY(cudaGetLastError());
         RTR_CUDA_TRY(cudaMemcpyAsync(g->nuc_vert.data(), mv, sizeof(int64_t) * cnt, cudaMemcpyDeviceToHost, rs));
     }

@@ -26,6 +26,9 @@ uint64_t* radix_sort_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int nbits
 uint64_t* radix_sort_bits_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int lo, int hi, void* temp,
                               cudaStream_t s);
 
+// Kernels that the calling thread's scans and sorts have launched since it last asked.
+int64_t take_primitive_launches();
+
 // Number of bits needed to represent values in [0, x].
 inline int bits_for(uint64_t x)
 {
