@@ -40,6 +40,7 @@
 #include "clean_units.cuh"
 #include "primitives.cuh"
 #include "rtr_graph.cuh"
+#include "unionfind.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -101,35 +102,6 @@ __global__ void k_clean_finish(const int32_t* __restrict__ fwd, int64_t m, const
         pe[i] = r.pe;
         sup[i] = r.ss & SS_SUP;
         st[i] = status_char(r.ss);
-    }
-}
-
-__device__ __forceinline__ int32_t uf_find(int32_t* p, int32_t x)
-{
-    while (true) {
-        const int32_t px = p[x];
-        if (px == x) return x;
-        const int32_t ppx = p[px];
-        if (ppx != px) atomicCAS(&p[x], px, ppx);
-        x = px;
-    }
-}
-
-__device__ __forceinline__ void uf_unite(int32_t* p, int32_t a, int32_t b)
-{
-    while (true) {
-        a = uf_find(p, a);
-        b = uf_find(p, b);
-        if (a == b) return;
-        if (a > b) {
-            const int32_t t = a;
-            a = b;
-            b = t;
-        }
-        // hook the larger root under the smaller: the final root is the minimum id
-        const int32_t old = atomicCAS(&p[b], b, a);
-        if (old == b) return;
-        b = old;
     }
 }
 

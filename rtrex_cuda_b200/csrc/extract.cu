@@ -19,6 +19,7 @@
 #include "primitives.cuh"
 #include "rtr_graph.cuh"
 #include "stl_order.cuh"
+#include "unionfind.cuh"
 
 #include <algorithm>
 
@@ -63,17 +64,6 @@ __global__ void k_rank(const uint64_t* __restrict__ sorted, int64_t n, uint64_t 
     }
 }
 
-__device__ __forceinline__ int32_t uf_find(int32_t* p, int32_t x)
-{
-    while (true) {
-        const int32_t px = p[x];
-        if (px == x) return x;
-        const int32_t ppx = p[px];
-        if (ppx != px) atomicCAS(&p[x], px, ppx);
-        x = px;
-    }
-}
-
 __global__ void k_uf_init(int32_t* __restrict__ p, int64_t n)
 {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
@@ -87,20 +77,7 @@ __global__ void k_uf_hook_alive(const int32_t* __restrict__ esrc, const int32_t*
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < m; k += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = fwd[k];
         if (st[i] != ST_Y) continue;
-        int32_t a = esrc[i], b = nb[i];
-        while (true) {
-            a = uf_find(p, a);
-            b = uf_find(p, b);
-            if (a == b) break;
-            if (a > b) {
-                const int32_t t = a;
-                a = b;
-                b = t;
-            }
-            const int32_t old = atomicCAS(&p[b], b, a);
-            if (old == b) break;
-            b = old;
-        }
+        uf_unite(p, esrc[i], nb[i]);
     }
 }
 
