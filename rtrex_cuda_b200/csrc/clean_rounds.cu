@@ -50,6 +50,7 @@
 // An item whose list does not fit is popped alone, its entries taken one block
 // width at a time.
 #include "clean_units.cuh"
+#include "fold_run.cuh"
 #include "primitives.cuh"
 #include "rtr_graph.cuh"
 
@@ -635,27 +636,20 @@ __global__ void k_log_gather(const uint64_t* __restrict__ keys, int64_t cnt, int
     }
 }
 
-// A warp per long run: 32 weights per load, the next 32 in flight, subtracted in
-// order (a missing weight subtracts +0.0, which changes no bit).
+// A warp per long run.
 __global__ void __launch_bounds__(128) k_fold_long_runs(const longlong2* __restrict__ runs,
                                                         const unsigned* __restrict__ nruns,
                                                         const uint64_t* __restrict__ keys, int lb,
                                                         const double* __restrict__ ws, double* __restrict__ pv)
 {
+    __shared__ __align__(16) double s_w[4][kFoldStep];
     const int lane = threadIdx.x & 31;
     const int64_t nr = *nruns;
     for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < nr;
          r += ((int64_t)gridDim.x * blockDim.x) >> 5) {
         const longlong2 run = runs[r];
         const int64_t v = (int64_t)(keys[run.x] >> lb);
-        double x = pv[v];
-        double w = run.x + lane < run.y ? ws[run.x + lane] : 0.0;
-        for (int64_t b = run.x; b < run.y; b += 32) {
-            const double nw = b + 32 + lane < run.y ? ws[b + 32 + lane] : 0.0;
-#pragma unroll
-            for (int k = 0; k < 32; ++k) x -= __shfl_sync(kFull, w, k);
-            w = nw;
-        }
+        const double x = fold_run<true>(ws + run.x, run.y - run.x, pv[v], s_w[threadIdx.x >> 5]);
         if (lane == 0) pv[v] = x;
     }
 }

@@ -35,6 +35,7 @@
 // which a vertex is folded by a warp; g->tune_edge: the degree sum from which an
 // edge is intersected by a warp) change how work is spread, never a result; the
 // autotuner (rtr_autotune) times candidates on the graph itself.
+#include "fold_run.cuh"
 #include "intersect.cuh"
 #include "primitives.cuh"
 #include "rowsets.cuh"
@@ -338,54 +339,107 @@ __global__ void __launch_bounds__(kHeavyEdgeBlock)
     }
 }
 
-// Entries of edge c = fwd(x,y) with z > y: [first, tl_off[c+1]).
-__device__ __forceinline__ int64_t first_above(const TriEntry* __restrict__ tl, int64_t lo, int64_t hi, int32_t y)
+// perVertex[x] = left fold over y in N(x) ascending, then z > y ascending, of the
+// triangle weights (Decomposition.h:95-101).  Slot i = (x,y) adds the last
+// cgt[i] entries of its edge's list (those with z > y).  Bound by one dependent
+// double add per term of the largest vertex (8 cycles each, 4.1 ns).
+//
+// k_fold_gather copies the terms' weights into fold order (lpos, the scan of
+// cgt over the slots): eight lanes per slot.  Then a vertex's terms lie side by
+// side: k_fold_terms_light folds a vertex of fewer than kFoldWarp terms per
+// thread, k_fold_terms_heavy one of more per warp (fold_run.cuh).  Vertices are
+// dealt by id modulo the warp count (power-law generators put hubs at
+// neighbouring ids).
+//   R-MAT, 500,009 edges, 6.1 M triangles: 5.58 -> 0.92 ms; 203,311 edges, 2.0 M
+//   triangles: 3.37 -> 0.57 ms (before: a binary search per slot for its first
+//   entry, and per 32 terms a search, a gather and the adds, none overlapped).
+constexpr int kFoldWarp = 64;
+// The gather visits every slot: it pays from one term per this many slots on
+// (4,152 terms over 10,000 slots 0.023 against 0.050 ms folded from the lists,
+// 358,398 over 1.85 M 0.11 against 0.13; but 23,409 over 400,000 0.038 against 0.029).
+constexpr int64_t kSlotsPerTerm = 8;
+
+__global__ void __launch_bounds__(kBlock)
+    k_fold_gather(const int32_t* __restrict__ esrc, const int32_t* __restrict__ nb, const int32_t* __restrict__ partner,
+                  int64_t m2, const int64_t* __restrict__ cgt, const int64_t* __restrict__ lpos,
+                  const int64_t* __restrict__ tl_off, const TriEntry* __restrict__ tl, double* __restrict__ terms)
 {
-    while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (tl[mid].z <= y) lo = mid + 1;
-        else hi = mid;
+    const int sub = threadIdx.x & 7;
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3; i < m2;
+         i += ((int64_t)gridDim.x * blockDim.x) >> 3) {
+        const int64_t len = cgt[i];
+        if (len == 0) continue;
+        const int64_t c = esrc[i] < nb[i] ? i : (int64_t)partner[i];
+        const TriEntry* from = tl + (tl_off[c + 1] - len);
+        double* to = terms + lpos[i];
+        for (int64_t j = sub; j < len; j += 8) to[j] = from[j].wgt;
     }
-    return lo;
 }
 
+__global__ void __launch_bounds__(kBlock)
+    k_fold_terms_light(const int64_t* __restrict__ off, const int64_t* __restrict__ lpos, int64_t n,
+                       const double* __restrict__ terms, double* __restrict__ pv)
+{
+    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t p0 = lpos[off[x]], p1 = lpos[off[x + 1]];
+        if (p1 - p0 >= kFoldWarp) continue;
+        double acc = 0.0;
+        for (int64_t p = p0; p < p1; ++p) acc += terms[p];
+        pv[x] = acc;
+    }
+}
 
-// perVertex[x] = left fold over y in N(x) ascending, then z > y ascending, of the
-// triangle weights (Decomposition.h:95-101).
+constexpr int kHeavyBlock = 128;
+__global__ void __launch_bounds__(kHeavyBlock)
+    k_fold_terms_heavy(const int64_t* __restrict__ off, const int64_t* __restrict__ lpos, int64_t n,
+                       const double* __restrict__ terms, double* __restrict__ pv)
+{
+    __shared__ __align__(16) double s_w[kHeavyBlock / 32][kFoldStep];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int64_t nwarps = (int64_t)gridDim.x * (kHeavyBlock / 32);
+    for (int64_t x = (int64_t)blockIdx.x * (kHeavyBlock / 32) + wib; x < n; x += nwarps) {
+        const int64_t p0 = lpos[off[x]], p1 = lpos[off[x + 1]];
+        if (p1 - p0 < kFoldWarp) continue;
+        const double acc = fold_run<false>(terms + p0, p1 - p0, 0.0, s_w[wib]);
+        if (lane == 0) pv[x] = acc;
+    }
+}
+
+// The same fold straight from the lists, without the terms' array: for graphs of
+// few triangles (fewer launches), or when there is no room for it.
 //
 // k_vertex_fold_light: one thread per vertex of degree < heavy (at most
 // heavy^2/2 entries each).
 __global__ void __launch_bounds__(kBlock)
     k_vertex_fold_light(const int64_t* __restrict__ off, const int32_t* __restrict__ nb,
                         const int32_t* __restrict__ deg, const int32_t* __restrict__ partner, int64_t n,
-                        const int64_t* __restrict__ tl_off, const TriEntry* __restrict__ tl, double* __restrict__ pv,
-                        int heavy)
+                        const int64_t* __restrict__ cgt, const int64_t* __restrict__ tl_off,
+                        const TriEntry* __restrict__ tl, double* __restrict__ pv, int heavy)
 {
     for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
         if (deg[x] >= heavy) continue;
         double acc = 0.0;
         for (int64_t i = off[x]; i < off[x + 1]; ++i) {
-            const int32_t y = nb[i];
-            const int64_t c = (x < y) ? i : (int64_t)partner[i];
+            const int64_t len = cgt[i];
+            if (len == 0) continue;
+            const int64_t c = (x < nb[i]) ? i : (int64_t)partner[i];
             const int64_t hi = tl_off[c + 1];
-            for (int64_t p = first_above(tl, tl_off[c], hi, y); p < hi; ++p) acc += tl[p].wgt;
+            for (int64_t p = hi - len; p < hi; ++p) acc += tl[p].wgt;
         }
         pv[x] = acc;
     }
 }
 
 // k_vertex_fold_heavy: one warp per vertex of degree >= heavy, dealt by id
-// modulo the warp count (power-law generators put hubs at neighbouring ids).
-// Per 32 neighbours the lanes find their entry ranges at once; the ranges'
-// entries are then loaded 32 at a time in fold order (each lane finds its range
-// by a 5-step search over the range ends in shared memory), staged in shared
-// memory, and added in order -- only the floating-point chain is sequential.
-constexpr int kHeavyBlock = 128;
+// modulo the warp count.  Per 32 neighbours the lanes find their entry ranges at
+// once; the ranges' entries are then loaded 32 at a time in fold order (each lane
+// finds its range by a 5-step search over the range ends in shared memory),
+// staged in shared memory, and added in order.
 __global__ void __launch_bounds__(kHeavyBlock)
     k_vertex_fold_heavy(const int64_t* __restrict__ off, const int32_t* __restrict__ nb,
                         const int32_t* __restrict__ deg, const int32_t* __restrict__ partner, int64_t n,
-                        const int64_t* __restrict__ tl_off, const TriEntry* __restrict__ tl, double* __restrict__ pv,
-                        int heavy)
+                        const int64_t* __restrict__ cgt, const int64_t* __restrict__ tl_off,
+                        const TriEntry* __restrict__ tl, double* __restrict__ pv, int heavy)
 {
     __shared__ int64_t s_end[kHeavyBlock / 32][32];
     __shared__ int64_t s_beg[kHeavyBlock / 32][32];
@@ -400,11 +454,9 @@ __global__ void __launch_bounds__(kHeavyBlock)
             const int64_t i = cb + lane;
             int64_t a = 0, len = 0;
             if (i < h1) {
-                const int32_t y = nb[i];
-                const int64_t c = (hx < y) ? i : (int64_t)partner[i];
-                const int64_t hi = tl_off[c + 1];
-                a = first_above(tl, tl_off[c], hi, y);
-                len = hi - a;
+                len = cgt[i];
+                const int64_t c = (hx < nb[i]) ? i : (int64_t)partner[i];
+                a = tl_off[c + 1] - len;
             }
             int64_t end = len;  // inclusive prefix of the range lengths
             for (int o = 1; o < 32; o <<= 1) {
@@ -431,6 +483,7 @@ __global__ void __launch_bounds__(kHeavyBlock)
                 for (int j = 0; j < cnt; ++j) acc += s_w[wib][j];
                 __syncwarp();
             }
+            __syncwarp();  // the ranges are rewritten next
         }
         if (lane == 0) pv[hx] = acc;
     }
@@ -485,16 +538,13 @@ int count_triangles(rtr_graph* g)
         const int rc = build_row_sets(g, sc, kSetDegree, &rs);
         if (rc) return rc;
     }
-    // per-slot counts of perVertex terms, for the rows layout's lists
-    int64_t* cgt = nullptr;
-    if (g->count_mode != 1) {
-        cgt = (int64_t*)sc.get(sizeof(int64_t) * (m2 + 1));
-        if (!cgt) {
-            set_error("device allocation failed (count scratch)");
-            return RTR_ERR_CUDA;
-        }
-        RTR_CUDA_TRY(cudaMemsetAsync(cgt, 0, sizeof(int64_t) * (m2 + 1), s));
+    // per-slot counts of perVertex terms
+    int64_t* cgt = (int64_t*)sc.get(sizeof(int64_t) * (m2 + 1));
+    if (!cgt) {
+        set_error("device allocation failed (count scratch)");
+        return RTR_ERR_CUDA;
     }
+    RTR_CUDA_TRY(cudaMemsetAsync(cgt, 0, sizeof(int64_t) * (m2 + 1), s));
     // heavy-edge perEdge folded by the count when the rows layout is likely
     const bool heavy_pe = g->count_mode == 2 || rs.tab != nullptr;
     ktime_begin(g, KT_EDGE_LIGHT);
@@ -527,7 +577,7 @@ int count_triangles(rtr_graph* g)
     std::unique_ptr<Scratch> msc;
     int64_t* moff = nullptr;
     uint32_t* masks = nullptr;
-    if (rs.tab && cgt) {
+    if (rs.tab) {
         unsigned nh = 0;
         RTR_CUDA_TRY(cudaMemcpyAsync(&nh, nheavy, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         RTR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -634,12 +684,29 @@ int count_triangles(rtr_graph* g)
     k_pe_fold_heavy<<<gh, kHeavyEdgeBlock, 0, s>>>(g->fwd, heavy_list, nheavy, g->tl_off, g->tl, g->pe);
     ktime_end(g, KT_TRI_FILL);
     ktime_begin(g, KT_VERTEX_FOLD);
-    k_vertex_fold_light<<<grid_for(n, kBlock), kBlock, 0, s>>>(g->offsets, g->nbors, g->deg, g->partner, n,
-                                                                g->tl_off, g->tl, g->pv, g->tune_heavy);
-    k_vertex_fold_heavy<<<grid_for(1ll << 40, kHeavyBlock, 16), kHeavyBlock, 0, s>>>(
-        g->offsets, g->nbors, g->deg, g->partner, n, g->tl_off, g->tl, g->pv, g->tune_heavy);
+    double* terms = nullptr;
+    if (kSlotsPerTerm * tl_len >= m2 && tl_len > 0) {
+        terms = (double*)sc.get(sizeof(double) * (size_t)tl_len);
+        if (!terms) cudaGetLastError();  // no room: the folds read the lists
+    }
+    if (terms) {
+        // cnt (scanned into tl_off above) is free: it takes the terms' offsets
+        exclusive_scan_i64(cgt, cnt, m2 + 1, nullptr, tmp, s);
+        k_fold_gather<<<grid_for(8 * m2, kBlock), kBlock, 0, s>>>(g->esrc, g->nbors, g->partner, m2, cgt, cnt,
+                                                                  g->tl_off, g->tl, terms);
+        k_fold_terms_light<<<grid_for(n, kBlock), kBlock, 0, s>>>(g->offsets, cnt, n, terms, g->pv);
+        k_fold_terms_heavy<<<grid_for(1ll << 40, kHeavyBlock, 16), kHeavyBlock, 0, s>>>(g->offsets, cnt, n, terms,
+                                                                                        g->pv);
+        g->launches += 3 + take_primitive_launches();
+    } else {
+        k_vertex_fold_light<<<grid_for(n, kBlock), kBlock, 0, s>>>(g->offsets, g->nbors, g->deg, g->partner, n, cgt,
+                                                                    g->tl_off, g->tl, g->pv, g->tune_heavy);
+        k_vertex_fold_heavy<<<grid_for(1ll << 40, kHeavyBlock, 16), kHeavyBlock, 0, s>>>(
+            g->offsets, g->nbors, g->deg, g->partner, n, cgt, g->tl_off, g->tl, g->pv, g->tune_heavy);
+        g->launches += 2;
+    }
     ktime_end(g, KT_VERTEX_FOLD);
-    g->launches += 5;
+    g->launches += 3;
     RTR_CUDA_TRY(cudaGetLastError());
     cudaEventRecord(e1, s);
     RTR_CUDA_TRY(cudaEventSynchronize(e1));
