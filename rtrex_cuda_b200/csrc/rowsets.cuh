@@ -27,6 +27,22 @@ struct RowSets {
     const int32_t* slot;   // the keys, -1 for empty slots
 };
 
+// The vertices whose perVertex chains are the longest (largest degrees), taken
+// ahead of the rest: their edges are counted first, their lists made from that,
+// and their folds run on the graph's second stream while the rest is counted
+// and filled (count_rows.cu).  Their slots are numbered together, row after row.
+struct PriorityRows {
+    int64_t count = 0;              // 0: none
+    int64_t slots = 0;              // of their rows together
+    int32_t* rows = nullptr;        // [count] vertices, degree descending
+    int32_t* rank = nullptr;        // [n] place in rows, -1 for the others
+    int64_t* base = nullptr;        // [count + 1] first slot of each row
+    int64_t edges = 0;              // heavy edges with an end among them: the front of the heavy list
+    int64_t entries = 0;            // list entries of their rows
+    bool folding = false;           // their folds are on the second stream
+    cudaEvent_t begin = nullptr, end = nullptr;
+};
+
 __device__ __forceinline__ int32_t rs_table(const RowSets& r, int32_t w) { return r.tab ? r.tab[w] : -1; }
 
 __device__ __forceinline__ uint32_t rs_hash(int32_t z, int bits)

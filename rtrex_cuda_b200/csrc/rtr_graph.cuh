@@ -94,6 +94,8 @@ struct rtr_graph {
     int64_t rows_masks_cap = 0;
     void* rows_lists = nullptr;
     int64_t rows_lists_cap = 0;
+    void* rows_ahead = nullptr;
+    int64_t rows_ahead_cap = 0;
     int count_hub = 1024;
     bool lists = false;  // the last count kept the triangle lists (the clean needs them)
     // clean units with at least this many seeds and triangle lists of at most
@@ -193,12 +195,17 @@ int build_csr(rtr_graph* g, const int64_t* d_u, const int64_t* d_v, int64_t m, b
 int build_csr_from_host_csr(rtr_graph* g, const int64_t* h_offsets, const int64_t* h_nbors);
 int count_triangles(rtr_graph* g);
 struct RowSets;
+struct PriorityRows;
+// the longest perVertex chains, ahead of the rest (count_rows.cu)
+int pick_priority_rows(rtr_graph* g, Scratch& sc, PriorityRows* pr);
+int fold_priority_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, PriorityRows* pr, const int64_t* cgt,
+                       const int32_t* heavy_list, const int64_t* moff, const uint32_t* masks);
 // hash sets of the rows of at least min_deg entries, in sc (count_rows.cu)
 int build_row_sets(rtr_graph* g, Scratch& sc, int min_deg, RowSets* out);
 // rows layout: perVertex from per-slot lists of z (count_rows.cu); cgt the
 // per-slot term counts, lpos room for their scan, heavy_list the heavy edges,
 // masks (may be null) the count's hit masks of them at word offsets moff
-int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const int64_t* cgt, int64_t* lpos,
+int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const PriorityRows& pr, int64_t* cgt, int64_t* lpos,
                const int32_t* heavy_list, const unsigned* nheavy, const int64_t* moff, const uint32_t* masks);
 int cuda_fail(cudaError_t e, const char* what, const char* file, int line);
 int initial_clean(rtr_graph* g, double eps);
