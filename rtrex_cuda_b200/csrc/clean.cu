@@ -719,8 +719,7 @@ int initial_clean(rtr_graph* g, double eps)
     g->launches += 5 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     uint32_t ns = 0;
-    RTR_CUDA_TRY(cudaMemcpyAsync(&ns, d_ns, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int rc = read_words(g, &ns, d_ns, sizeof(uint32_t))) return rc;
     g->kms[KT_CLEAN_UNITS] = 0;
     // an empty timer pair keeps the reading defined when no unit exists
     ktime_begin(g, KT_CLEAN_UNITS);
@@ -748,8 +747,7 @@ int initial_clean(rtr_graph* g, double eps)
         k_seed_info<<<gs, kBlock, 0, s>>>(sorted, ns, rmask, g->fwd, g->esrc, g->nbors, g->deg, rec, seeds);
         g->launches += 3 + take_primitive_launches();
         uint32_t nu = 0;
-        RTR_CUDA_TRY(cudaMemcpyAsync(&nu, d_ns + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        RTR_CUDA_TRY(cudaStreamSynchronize(s));
+        if (const int rc = read_words(g, &nu, d_ns + 1, sizeof(uint32_t))) return rc;
         UnitDesc* units = (UnitDesc*)sc.get(sizeof(UnitDesc) * (nu + 1));
         int64_t* cap = (int64_t*)sc.get(sizeof(int64_t) * (nu + 1));
         int64_t* capoff = (int64_t*)sc.get(sizeof(int64_t) * (nu + 1));
@@ -780,8 +778,7 @@ int initial_clean(rtr_graph* g, double eps)
         uint64_t* order = radix_sort_bits_u64(okeys, oalt, nu, 32, 64, otmp, s);
         g->launches += 3 + take_primitive_launches();
         int64_t tot[4] = {0, 0, 0, 0};
-        RTR_CUDA_TRY(cudaMemcpyAsync(tot, d_tot, sizeof tot, cudaMemcpyDeviceToHost, s));
-        RTR_CUDA_TRY(cudaStreamSynchronize(s));
+        if (const int rc = read_words(g, tot, d_tot, sizeof tot)) return rc;
         const unsigned* nc = (const unsigned*)(tot + 2);
         const int64_t nwide = nc[UNIT_WIDE], nnarrow = nc[UNIT_NARROW], nbig = nwide + nnarrow;
         StackEntry* stacks = (StackEntry*)sc.get(sizeof(StackEntry) * (tot[0] + 1));
@@ -790,20 +787,29 @@ int initial_clean(rtr_graph* g, double eps)
             return RTR_ERR_CUDA;
         }
         ktime_begin(g, KT_CLEAN_UNITS);
-        // the units order[0, nbig) take the window replay on the side streams
-        // while the others replay one warp per unit here
+        // The units order[0, nbig) take the window replay, the others replay one warp
+        // per unit; each of the three kinds that exists takes a stream of its own, the
+        // first the graph's (a side stream costs 0.1 ms to make and to destroy, a third
+        // of what a graph of 1,000 edges spends in this stage).
         RoundReplay rr;
         SideWait side_wait, side_wait2;  // an early return waits for the side streams before scratch is freed
-        if (nbig > 0) {
+        const bool has_small = nbig < (int64_t)nu;
+        cudaStream_t wide_st = s, narrow_st = s;
+        if (nwide > 0 && has_small) {
             if (!g->side) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking));
-            if (!g->side2) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&g->side2, cudaStreamNonBlocking));
-            side_wait.st = g->side;
-            side_wait2.st = g->side2;
-            const int rc = clean_rounds_launch(g, sc, g->side, g->side2, rec, seeds, units, order, nwide, nnarrow,
+            wide_st = side_wait.st = g->side;
+        }
+        if (nnarrow > 0 && (nwide > 0 || has_small)) {
+            cudaStream_t& st = wide_st == s ? g->side : g->side2;
+            if (!st) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+            narrow_st = side_wait2.st = st;
+        }
+        if (nbig > 0) {
+            const int rc = clean_rounds_launch(g, sc, wide_st, narrow_st, rec, seeds, units, order, nwide, nnarrow,
                                                tot[0], tot[1], stacks, &rr);
             if (rc) return rc;
         }
-        if (nbig < (int64_t)nu) {
+        if (has_small) {
             CleanArgs ca{g->tl, rec, g->pv, 1 / (double)n, seeds,
                          g->clean_wait_first > 0 ? (long)g->clean_wait_first : kWaitLimit, g->clean_stack_limit};
             // one warp per unit, persistent over the unit list (largest units first)
@@ -819,7 +825,8 @@ int initial_clean(rtr_graph* g, double eps)
             RTR_CUDA_TRY(cudaGetLastError());
         }
         if (nbig > 0) {
-            for (cudaStream_t st : {g->side, g->side2}) {
+            for (cudaStream_t st : {wide_st, narrow_st}) {
+                if (st == s) continue;
                 cudaEvent_t joined;
                 RTR_CUDA_TRY(cudaEventCreateWithFlags(&joined, cudaEventDisableTiming));
                 cudaEventRecord(joined, st);
@@ -835,13 +842,12 @@ int initial_clean(rtr_graph* g, double eps)
     g->launches += 1;
     RTR_CUDA_TRY(cudaGetLastError());
     cudaEventRecord(e1, s);
-    RTR_CUDA_TRY(cudaEventSynchronize(e1));
+    unsigned long long h[3];
+    if (const int rc = read_words(g, h, g->ctr, sizeof h, true)) return rc;
     cudaEventElapsedTime(&g->ms_clean, e0, e1);
     ktime_read(g, KT_CLEAN_UNITS);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    unsigned long long h[3];
-    RTR_CUDA_TRY(cudaMemcpy(h, g->ctr, sizeof h, cudaMemcpyDeviceToHost));
     if (h[1] != 0) {
         set_error("device error word 0x%llx during the clean:%s%s%s%s%s", h[1],
                   (h[1] & DEV_ERR_STACK_OVERFLOW) ? " a unit's cascade stack overflowed its region;" : "",

@@ -684,13 +684,15 @@ int clean_rounds_launch(rtr_graph* g, Scratch& sc, cudaStream_t wide_st, cudaStr
     cudaStream_t s = g->stream;
     RTR_CUDA_TRY(cudaMemsetAsync(rr->plog, 0xff, sizeof(PopLog) * (stack_entries + 1), s));
     RTR_CUDA_TRY(cudaMemsetAsync(rr->live8, 0, (size_t)g->tl_len + 16, s));
-    // the replays run on the side streams, after everything above
-    cudaEvent_t ready;
-    RTR_CUDA_TRY(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
-    cudaEventRecord(ready, s);
-    cudaStreamWaitEvent(wide_st, ready, 0);
-    cudaStreamWaitEvent(narrow_st, ready, 0);
-    cudaEventDestroy(ready);
+    // the replays on side streams run after everything above
+    if (wide_st != s || narrow_st != s) {
+        cudaEvent_t ready;
+        RTR_CUDA_TRY(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+        cudaEventRecord(ready, s);
+        for (cudaStream_t st : {wide_st, narrow_st})
+            if (st != s) cudaStreamWaitEvent(st, ready, 0);
+        cudaEventDestroy(ready);
+    }
     RoundArgs ra{g->tl,    rec,       1 / (double)g->n,         seeds,  units,     order, stacks,
                  rr->plog, rr->live8, (unsigned*)(g->ctr + 1), g->ctr, g->ctr + 2};
     if (nwide > 0) {

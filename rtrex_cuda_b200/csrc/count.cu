@@ -524,9 +524,9 @@ int count_triangles(rtr_graph* g)
     int64_t* cnt = (int64_t*)sc.get(sizeof(int64_t) * (m2 + 1));
     int64_t* tmp = (int64_t*)sc.get(sizeof(int64_t) * scan_temp_elems(m2 + 1));
     int32_t* heavy_list = (int32_t*)sc.get(sizeof(int32_t) * (m + 1));
-    unsigned* nheavy = (unsigned*)sc.get(sizeof(unsigned) * 2);
+    unsigned* nheavy = (unsigned*)(g->ctr + 5);  // heavy edges; those of the priority rows
     unsigned long long* hq = (unsigned long long*)sc.get(sizeof(unsigned long long) * 3);  // k_edge_count_heavy's queues
-    if (!cnt || !tmp || !heavy_list || !nheavy || !hq) {
+    if (!cnt || !tmp || !heavy_list || !hq) {
         set_error("device allocation failed (count scratch)");
         return RTR_ERR_CUDA;
     }
@@ -534,14 +534,13 @@ int count_triangles(rtr_graph* g)
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
-    RTR_CUDA_TRY(cudaMemsetAsync(g->ctr, 0, 2 * sizeof(unsigned long long), s));
+    RTR_CUDA_TRY(cudaMemsetAsync(g->ctr, 0, 8 * sizeof(unsigned long long), s));
     RTR_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int64_t) * (m2 + 1), s));
     RTR_CUDA_TRY(cudaMemsetAsync(g->pe, 0, sizeof(double) * (m2 + 1), s));
     RTR_CUDA_TRY(cudaMemsetAsync(g->sup, 0, sizeof(uint32_t) * (m2 + 1), s));
     const int ge = grid_for(m, kBlock);
     const int gh = grid_for(1ll << 40, kHeavyEdgeBlock, 16);
     const int gc = grid_for(1ll << 40, kHeavyEdgeBlock, 6);  // k_edge_count_heavy: the resident blocks
-    RTR_CUDA_TRY(cudaMemsetAsync(nheavy, 0, sizeof(unsigned), s));
     RTR_CUDA_TRY(cudaMemsetAsync(hq, 0, sizeof(unsigned long long) * 3, s));
     ktime_begin(g, KT_EDGE_FOLD);
     // Hash sets of the long rows, for the heavy-edge count and the rows layout:
@@ -585,8 +584,7 @@ int count_triangles(rtr_graph* g)
     } side_guard{g, &pr};
     if (rs.tab) {  // heavy edges in the order of the sets they probe
         unsigned nh = 0;
-        RTR_CUDA_TRY(cudaMemcpyAsync(&nh, nheavy, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-        RTR_CUDA_TRY(cudaStreamSynchronize(s));
+        if (const int rc = read_words(g, &nh, nheavy, sizeof(unsigned))) return rc;
         if (nh > 1) {
             uint64_t* hkeys = (uint64_t*)sc.get(sizeof(uint64_t) * (nh + 1));
             uint64_t* halt = (uint64_t*)sc.get(sizeof(uint64_t) * (nh + 1));
@@ -596,13 +594,11 @@ int count_triangles(rtr_graph* g)
                 return RTR_ERR_CUDA;
             }
             const int nbits = bits_for((uint64_t)(n > 0 ? n - 1 : 0));
-            RTR_CUDA_TRY(cudaMemsetAsync(nheavy + 1, 0, sizeof(unsigned), s));
             k_heavy_keys<<<grid_for(nh, 256), 256, 0, s>>>(g->offsets, g->esrc, g->nbors, g->fwd, heavy_list, nh,
                                                             pr.rank, nbits, hkeys, nheavy + 1);
             const uint64_t* sorted = radix_sort_u64(hkeys, halt, nh, nbits + (pr.count > 0 ? 1 : 0), htmp, s);
             unsigned npri = 0;
-            RTR_CUDA_TRY(cudaMemcpyAsync(&npri, nheavy + 1, sizeof npri, cudaMemcpyDeviceToHost, s));
-            RTR_CUDA_TRY(cudaStreamSynchronize(s));
+            if (const int rc = read_words(g, &npri, nheavy + 1, sizeof npri)) return rc;
             pr.edges = npri;
             k_heavy_order<<<grid_for(nh, 256), 256, 0, s>>>(sorted, nh, heavy_list);
             g->launches += 2 + take_primitive_launches();
@@ -616,8 +612,7 @@ int count_triangles(rtr_graph* g)
     uint32_t* masks = nullptr;
     if (rs.tab) {
         unsigned nh = 0;
-        RTR_CUDA_TRY(cudaMemcpyAsync(&nh, nheavy, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-        RTR_CUDA_TRY(cudaStreamSynchronize(s));
+        if (const int rc = read_words(g, &nh, nheavy, sizeof(unsigned))) return rc;
         if (nh > 0) {
             msc.reset(new Scratch(g));
             int64_t* wcount = (int64_t*)msc->get(sizeof(int64_t) * (nh + 1));
@@ -631,8 +626,7 @@ int count_triangles(rtr_graph* g)
                                                                 nh, rs, wcount);
             exclusive_scan_i64(wcount, moff, nh + 1, nullptr, wtmp, s);
             int64_t words = 0;
-            RTR_CUDA_TRY(cudaMemcpyAsync(&words, moff + nh, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-            RTR_CUDA_TRY(cudaStreamSynchronize(s));
+            if (const int rc = read_words(g, &words, moff + nh, sizeof(int64_t))) return rc;
             const int64_t bytes = (int64_t)sizeof(uint32_t) * (words + 1);
             if (g->rows_masks_cap >= bytes)
                 masks = (uint32_t*)g->rows_masks;
@@ -661,23 +655,25 @@ int count_triangles(rtr_graph* g)
                                                       heavy_pe ? g->pe : nullptr, g->ctr, moff, masks, hq + 1);
     ktime_end(g, KT_EDGE_HEAVY);
     ktime_end(g, KT_EDGE_FOLD);
-    exclusive_scan_i64(cnt, g->tl_off, m2 + 1, nullptr, tmp, s);
+    exclusive_scan_i64(cnt, g->tl_off, m2 + 1, (int64_t*)(g->ctr + 4), tmp, s);
     g->launches += 2 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
-    int64_t tl_len = 0;
-    RTR_CUDA_TRY(cudaMemcpyAsync(&tl_len, g->tl_off + m2, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    unsigned long long words[2] = {0, 0};  // list entries, heavy edges (low half)
+    if (const int rc = read_words(g, words, g->ctr + 4, sizeof words)) return rc;
+    const int64_t tl_len = (int64_t)words[0];
+    const bool heavy = (unsigned)words[1] != 0;
     bool keep_lists = g->count_mode != 2;
     if (g->count_mode == 0 && (tl_len > g->tl_len || !g->tl)) {
         // keep the lists only when they fit beside what the clean will need (records, stacks);
         // a large graph first has the pool return its cached blocks
         // free memory counts the pool's cached blocks (an earlier graph's freed buffers, which a
         // later allocation reuses) and this graph's own rows-layout buffers
-        const size_t free_b =
-            device_avail_bytes(g) + (size_t)(g->rows_masks_cap + g->rows_lists_cap + g->rows_ahead_cap);
-        const double need = (double)sizeof(TriEntry) * (double)(tl_len + 1) + 64.0 * (double)(m + 1) +
-                            (double)(1ll << 30);
-        keep_lists = need <= (double)free_b;
+        const double use = (double)sizeof(TriEntry) * (double)(tl_len + 1) + 64.0 * (double)(m + 1);
+        const double own = (double)(g->rows_masks_cap + g->rows_lists_cap + g->rows_ahead_cap);
+        // the pool's cached blocks alone may do; only then the device is not asked for its free
+        // memory, which takes 64 us, as long as the rest of a small graph's count
+        keep_lists = use <= (double)pool_cached_bytes(g) ||
+                     use + (double)(1ll << 30) <= (double)device_avail_bytes(g) + own;
     }
     if (!keep_lists) {
         // rows layout: perVertex and heavy-edge perEdge straight from the CSR rows
@@ -731,9 +727,9 @@ int count_triangles(rtr_graph* g)
     ktime_begin(g, KT_TRI_FILL);
     k_tri_fill<<<ge, kBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->partner, g->fwd, g->frank, m,
                                      g->tl_off, g->tl, g->tune_gallop, g->tune_edge);
-    k_tri_fill_heavy<<<gh, kHeavyEdgeBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->partner, g->fwd,
+    if (heavy) k_tri_fill_heavy<<<gh, kHeavyEdgeBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->partner, g->fwd,
                                                     g->frank, heavy_list, nheavy, g->tune_gallop, g->tl_off, g->tl);
-    k_pe_fold_heavy<<<gh, kHeavyEdgeBlock, 0, s>>>(g->fwd, heavy_list, nheavy, g->tl_off, g->tl, g->pe);
+    if (heavy) k_pe_fold_heavy<<<gh, kHeavyEdgeBlock, 0, s>>>(g->fwd, heavy_list, nheavy, g->tl_off, g->tl, g->pe);
     ktime_end(g, KT_TRI_FILL);
     ktime_begin(g, KT_VERTEX_FOLD);
     double* terms = nullptr;
@@ -758,7 +754,7 @@ int count_triangles(rtr_graph* g)
         g->launches += 2;
     }
     ktime_end(g, KT_VERTEX_FOLD);
-    g->launches += 3;
+    g->launches += heavy ? 3 : 1;
     RTR_CUDA_TRY(cudaGetLastError());
     cudaEventRecord(e1, s);
     RTR_CUDA_TRY(cudaEventSynchronize(e1));

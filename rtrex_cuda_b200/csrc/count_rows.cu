@@ -639,8 +639,7 @@ int build_row_sets(rtr_graph* g, Scratch& sc, int min_deg, RowSets* out)
     k_rs_flags<<<grid_for(n + 1, 256), 256, 0, s>>>(g->deg, n, min_deg, flag);
     exclusive_scan_i64(flag, num, n + 1, nullptr, tmp, s);
     int64_t nt = 0;
-    RTR_CUDA_TRY(cudaMemcpyAsync(&nt, num + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int rc = read_words(g, &nt, num + n, sizeof(int64_t))) return rc;
     g->launches += 2;
     if (nt == 0) return RTR_OK;
     int32_t* owner = (int32_t*)sc.get(sizeof(int32_t) * (nt + 1));
@@ -656,8 +655,7 @@ int build_row_sets(rtr_graph* g, Scratch& sc, int min_deg, RowSets* out)
     k_rs_sizes<<<grid_for(n, 256), 256, 0, s>>>(g->deg, n, num, tab, owner, tbits, tsize);
     exclusive_scan_i64(tsize, toff, nt + 1, nullptr, ltmp, s);
     int64_t total = 0;
-    RTR_CUDA_TRY(cudaMemcpyAsync(&total, toff + nt, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int rc = read_words(g, &total, toff + nt, sizeof(int64_t))) return rc;
     int32_t* slot = (int32_t*)sc.get(sizeof(int32_t) * (total + 1));
     if (!slot) {
         set_error("device allocation failed (row sets: %lld slots)", (long long)total);
@@ -699,8 +697,7 @@ int pick_priority_rows(rtr_graph* g, Scratch& sc, PriorityRows* pr)
     const int min_deg = g->tune_edge > kPriDegree ? g->tune_edge : kPriDegree;
     k_pri_keys<<<grid_for(n, 256), 256, 0, s>>>(g->deg, n, min_deg, keys, cnt);
     unsigned found = 0;
-    RTR_CUDA_TRY(cudaMemcpyAsync(&found, cnt, sizeof found, cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int rc = read_words(g, &found, cnt, sizeof found)) return rc;
     g->launches += 1;
     if (found == 0) return RTR_OK;
     void* rtmp = tmp.get(radix_temp_bytes(found));
@@ -711,8 +708,7 @@ int pick_priority_rows(rtr_graph* g, Scratch& sc, PriorityRows* pr)
     const uint64_t* sorted = radix_sort_u64(keys, alt, found, 64, rtmp, s);
     const int64_t k = found < (unsigned)kPriRows ? found : kPriRows;
     uint64_t h[kPriRows];
-    RTR_CUDA_TRY(cudaMemcpyAsync(h, sorted, sizeof(uint64_t) * k, cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int rc = read_words(g, h, sorted, sizeof(uint64_t) * k)) return rc;
     int32_t rows[kPriRows];
     int64_t base[kPriRows + 1] = {0};
     for (int64_t i = 0; i < k; ++i) {
@@ -762,8 +758,7 @@ int fold_priority_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, PriorityRow
     exclusive_scan_i64(scnt, segoff, k + 1, nullptr, tmp, s);
     int64_t entries = 0, nseg = 0;
     RTR_CUDA_TRY(cudaMemcpyAsync(&entries, lpos + S, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaMemcpyAsync(&nseg, segoff + k, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int rc = read_words(g, &nseg, segoff + k, sizeof(int64_t))) return rc;
     g->launches += 2 + take_primitive_launches();
     // a graph-owned buffer (reused by later counts) of at most an eighth of the free memory: a
     // smaller row's list then fits in what is left
@@ -870,8 +865,7 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const PriorityRows&
         k_seg_counts<<<grid_for(nhuge + 1, 256), 256, 0, s>>>(g->offsets, lpos, nullptr, big, nhuge, scnt);
         exclusive_scan_i64(scnt, segoff, nhuge + 1, nullptr, stmp, s);
         int64_t nseg = 0;
-        RTR_CUDA_TRY(cudaMemcpyAsync(&nseg, segoff + nhuge, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        RTR_CUDA_TRY(cudaStreamSynchronize(s));
+        if (const int rc = read_words(g, &nseg, segoff + nhuge, sizeof(int64_t))) return rc;
         segslot = (int32_t*)sc.get(sizeof(int32_t) * (nseg + 1));
         if (!segslot) {
             set_error("device allocation failed (rows layout)");

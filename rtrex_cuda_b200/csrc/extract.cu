@@ -847,11 +847,12 @@ __global__ void k_cluster_gather(const uint64_t* __restrict__ sorted, int64_t nc
     }
 }
 
-__global__ void k_cluster_members(const uint64_t* __restrict__ sorted, int64_t ncl, uint64_t mask,
+__global__ void k_cluster_members(const uint64_t* __restrict__ sorted, int64_t ncl, int64_t n, uint64_t mask,
                                   const int64_t* __restrict__ hdr_start, const int64_t* __restrict__ cl_off,
                                   const int32_t* __restrict__ out_vert, int32_t* __restrict__ cl_vert,
                                   int32_t* __restrict__ cluster_of)
 {
+    if (cl_off[ncl] != n) return;  // reported by the host
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ncl; g += (int64_t)gridDim.x * blockDim.x) {
         const int64_t h = (int64_t)(sorted[g] & mask);
         const int64_t src = hdr_start[h];
@@ -865,9 +866,10 @@ __global__ void k_cluster_members(const uint64_t* __restrict__ sorted, int64_t n
 
 // populateStats over the original adjacency (integer counts, order-free).
 __global__ void k_cluster_stats(const int64_t* __restrict__ off, const int32_t* __restrict__ nb, int64_t n,
-                                const int32_t* __restrict__ cluster_of, unsigned long long* __restrict__ ne,
-                                unsigned long long* __restrict__ cut)
+                                const int32_t* __restrict__ cluster_of, const int64_t* __restrict__ members,
+                                unsigned long long* __restrict__ ne, unsigned long long* __restrict__ cut)
 {
+    if (*members != n) return;  // reported by the host
     for (int64_t z = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; z < n; z += (int64_t)gridDim.x * blockDim.x) {
         const int32_t c = cluster_of[z];
         unsigned long long in = 0, outc = 0;
@@ -897,8 +899,11 @@ __global__ void k_big_count(const CompDesc* __restrict__ comps, int64_t nc, int6
         }
 }
 
-__global__ void k_halve(int64_t* __restrict__ ne, int64_t ncl)
+// Internal edges were counted from both ends; `members` takes the cluster sizes' sum.
+__global__ void k_halve(int64_t* __restrict__ ne, int64_t ncl, const int64_t* __restrict__ off,
+                        unsigned long long* __restrict__ members)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *members = (unsigned long long)off[ncl];
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ncl; g += (int64_t)gridDim.x * blockDim.x)
         ne[g] /= 2;
 }
@@ -983,8 +988,7 @@ int extract_clusters(rtr_graph* g)
     g->launches += 8 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     uint32_t nc = 0;
-    RTR_CUDA_TRY(cudaMemcpyAsync(&nc, d_nc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int rc = read_words(g, &nc, d_nc, sizeof(uint32_t))) return rc;
 
     CompDesc* comps = (CompDesc*)sc.get(sizeof(CompDesc) * (nc + 1));
     int64_t* bneed = (int64_t*)sc.get(sizeof(int64_t) * (nc + 1));
@@ -992,7 +996,7 @@ int extract_clusters(rtr_graph* g)
     int64_t* boff = (int64_t*)sc.get(sizeof(int64_t) * (nc + 1));
     int64_t* soff = (int64_t*)sc.get(sizeof(int64_t) * (nc + 1));
     int64_t* ltmp = (int64_t*)sc.get(sizeof(int64_t) * scan_temp_elems(nc + 1));
-    int64_t* d_tot = (int64_t*)sc.get(sizeof(int64_t) * 2);
+    int64_t* d_tot = (int64_t*)sc.get(sizeof(int64_t) * 4);  // buckets, stack entries, big components, the largest
     uint64_t* okeys = (uint64_t*)sc.get(sizeof(uint64_t) * (nc + 1));
     uint64_t* oalt = (uint64_t*)sc.get(sizeof(uint64_t) * (nc + 1));
     void* otmp = sc.get(radix_temp_bytes(nc));
@@ -1003,15 +1007,17 @@ int extract_clusters(rtr_graph* g)
     k_comp_begin<<<gn, kBlock, 0, s>>>(csorted, n, B, head, hpos, comps);
     const int gc = grid_for(nc, kBlock);
     k_comp_sizes<<<gc, kBlock, 0, s>>>(comps, nc, n, csorted, B, acount, bneed, sneed);
+    RTR_CUDA_TRY(cudaMemsetAsync(d_tot + 2, 0, sizeof(int64_t) * 2, s));
+    k_big_count<<<gc, kBlock, 0, s>>>(comps, nc, g->extract_big, (unsigned*)(d_tot + 2),
+                                      (unsigned long long*)(d_tot + 3));
     exclusive_scan_i64(bneed, boff, nc, d_tot, ltmp, s);
     exclusive_scan_i64(sneed, soff, nc, d_tot + 1, ltmp, s);
     k_comp_finish<<<gc, kBlock, 0, s>>>(comps, nc, boff, soff, sneed, okeys, g->extract_big);
     // components ascend in the keys' low half already
     uint64_t* order = radix_sort_bits_u64(okeys, oalt, nc, 32, 64, otmp, s);
-    g->launches += 3 + take_primitive_launches();
-    int64_t tots[2] = {0, 0};
-    RTR_CUDA_TRY(cudaMemcpyAsync(tots, d_tot, sizeof tots, cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    g->launches += 4 + take_primitive_launches();
+    int64_t tots[4] = {0, 0, 0, 0};
+    if (const int rc = read_words(g, tots, d_tot, sizeof tots)) return rc;
 
     ExtractArgs a;
     a.vbase = g->vbase;
@@ -1058,26 +1064,14 @@ int extract_clusters(rtr_graph* g)
     RTR_CUDA_TRY(cudaMemsetAsync(a.in2hop, 0, n + 16, s));
     RTR_CUDA_TRY(cudaMemsetAsync(a.triwgt, 0, sizeof(double) * (n + 1), s));
     RTR_CUDA_TRY(cudaMemsetAsync(next_comp, 0, sizeof(unsigned) * 2, s));
-    // components of at least extract_big vertices: a thread block each, on the
-    // side stream, while the others take a warp each here
-    unsigned* d_big = (unsigned*)sc.get(sizeof(unsigned) * 2);
-    unsigned long long* d_maxv = (unsigned long long*)sc.get(sizeof(unsigned long long));
-    if (!d_big || !d_maxv) {
-        set_error("device allocation failed (extract split)");
-        return RTR_ERR_CUDA;
-    }
-    RTR_CUDA_TRY(cudaMemsetAsync(d_big, 0, sizeof(unsigned) * 2, s));
-    RTR_CUDA_TRY(cudaMemsetAsync(d_maxv, 0, sizeof(unsigned long long), s));
-    k_big_count<<<gc, kBlock, 0, s>>>(comps, nc, g->extract_big, d_big, d_maxv);
-    unsigned nbig = 0;
-    unsigned long long maxv = 0;
-    RTR_CUDA_TRY(cudaMemcpyAsync(&nbig, d_big, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaMemcpyAsync(&maxv, d_maxv, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
-    g->launches += 1;
+    // components of at least extract_big vertices: a thread block each, on the side
+    // stream while the others (if any) take a warp each here
+    const unsigned nbig = (unsigned)tots[2];
+    const int64_t maxv = tots[3], warps = (int64_t)nc - nbig;
+    ktime_begin(g, KT_EXTRACT);
     SideJoin side_join;  // an early return waits for the side stream before scratch is freed
     if (nbig > 0) {
-        const int64_t hcap = (int64_t)maxv + 32;
+        const int64_t hcap = maxv + 32;
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device);
         const int64_t per_block = hcap * ((int64_t)sizeof(int32_t) + 2 * (kBigWarps - 1) * (int64_t)sizeof(PairHit));
@@ -1089,29 +1083,29 @@ int extract_clusters(rtr_graph* g)
             set_error("device allocation failed (extract pair buffers)");
             return RTR_ERR_CUDA;
         }
-        if (!g->side) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking));
-        cudaEvent_t ready;
-        RTR_CUDA_TRY(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
-        RTR_CUDA_TRY(cudaEventRecord(ready, s));
-        RTR_CUDA_TRY(cudaStreamWaitEvent(g->side, ready, 0));
-        cudaEventDestroy(ready);
-        side_join.side = g->side;
-        side_join.main = s;
-        k_extract_big<<<(unsigned)bgrid, kBigBlock, 0, g->side>>>(a, comps, order, (int64_t)nbig, next_comp + 1,
-                                                                   fbuf, hbuf, hcap);
+        cudaStream_t st = s;
+        if (warps > 0) {
+            if (!g->side) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking));
+            cudaEvent_t ready;
+            RTR_CUDA_TRY(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+            RTR_CUDA_TRY(cudaEventRecord(ready, s));
+            RTR_CUDA_TRY(cudaStreamWaitEvent(g->side, ready, 0));
+            cudaEventDestroy(ready);
+            st = side_join.side = g->side;
+            side_join.main = s;
+        }
+        k_extract_big<<<(unsigned)bgrid, kBigBlock, 0, st>>>(a, comps, order, (int64_t)nbig, next_comp + 1, fbuf,
+                                                             hbuf, hcap);
         g->launches += 1;
     }
-    {
+    if (warps > 0) {
         const int blk = kExtractBlock;
-        const int64_t warps = (int64_t)nc - nbig;  // one component per warp
         const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((warps + 3) / 4, grid_for(1 << 30, blk, 16)));
-        ktime_begin(g, KT_EXTRACT);
-        if (warps > 0)
-            k_extract_components<<<blocks, blk, 0, s>>>(a, comps, order + nbig, warps, next_comp);
-        if (nbig > 0) side_join.join();
-        ktime_end(g, KT_EXTRACT);
+        k_extract_components<<<blocks, blk, 0, s>>>(a, comps, order + nbig, warps, next_comp);
         g->launches += 1;
     }
+    side_join.join();
+    ktime_end(g, KT_EXTRACT);
     RTR_CUDA_TRY(cudaGetLastError());
 
     // clusters in creation order = ascending rank of their seeds
@@ -1122,19 +1116,15 @@ int extract_clusters(rtr_graph* g)
         return RTR_ERR_CUDA;
     }
     k_widen<<<gc, kBlock, 0, s>>>(a.ncl, ncl64, nc);
-    exclusive_scan_i64(ncl64, cpos, nc, d_tot, ltmp, s);
-    int64_t ncl = 0;
-    RTR_CUDA_TRY(cudaMemcpyAsync(&ncl, d_tot, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
-    {
-        unsigned long long h[3];
-        RTR_CUDA_TRY(cudaMemcpy(h, g->ctr, sizeof h, cudaMemcpyDeviceToHost));
-        if (h[1] != 0) {
-            set_error("device error word 0x%llx during extraction", h[1]);
-            return RTR_ERR_DEVICE;
-        }
-        g->diag_residual += (long long)h[2];
+    exclusive_scan_i64(ncl64, cpos, nc, (int64_t*)(g->ctr + 4), ltmp, s);
+    unsigned long long h[5];
+    if (const int rc = read_words(g, h, g->ctr, sizeof h, true)) return rc;
+    if (h[1] != 0) {
+        set_error("device error word 0x%llx during extraction", h[1]);
+        return RTR_ERR_DEVICE;
     }
+    g->diag_residual += (long long)h[2];
+    const int64_t ncl = (int64_t)h[4];
     uint64_t* ckeys = (uint64_t*)sc.get(sizeof(uint64_t) * (ncl + 1));
     uint64_t* calt2 = (uint64_t*)sc.get(sizeof(uint64_t) * (ncl + 1));
     void* ctmp = sc.get(radix_temp_bytes(ncl));
@@ -1164,31 +1154,27 @@ int extract_clusters(rtr_graph* g)
     const int gk = grid_for(ncl, kBlock);
     k_cluster_gather<<<gk, kBlock, 0, s>>>(csort, ncl, bmask, a.hdr_seed, a.hdr_size, g->cl_seed, size64);
     exclusive_scan_i64(size64, g->cl_off, ncl + 1, nullptr, ltmp, s);
-    {
-        // the clusters must partition the vertex set
-        int64_t members = -1;
-        RTR_CUDA_TRY(cudaMemcpyAsync(&members, g->cl_off + ncl, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        RTR_CUDA_TRY(cudaStreamSynchronize(s));
-        if (members != n) {
-            set_error("extraction produced %lld cluster members for %lld vertices", (long long)members, (long long)n);
-            return RTR_ERR_DEVICE;
-        }
-    }
-    k_cluster_members<<<gk, kBlock, 0, s>>>(csort, ncl, bmask, a.hdr_start, g->cl_off, a.out_vert, g->cl_vert,
+    k_cluster_members<<<gk, kBlock, 0, s>>>(csort, ncl, n, bmask, a.hdr_start, g->cl_off, a.out_vert, g->cl_vert,
                                             g->cluster_of);
     RTR_CUDA_TRY(cudaMemsetAsync(g->cl_ne, 0, sizeof(int64_t) * (ncl + 1), s));
     RTR_CUDA_TRY(cudaMemsetAsync(g->cl_cut, 0, sizeof(int64_t) * (ncl + 1), s));
-    k_cluster_stats<<<gn, kBlock, 0, s>>>(g->offsets, g->nbors, n, g->cluster_of,
+    k_cluster_stats<<<gn, kBlock, 0, s>>>(g->offsets, g->nbors, n, g->cluster_of, g->cl_off + ncl,
                                           (unsigned long long*)g->cl_ne, (unsigned long long*)g->cl_cut);
-    k_halve<<<gk, kBlock, 0, s>>>(g->cl_ne, ncl);
+    k_halve<<<gk, kBlock, 0, s>>>(g->cl_ne, ncl, g->cl_off, g->ctr + 5);
     g->launches += 6 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     cudaEventRecord(e1, s);
-    RTR_CUDA_TRY(cudaEventSynchronize(e1));
+    unsigned long long members = 0;
+    if (const int rc = read_words(g, &members, g->ctr + 5, sizeof members)) return rc;
     cudaEventElapsedTime(&g->ms_extract, e0, e1);
     ktime_read(g, KT_EXTRACT);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    // the clusters must partition the vertex set
+    if ((int64_t)members != n) {
+        set_error("extraction produced %lld cluster members for %lld vertices", (long long)members, (long long)n);
+        return RTR_ERR_DEVICE;
+    }
     g->stage = 4;
     return RTR_OK;
 }

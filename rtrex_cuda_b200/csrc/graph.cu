@@ -50,6 +50,14 @@ void* dev_alloc(rtr_graph* g, size_t bytes)
     return p;
 }
 
+int read_words(rtr_graph* g, void* h, const void* d, size_t bytes, bool wait)
+{
+    if (wait) RTR_CUDA_TRY(cudaStreamSynchronize(g->stream));
+    RTR_CUDA_TRY(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, g->stream));
+    RTR_CUDA_TRY(cudaStreamSynchronize(g->stream));
+    return RTR_OK;
+}
+
 void dev_free_all(rtr_graph* g)
 {
     for (void* p : g->owned) cudaFreeAsync(p, g->stream);
@@ -79,17 +87,22 @@ Scratch::~Scratch()
 // threshold is unbounded), and cudaMemGetInfo counts them as used; with trim the
 // pool first returns the blocks no allocation holds, so the figure is what a
 // large allocation can get.
-size_t device_avail_bytes(rtr_graph* g)
+size_t pool_cached_bytes(rtr_graph* g)
 {
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
     cudaMemPool_t pool;
     uint64_t reserved = 0, used = 0;
     if (cudaDeviceGetDefaultMemPool(&pool, g->device) == cudaSuccess &&
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
-        free_b += (size_t)(reserved - used);
-    return free_b;
+        return (size_t)(reserved - used);
+    return 0;
+}
+
+size_t device_avail_bytes(rtr_graph* g)
+{
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
+    return free_b + pool_cached_bytes(g);
 }
 
 void release_owned(rtr_graph* g, void** buf, int64_t* cap)
@@ -291,8 +304,7 @@ int finish_csr(rtr_graph* g, unsigned long long* h_ctr)
     k_fwd_list<<<grid_for(m2, kBlock), kBlock, 0, s>>>(flag, pos, m2, g->fwd, g->frank);
     g->launches += 2 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
-    RTR_CUDA_TRY(cudaMemcpyAsync(h_ctr, g->ctr, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int rc = read_words(g, h_ctr, g->ctr, 4 * sizeof(unsigned long long))) return rc;
     if (h_ctr[3] != 0) {
         set_error("graph is not symmetric: %llu directed edges have no reverse copy", h_ctr[3]);
         return RTR_ERR_INPUT;
@@ -340,8 +352,7 @@ int build_csr(rtr_graph* g, const int64_t* d_u, const int64_t* d_v, int64_t m, b
     k_flag_keys<<<grid_for(m2, kBlock), kBlock, 0, s>>>(sorted, m2, B, keep, g->ctr + 5, g->ctr + 6);
     g->launches += 1;
     RTR_CUDA_TRY(cudaGetLastError());
-    RTR_CUDA_TRY(cudaMemcpyAsync(h_ctr, g->ctr, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int rc = read_words(g, h_ctr, g->ctr, 8 * sizeof(unsigned long long))) return rc;
     if (h_ctr[4]) {
         set_error("%llu edges have an endpoint outside [0, %lld)", h_ctr[4], (long long)n);
         return RTR_ERR_INPUT;
@@ -361,8 +372,7 @@ int build_csr(rtr_graph* g, const int64_t* d_u, const int64_t* d_v, int64_t m, b
         k_compact_keys<<<grid_for(m2, kBlock), kBlock, 0, s>>>(sorted, keep, pos, m2, out);
         g->launches += 1 + take_primitive_launches();
         uint32_t tot = 0;
-        RTR_CUDA_TRY(cudaMemcpyAsync(&tot, d_tot, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        RTR_CUDA_TRY(cudaStreamSynchronize(s));
+        if (const int rc = read_words(g, &tot, d_tot, sizeof(uint32_t))) return rc;
         sorted = out;
         m2 = tot;
     }
@@ -406,8 +416,7 @@ int build_csr_from_host_csr(rtr_graph* g, const int64_t* h_offsets, const int64_
     k_from_host_csr<<<grid_for(n, kBlock), kBlock, 0, s>>>(g->offsets, nb64, n, g->nbors, g->esrc, g->ctr + 4);
     g->launches += 1;
     RTR_CUDA_TRY(cudaGetLastError());
-    RTR_CUDA_TRY(cudaMemcpyAsync(h_ctr, g->ctr, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    RTR_CUDA_TRY(cudaStreamSynchronize(s));
+    if (const int rc = read_words(g, h_ctr, g->ctr, 8 * sizeof(unsigned long long))) return rc;
     if (h_ctr[4]) {
         set_error("CSR rows must be strictly ascending, in range and free of self-loops (%llu violations)", h_ctr[4]);
         return RTR_ERR_INPUT;
