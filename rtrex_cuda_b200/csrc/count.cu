@@ -25,7 +25,9 @@
 // 256 entries get hash sets first (rowsets.cuh); an intersection whose longer
 // row has one walks the shorter row against it (a warp per heavy edge four
 // chunks of 32 per step, the heavy edges in the order of the sets they probe,
-// so that the probed sets stay in L2).  The same pass also counts, for both
+// so that the probed sets stay in L2); with at most 2^20 vertices, against a row
+// of bits in shared memory where many edges share it (k_edge_count_bits).  The
+// same pass also counts, for both
 // slots of every edge, the common neighbours above the slot's neighbour (the
 // rows layout's per-slot term counts, count_rows.cu), folds the heavy edges'
 // perEdge in z order, and records each heavy edge's per-chunk hit masks for the
@@ -41,6 +43,7 @@
 #include "rowsets.cuh"
 #include "rtr_graph.cuh"
 
+#include <algorithm>
 #include <memory>
 
 namespace rtr {
@@ -79,7 +82,7 @@ __global__ void __launch_bounds__(kBlock)
         const int64_t i = fwd[k];
         const int32_t u = esrc[i], v = nb[i];
         if (deg[u] + deg[v] >= heavy_edge) {  // a warp takes it (k_edge_count_heavy)
-            heavy_list[atomicAdd(nheavy, 1u)] = (int32_t)k;
+            if (heavy_list) heavy_list[atomicAdd(nheavy, 1u)] = (int32_t)k;
             continue;
         }
         const int64_t duv = (int64_t)deg[u] * (int64_t)deg[v];
@@ -137,23 +140,157 @@ __global__ void __launch_bounds__(kBlock)
 // (the same left fold over z ascending as the thread path).
 constexpr int kHeavyEdgeBlock = 128;
 
-// pe (may be null): also fold perEdge of the heavy edges, in ascending z, from
-// an ordered walk of the shorter row (the lists layout folds them from the
-// lists instead, k_pe_fold_heavy).  cgt as in k_edge_fold.  Takes the heavy edges
-// [h0, h1) (h1 < 0: to the end).
-__global__ void __launch_bounds__(kHeavyEdgeBlock, 6)
-    k_edge_count_heavy(const int64_t* __restrict__ off, const int32_t* __restrict__ nb, const int32_t* __restrict__ esrc,
-                       const int32_t* __restrict__ deg, const int32_t* __restrict__ fwd,
-                       const int32_t* __restrict__ partner, const int32_t* __restrict__ heavy_list, int64_t h0,
-                       int64_t h1, const unsigned* __restrict__ nheavy, int gallop, RowSets rs,
-                       uint32_t* __restrict__ sup,
-                       int64_t* __restrict__ cnt, int64_t* __restrict__ cgt, double* __restrict__ pe,
-                       unsigned long long* __restrict__ total, const int64_t* __restrict__ moff,
-                       uint32_t* __restrict__ masks, unsigned long long* __restrict__ next)
+struct HeavyArgs {
+    const int64_t* off;
+    const int32_t* nb;
+    const int32_t* esrc;
+    const int32_t* deg;
+    const int32_t* fwd;
+    const int32_t* partner;
+    const int32_t* heavy_list;
+    int gallop;
+    RowSets rs;
+    uint32_t* sup;
+    int64_t* cnt;
+    int64_t* cgt;  // may be null; as in k_edge_fold
+    double* pe;    // may be null: also fold perEdge of the heavy edges, in ascending z, from an ordered walk of
+                   // the shorter row (the lists layout folds them from the lists instead, k_pe_fold_heavy)
+    unsigned long long* total;
+    const int64_t* moff;  // hit masks, for the rows layout's list fill (may be null)
+    uint32_t* masks;
+};
+
+// Heavy edges in the order of their longer row w (k_heavy_keys): a run is the
+// edges of one w, apart for the priority rows' edges.  With at most 2^20 vertices
+// a run that walks at least kRunWords words of 32 elements is cut into pieces of
+// kPieceWords words, for k_edge_count_bits; the others are k_edge_count_heavy's.
+// A piece sets up a row of at most 128 KB in a microsecond or two: 256 words (8,192
+// bit tests) repay that, and pieces of 2,048 / 4,096 / 8,192 / 16,384 words take
+// 39.4 / 38.8 / 38.8 / 38.3 ms for the count of R-MAT scale 19 and 108 / 100 / 96 /
+// 94 for scale 20.  More vertices than fit one block's shared memory keep the hash
+// sets: bits shared by several ids, with the hits looked up, took three times as
+// long (scale 22: 950 ms for the heavy edges against 332).
+constexpr int64_t kRunWords = 256;
+constexpr int64_t kPieceWords = 8192;
+constexpr int kMaxBits = 20;  // of the shared-memory row: 128 KB, a block an SM; below, two blocks
+constexpr int kBitsBlock = 512, kBitsWide = 768;
+
+struct HeavyRuns {
+    const uint64_t* keys;  // per list place: w below wbits, the not-priority bit at wbits
+    int wbits;
+    int64_t n;
+    const int64_t* poff;  // [2n + 1] first piece of run w (priority edges), n + w (others); null: no pieces
+    const int32_t* fstart;  // [n] first slot of each vertex's neighbours above it
+
+    __device__ __forceinline__ int64_t run(int64_t h) const
+    {
+        const uint32_t k = (uint32_t)keys[h];
+        return (int64_t)(k & ((1u << wbits) - 1u)) + ((k >> wbits) & 1u ? n : 0);
+    }
+};
+
+// One edge's walk, a warp's: the sums, and the hits not yet in the perEdge chain.
+struct HeavyEdge {
+    int32_t u, v;
+    int64_t duv;
+    int64_t mw0, mwn, word;  // the edge's mask words, and the next one
+    unsigned c = 0, above = 0, above_u = 0;
+    int pending = 0;
+    double acc = 0.0;
+};
+
+struct alignas(16) HitBuf {
+    int32_t z[160];  // 31 left over and a step's 128
+    double w[32];
+};
+
+// The first cnt (<= 32) buffered hits enter the chain, in order.
+__device__ __forceinline__ void chain_hits(const int32_t* __restrict__ deg, int64_t duv, HitBuf& hb, int base, int cnt,
+                                           int lane, double& acc)
 {
-    __shared__ double s_w[kHeavyEdgeBlock / 32][32];
-    __shared__ int32_t s_z[kHeavyEdgeBlock / 32][128];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    hb.w[lane] = lane < cnt ? 1.0 / (double)(duv * (int64_t)deg[hb.z[base + lane]]) : 0.0;
+    __syncwarp();
+    const double2* w2 = reinterpret_cast<const double2*>(hb.w);
+    if (cnt == 32) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const double2 x = w2[q];
+            acc += x.x;
+            acc += x.y;
+        }
+    } else {
+        for (int q = 0; q < cnt; q += 2) {  // a missing weight is +0.0, which changes no sum that is not -0.0
+            const double2 x = w2[q >> 1];
+            acc += x.x;
+            acc += x.y;
+        }
+    }
+    __syncwarp();
+}
+
+// A step of B chunks of 32 elements of the shorter row, in ascending order.
+template <int B>
+__device__ __forceinline__ void take_step(const HeavyArgs& a, HeavyEdge& e, HitBuf& hb, const bool (&hit)[B],
+                                          const int32_t (&x)[B], int lane)
+{
+    const unsigned lt = (1u << lane) - 1u;
+    unsigned mine = 0;
+    int tot = e.pending;
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+        e.c += hit[b] ? 1u : 0u;
+        e.above += (hit[b] && x[b] > e.v) ? 1u : 0u;
+        e.above_u += (hit[b] && x[b] > e.u) ? 1u : 0u;
+        const unsigned mb = __ballot_sync(0xffffffffu, hit[b]);
+        if (lane == b) mine = mb;
+        if (a.pe && hit[b]) hb.z[tot + __popc(mb & lt)] = x[b];
+        tot += __popc(mb);
+    }
+    if (lane < B && e.word + lane < e.mwn) a.masks[e.mw0 + e.word + lane] = mine;
+    e.word += B;
+    if (!a.pe) return;
+    if (tot >= 32) {
+        __syncwarp();
+        int done = 0;
+        for (; tot - done >= 32; done += 32) chain_hits(a.deg, e.duv, hb, done, 32, lane, e.acc);
+        tot -= done;
+        const int32_t z = lane < tot ? hb.z[done + lane] : 0;
+        __syncwarp();
+        if (lane < tot) hb.z[lane] = z;
+    }
+    e.pending = tot;
+}
+
+__device__ __forceinline__ void finish_edge(const HeavyArgs& a, HeavyEdge& e, HitBuf& hb, int64_t i, int lane,
+                                            unsigned long long& tri)
+{
+    if (a.pe && e.pending) {
+        __syncwarp();
+        chain_hits(a.deg, e.duv, hb, 0, e.pending, lane, e.acc);
+    }
+    e.c = __reduce_add_sync(0xffffffffu, e.c);
+    e.above = __reduce_add_sync(0xffffffffu, e.above);
+    e.above_u = __reduce_add_sync(0xffffffffu, e.above_u);
+    if (lane == 0) {
+        if (a.pe) a.pe[i] = e.acc;
+        a.sup[i] = e.c;
+        a.cnt[i] = e.c;
+        if (a.cgt) {
+            a.cgt[i] = e.above;
+            a.cgt[a.partner[i]] = e.above_u;
+        }
+        tri += e.above;
+    }
+}
+
+// The heavy edges [h0, h1) (h1 < 0: to the end) that no piece covers, a warp each.
+__global__ void __launch_bounds__(kHeavyEdgeBlock, 6)
+    k_edge_count_heavy(HeavyArgs a, HeavyRuns runs, int64_t h0, int64_t h1, const unsigned* __restrict__ nheavy,
+                       unsigned long long* __restrict__ next)
+{
+    __shared__ HitBuf s_hits[kHeavyEdgeBlock / 32];
+    const int lane = threadIdx.x & 31;
+    HitBuf& hb = s_hits[threadIdx.x >> 5];
     const int64_t nh = h1 >= 0 ? h1 : (int64_t)*nheavy;
     const int64_t take = heavy_take(nh - h0);
     unsigned long long tri = 0;
@@ -161,82 +298,257 @@ __global__ void __launch_bounds__(kHeavyEdgeBlock, 6)
     while (true) {
         if (h >= hend && !next_heavy(next, h0, nh, take, h, hend)) break;
         const int64_t hh = h++;
-        const int64_t i = fwd[heavy_list[hh]];
-        const int32_t u = esrc[i], v = nb[i];
-        const int64_t u0 = off[u], u1 = off[u + 1], v0 = off[v], v1 = off[v + 1];
-        unsigned c = 0, above = 0, above_u = 0;
+        if (runs.poff) {
+            const int64_t r = runs.run(hh);
+            if (runs.poff[r + 1] > runs.poff[r]) continue;
+        }
+        const int64_t i = a.fwd[a.heavy_list[hh]];
+        HeavyEdge e;
+        e.u = a.esrc[i];
+        e.v = a.nb[i];
+        e.duv = (int64_t)a.deg[e.u] * (int64_t)a.deg[e.v];
+        e.mw0 = a.masks ? a.moff[hh] : 0;
+        e.mwn = a.masks ? a.moff[hh + 1] - e.mw0 : 0;
+        e.word = 0;
+        const int64_t u0 = a.off[e.u], u1 = a.off[e.u + 1], v0 = a.off[e.v], v1 = a.off[e.v + 1];
         // the shorter row walked against the longer one
         const bool u_short = u1 - u0 <= v1 - v0;
-        const int32_t t = rs_table(rs, u_short ? v : u);
-        const int64_t duv = (int64_t)deg[u] * (int64_t)deg[v];
-        double acc = 0.0;
+        const int32_t t = rs_table(a.rs, u_short ? e.v : e.u);
         if (t >= 0) {
-            // 4 chunks per step, their lookups and then their degrees in flight together
+            // 4 chunks per step, their lookups in flight together
             constexpr int B = 4;
-            // perEdge: the step's hits, in order, are packed one per lane (ballot ranks), so that one
-            // pass of divisions serves all four chunks, and enter the chain by shuffle
-            const unsigned lt = (1u << lane) - 1u;
-            // masks: each chunk's hit ballot, for the rows layout's list fill
-            const int64_t mw0 = masks ? moff[hh] : 0, mwn = masks ? moff[hh + 1] - mw0 : 0;
-            int64_t chunk = 0;
-            warp_probe_walk<B>(rs, t, nb, u_short ? u0 : v0, u_short ? u1 : v1, nb[(u_short ? v1 : u1) - 1], lane,
-                               [&](const bool (&hit)[B], const int32_t (&x)[B]) {
-                                   int tot = 0;
-#pragma unroll
-                                   for (int b = 0; b < B; ++b) {
-                                       c += hit[b] ? 1u : 0u;
-                                       above += (hit[b] && x[b] > v) ? 1u : 0u;
-                                       above_u += (hit[b] && x[b] > u) ? 1u : 0u;
-                                       const unsigned mb = __ballot_sync(0xffffffffu, hit[b]);
-                                       if (pe && hit[b]) s_z[wib][tot + __popc(mb & lt)] = x[b];
-                                       if (lane == 0 && chunk + b < mwn) masks[mw0 + chunk + b] = mb;
-                                       tot += __popc(mb);
-                                   }
-                                   chunk += B;
-                                   if (!pe || tot == 0) return;
-                                   __syncwarp();
-                                   for (int q0 = 0; q0 < tot; q0 += 32) {
-                                       const int j = q0 + lane;
-                                       const double w =
-                                           j < tot ? 1.0 / (double)(duv * (int64_t)deg[s_z[wib][j]]) : 0.0;
-                                       const int cc = tot - q0 < 32 ? tot - q0 : 32;
-#pragma unroll 4
-                                       for (int k = 0; k < cc; ++k) acc += __shfl_sync(0xffffffffu, w, k);
-                                   }
-                                   __syncwarp();
+            warp_probe_walk<B>(a.rs, t, a.nb, u_short ? u0 : v0, u_short ? u1 : v1, a.nb[(u_short ? v1 : u1) - 1],
+                               lane, [&](const bool (&hit)[B], const int32_t (&x)[B]) {
+                                   take_step<B>(a, e, hb, hit, x, lane);
                                });
-            if (pe && lane == 0) pe[i] = acc;
-        } else if (pe) {
-            warp_walk(rs, off, nb, u_short ? u0 : v0, u_short ? u1 : v1, u_short ? v : u, u_short ? v0 : u0,
-                      u_short ? v1 : u1, lane, [&](bool hit, int32_t z) {
-                          c += hit ? 1u : 0u;
-                          above += (hit && z > v) ? 1u : 0u;
-                          above_u += (hit && z > u) ? 1u : 0u;
-                          const double w = hit ? 1.0 / (double)(duv * (int64_t)deg[z]) : 0.0;
-                          fold_hits(hit, w, s_w[wib], lane, &acc, nullptr, 0);
+        } else if (a.pe) {
+            warp_walk(a.rs, a.off, a.nb, u_short ? u0 : v0, u_short ? u1 : v1, u_short ? e.v : e.u,
+                      u_short ? v0 : u0, u_short ? v1 : u1, lane, [&](bool hit, int32_t z) {
+                          const bool h1[1] = {hit};
+                          const int32_t x1[1] = {z};
+                          take_step<1>(a, e, hb, h1, x1, lane);
                       });
-            if (lane == 0) pe[i] = acc;
         } else {
-            warp_intersect_part(nb, u0, u1, v0, v1, gallop, lane, [&](int32_t z, int64_t, int64_t) {
-                ++c;
-                above += (z > v) ? 1u : 0u;
-                above_u += (z > u) ? 1u : 0u;
+            warp_intersect_part(a.nb, u0, u1, v0, v1, a.gallop, lane, [&](int32_t z, int64_t, int64_t) {
+                ++e.c;
+                e.above += (z > e.v) ? 1u : 0u;
+                e.above_u += (z > e.u) ? 1u : 0u;
             });
         }
-        c = __reduce_add_sync(0xffffffffu, c);
-        above = __reduce_add_sync(0xffffffffu, above);
-        above_u = __reduce_add_sync(0xffffffffu, above_u);
-        if (lane == 0) {
-            sup[i] = c;
-            cnt[i] = c;
-            if (cgt) {
-                cgt[i] = above;
-                cgt[partner[i]] = above_u;
+        finish_edge(a, e, hb, i, lane, tri);
+    }
+    if (lane == 0 && tri) atomicAdd(a.total, tri);
+}
+
+// Pieces of long runs (n <= 2^lb): a block sets the row of w as bits in shared
+// memory, and its warps walk the shorter rows against them, a bit test per
+// element.  Against the hash sets (two 16-byte loads of a random bucket each) the
+// walk was bound by the L1's lookups (95% of its peak at R-MAT scale 18); this one
+// by instructions.  The hits below v and u (cgt) are counted in the one step that
+// holds their places in the row.  Heavy edges of R-MAT scale 19 (4.7 M edges, 2.5 G
+// tests): 23.4 -> 10.7 ms; scale 20: 56 -> 32.
+__global__ void __launch_bounds__(1024, 1)
+    k_edge_count_bits(HeavyArgs a, HeavyRuns runs, const longlong2* __restrict__ pieces, int64_t np, int lb,
+                      unsigned long long* __restrict__ next)
+{
+    extern __shared__ __align__(16) unsigned char bits_raw[];
+    unsigned* bm = reinterpret_cast<unsigned*>(bits_raw);
+    HitBuf& hb = reinterpret_cast<HitBuf*>(bits_raw + ((size_t)1 << lb) / 8)[threadIdx.x >> 5];
+    __shared__ long long s_piece;
+    __shared__ int s_next;
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    constexpr int B = 4;
+    unsigned long long tri = 0;
+    while (true) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s_piece = (long long)atomicAdd(next, 1ull);
+            s_next = 0;
+        }
+        __syncthreads();
+        if (s_piece >= np) break;
+        const longlong2 pc = pieces[s_piece];
+        if (pc.x >= pc.y) continue;
+        uint4* b4 = reinterpret_cast<uint4*>(bm);
+        for (int k = threadIdx.x; k < (1 << lb) / 128; k += blockDim.x) b4[k] = make_uint4(0, 0, 0, 0);
+        const int32_t w = (int32_t)(runs.run(pc.x) % runs.n);
+        const int64_t w0 = a.off[w], w1 = a.off[w + 1];
+        const int32_t dw = a.deg[w];
+        __syncthreads();
+        for (int64_t j = w0 + threadIdx.x; j < w1; j += blockDim.x) {
+            const uint32_t x = (uint32_t)a.nb[j];
+            atomicOr(&bm[x >> 5], 1u << (x & 31));
+        }
+        __syncthreads();
+        // up to 8 edges at a time, so that every warp takes several times
+        const int64_t share = (pc.y - pc.x) / (int64_t)(blockDim.x / 32 * 8);
+        const int take = share < 1 ? 1 : share < 8 ? (int)share : 8;
+        while (true) {
+            int k0 = 0;
+            if (lane == 0) k0 = atomicAdd(&s_next, take);
+            const int64_t h0 = pc.x + __shfl_sync(0xffffffffu, k0, 0);
+            if (h0 >= pc.y) break;
+            const int ne = pc.y - h0 < take ? (int)(pc.y - h0) : take;
+            // the take's edges, one per lane
+            int32_t ei = 0, er = 0, es0 = 0, elen = 0, edy = 0, epv = 0, epu = 0;
+            int64_t em = 0;
+            if (lane <= ne && a.masks) em = a.moff[h0 + lane];
+            if (lane < ne) {
+                ei = a.fwd[a.heavy_list[h0 + lane]];
+                er = a.partner[ei];
+                const int32_t u = a.esrc[ei], v = a.nb[ei];
+                const int32_t y = u == w ? v : u;
+                es0 = (int32_t)a.off[y];
+                elen = (int32_t)(a.off[y + 1] - es0);
+                edy = a.deg[y];
+                const int32_t past_w = (y == u ? ei : er) - es0 + 1, past_y = runs.fstart[y] - es0;
+                epv = y == u ? past_w : past_y;
+                epu = y == u ? past_y : past_w;
             }
-            tri += above;
+            for (int k = 0; k < ne; ++k) {
+                const int32_t* row = a.nb + __shfl_sync(0xffffffffu, es0, k);
+                const int len = __shfl_sync(0xffffffffu, elen, k);
+                const int pv = __shfl_sync(0xffffffffu, epv, k), pu = __shfl_sync(0xffffffffu, epu, k);
+                const int64_t duv = (int64_t)dw * (int64_t)__shfl_sync(0xffffffffu, edy, k);
+                const int64_t mw0 = __shfl_sync(0xffffffffu, em, k);
+                const int mwn = (int)(__shfl_sync(0xffffffffu, em, k + 1) - mw0);
+                int c = 0, below_v = -1, below_u = -1, pending = 0;
+                double acc = 0.0;
+                uint32_t xn[B];  // past the end: w, which is not in its own row
+#pragma unroll
+                for (int b = 0; b < B; ++b) xn[b] = 32 * b + lane < len ? row[32 * b + lane] : w;
+                for (int base = 0; base < len; base += 32 * B) {
+                    uint32_t x[B];
+                    unsigned mb[B], mine = 0;
+                    bool hit[B];
+#pragma unroll
+                    for (int b = 0; b < B; ++b) {
+                        x[b] = xn[b];
+                        const int p = base + 32 * (B + b) + lane;
+                        xn[b] = p < len ? row[p] : w;
+                    }
+#pragma unroll
+                    for (int b = 0; b < B; ++b) {
+                        hit[b] = (bm[x[b] >> 5] >> (x[b] & 31)) & 1u;
+                        mb[b] = __ballot_sync(0xffffffffu, hit[b]);
+                        if (lane == b) mine = mb[b];
+                    }
+                    int tot = pending;
+#pragma unroll
+                    for (int b = 0; b < B; ++b) {
+                        if (hit[b]) hb.z[tot + __popc(mb[b] & lt)] = (int32_t)x[b];
+                        tot += __popc(mb[b]);
+                    }
+                    auto below = [&](int at) {  // hits before place `at` of the row, in this step or earlier
+                        int r = c;
+#pragma unroll
+                        for (int b = 0; b < B; ++b) {
+                            const int q = at - base - 32 * b;
+                            r += q <= 0 ? 0 : __popc(q >= 32 ? mb[b] : mb[b] & ((1u << q) - 1u));
+                        }
+                        return r;
+                    };
+                    if ((unsigned)(pv - base) < 32u * B) below_v = below(pv);
+                    if ((unsigned)(pu - base) < 32u * B) below_u = below(pu);
+                    c += tot - pending;
+                    if (lane < B && (base >> 5) + lane < mwn) a.masks[mw0 + (base >> 5) + lane] = mine;
+                    if (tot >= 32) {
+                        __syncwarp();
+                        int done = 0;
+                        for (; tot - done >= 32; done += 32) chain_hits(a.deg, duv, hb, done, 32, lane, acc);
+                        tot -= done;
+                        const int32_t z = lane < tot ? hb.z[done + lane] : 0;
+                        __syncwarp();
+                        if (lane < tot) hb.z[lane] = z;
+                    }
+                    pending = tot;
+                }
+                __syncwarp();
+                if (pending) chain_hits(a.deg, duv, hb, 0, pending, lane, acc);
+                const int64_t i = __shfl_sync(0xffffffffu, ei, k), r = __shfl_sync(0xffffffffu, er, k);
+                if (lane == 0) {
+                    const int above = below_v < 0 ? 0 : c - below_v;
+                    a.pe[i] = acc;
+                    a.sup[i] = (uint32_t)c;
+                    a.cnt[i] = c;
+                    a.cgt[i] = above;
+                    a.cgt[r] = below_u < 0 ? 0 : c - below_u;
+                    tri += (unsigned long long)above;
+                }
+            }
         }
     }
-    if (lane == 0 && tri) atomicAdd(total, tri);
+    if (lane == 0 && tri) atomicAdd(a.total, tri);
+}
+
+// The first slot of each vertex's neighbours above it.
+__global__ void k_fwd_start(const int64_t* __restrict__ off, const int32_t* __restrict__ nb, int64_t n,
+                            int32_t* __restrict__ fstart)
+{
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
+        fstart[v] = (int32_t)lower_bound_row(nb, off[v], off[v + 1], (int32_t)v);
+}
+
+// First and last place of each run in the list.
+__global__ void k_run_ends(HeavyRuns runs, int64_t nh, int32_t* __restrict__ first, int32_t* __restrict__ last)
+{
+    for (int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; h < nh; h += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = runs.run(h);
+        if (h == 0 || runs.run(h - 1) != r) first[r] = (int32_t)h;
+        if (h + 1 == nh || runs.run(h + 1) != r) last[r] = (int32_t)h + 1;
+    }
+}
+
+// Pieces of each run (`pre`: the words of the list's edges, scanned).
+__global__ void k_piece_counts(const int32_t* __restrict__ first, const int32_t* __restrict__ last,
+                               const int64_t* __restrict__ pre, RowSets rs, int64_t n, int64_t* __restrict__ cnt)
+{
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r <= 2 * n; r += (int64_t)gridDim.x * blockDim.x) {
+        int64_t c = 0;
+        if (r < 2 * n && last[r] > first[r] && rs_table(rs, (int32_t)(r % n)) >= 0) {
+            const int64_t words = pre[last[r]] - pre[first[r]];
+            if (words >= kRunWords) c = (words + kPieceWords - 1) / kPieceWords;
+        }
+        cnt[r] = c;
+    }
+}
+
+// Piece j of a run: its edges whose words begin in [j, j + 1) x kPieceWords of the run's.
+__global__ void k_pieces(const int32_t* __restrict__ first, const int32_t* __restrict__ last,
+                         const int64_t* __restrict__ pre, const int64_t* __restrict__ poff, int64_t n, int64_t np,
+                         longlong2* __restrict__ pieces)
+{
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np; p += (int64_t)gridDim.x * blockDim.x) {
+        int64_t lo = 0, hi = 2 * n;  // the last run whose first piece is at most p
+        while (hi - lo > 1) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (poff[mid] <= p) lo = mid;
+            else hi = mid;
+        }
+        const int64_t f = first[lo], l = last[lo], target = pre[f] + (p - poff[lo]) * kPieceWords;
+        auto at = [&](int64_t t) {  // the first edge whose words begin at t or later
+            int64_t x = f, y = l;
+            while (x < y) {
+                const int64_t mid = (x + y) >> 1;
+                if (pre[mid] < t) x = mid + 1;
+                else y = mid;
+            }
+            return x;
+        };
+        pieces[p] = make_longlong2(at(target), at(target + kPieceWords));
+    }
+}
+
+// The heavy edges alone, where they are to be counted before the light ones.
+__global__ void k_heavy_list(const int32_t* __restrict__ esrc, const int32_t* __restrict__ nb,
+                             const int32_t* __restrict__ deg, const int32_t* __restrict__ fwd, int64_t m,
+                             int heavy_edge, int32_t* __restrict__ heavy_list, unsigned* __restrict__ nheavy)
+{
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < m; k += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = fwd[k];
+        if (deg[esrc[i]] + deg[nb[i]] >= heavy_edge) heavy_list[atomicAdd(nheavy, 1u)] = (int32_t)k;
+    }
 }
 
 // Heavy edges keyed by the vertex whose hash set their intersection probes
@@ -499,6 +811,62 @@ __global__ void __launch_bounds__(kHeavyBlock)
     }
 }
 
+// The pieces of the list's long runs; none (runs->poff null) when there is no room.
+int cut_runs(rtr_graph* g, Scratch& sc, const RowSets& rs, int64_t nh, const int64_t* pre, HeavyRuns* runs,
+             longlong2** pieces, int64_t* np)
+{
+    cudaStream_t s = g->stream;
+    const int64_t n = g->n;
+    int32_t* ends = (int32_t*)sc.get(sizeof(int32_t) * 4 * (n + 1));
+    int64_t* pcnt = (int64_t*)sc.get(sizeof(int64_t) * (2 * n + 1));
+    int64_t* poff = (int64_t*)sc.get(sizeof(int64_t) * (2 * n + 1));
+    int64_t* tmp = (int64_t*)sc.get(sizeof(int64_t) * scan_temp_elems(2 * n + 1));
+    int32_t* fstart = (int32_t*)sc.get(sizeof(int32_t) * (n + 1));
+    if (!ends || !pcnt || !poff || !tmp || !fstart) {
+        cudaGetLastError();
+        return RTR_OK;
+    }
+    int32_t *first = ends, *last = ends + 2 * (n + 1);
+    RTR_CUDA_TRY(cudaMemsetAsync(ends, 0, sizeof(int32_t) * 4 * (n + 1), s));
+    k_fwd_start<<<grid_for(n, 256), 256, 0, s>>>(g->offsets, g->nbors, n, fstart);
+    k_run_ends<<<grid_for(nh, 256), 256, 0, s>>>(*runs, nh, first, last);
+    k_piece_counts<<<grid_for(2 * n + 1, 256), 256, 0, s>>>(first, last, pre, rs, n, pcnt);
+    exclusive_scan_i64(pcnt, poff, 2 * n + 1, nullptr, tmp, s);
+    g->launches += 3 + take_primitive_launches();
+    int64_t all = 0;
+    if (const int rc = read_words(g, &np[0], poff + n, sizeof(int64_t))) return rc;
+    if (const int rc = read_words(g, &all, poff + 2 * n, sizeof(int64_t))) return rc;
+    np[1] = all - np[0];
+    if (all == 0) return RTR_OK;
+    *pieces = (longlong2*)sc.get(sizeof(longlong2) * (size_t)all);
+    if (!*pieces) {
+        cudaGetLastError();
+        np[0] = np[1] = 0;
+        return RTR_OK;
+    }
+    k_pieces<<<grid_for(all, 256), 256, 0, s>>>(first, last, pre, poff, n, all, *pieces);
+    g->launches += 1;
+    runs->poff = poff;
+    runs->fstart = fstart;
+    return RTR_OK;
+}
+
+int launch_bits(rtr_graph* g, const HeavyArgs& ha, const HeavyRuns& runs, const longlong2* pieces, int64_t np,
+                unsigned long long* next)
+{
+    if (np == 0) return RTR_OK;
+    const int nb = bits_for((uint64_t)(g->n > 1 ? g->n - 1 : 1));
+    const int lb = nb < 10 ? 10 : nb < kMaxBits ? nb : kMaxBits;
+    const int threads = lb == kMaxBits ? kBitsWide : kBitsBlock;
+    const size_t smem = ((size_t)1 << lb) / 8 + sizeof(HitBuf) * (threads / 32);
+    RTR_CUDA_TRY(cudaFuncSetAttribute(k_edge_count_bits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t grid = std::min<int64_t>(np, grid_for(1ll << 40, threads, lb == kMaxBits ? 1 : 2));
+    k_edge_count_bits<<<(unsigned)grid, threads, smem, g->stream>>>(ha, runs, pieces, np, lb, next);
+    g->launches += 1;
+    RTR_CUDA_TRY(cudaGetLastError());
+    return RTR_OK;
+}
+
 }  // namespace
 
 int count_triangles(rtr_graph* g)
@@ -525,7 +893,7 @@ int count_triangles(rtr_graph* g)
     int64_t* tmp = (int64_t*)sc.get(sizeof(int64_t) * scan_temp_elems(m2 + 1));
     int32_t* heavy_list = (int32_t*)sc.get(sizeof(int32_t) * (m + 1));
     unsigned* nheavy = (unsigned*)(g->ctr + 5);  // heavy edges; those of the priority rows
-    unsigned long long* hq = (unsigned long long*)sc.get(sizeof(unsigned long long) * 3);  // k_edge_count_heavy's queues
+    unsigned long long* hq = (unsigned long long*)sc.get(sizeof(unsigned long long) * 5);  // the heavy counts' queues
     if (!cnt || !tmp || !heavy_list || !hq) {
         set_error("device allocation failed (count scratch)");
         return RTR_ERR_CUDA;
@@ -541,7 +909,7 @@ int count_triangles(rtr_graph* g)
     const int ge = grid_for(m, kBlock);
     const int gh = grid_for(1ll << 40, kHeavyEdgeBlock, 16);
     const int gc = grid_for(1ll << 40, kHeavyEdgeBlock, 6);  // k_edge_count_heavy: the resident blocks
-    RTR_CUDA_TRY(cudaMemsetAsync(hq, 0, sizeof(unsigned long long) * 3, s));
+    RTR_CUDA_TRY(cudaMemsetAsync(hq, 0, sizeof(unsigned long long) * 5, s));
     ktime_begin(g, KT_EDGE_FOLD);
     // Hash sets of the long rows, for the heavy-edge count and the rows layout:
     // built when the rows layout is asked for, or may be chosen (2m >= 2^25).
@@ -559,10 +927,20 @@ int count_triangles(rtr_graph* g)
     RTR_CUDA_TRY(cudaMemsetAsync(cgt, 0, sizeof(int64_t) * (m2 + 1), s));
     // heavy-edge perEdge folded by the count when the rows layout is likely
     const bool heavy_pe = g->count_mode == 2 || rs.tab != nullptr;
-    ktime_begin(g, KT_EDGE_LIGHT);
-    k_edge_fold<<<ge, kBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->fwd, g->partner, m, rs, g->pe,
-                                      g->sup, cnt, cgt, g->ctr, g->tune_gallop, g->tune_edge, heavy_list, nheavy);
-    ktime_end(g, KT_EDGE_LIGHT);
+    // The light edges, and the list of the heavy ones; with the rows layout likely, the light edges
+    // wait until the longest perVertex chains (below) are under way.
+    auto light = [&](int32_t* list) {
+        ktime_begin(g, KT_EDGE_LIGHT);
+        k_edge_fold<<<ge, kBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->fwd, g->partner, m, rs, g->pe,
+                                          g->sup, cnt, cgt, g->ctr, g->tune_gallop, g->tune_edge, list, nheavy);
+        ktime_end(g, KT_EDGE_LIGHT);
+    };
+    if (rs.tab) {
+        k_heavy_list<<<ge, kBlock, 0, s>>>(g->esrc, g->nbors, g->deg, g->fwd, m, g->tune_edge, heavy_list, nheavy);
+        g->launches += 1;
+    } else {
+        light(heavy_list);
+    }
     // the longest perVertex chains ahead of the rest, where the rows layout is likely.  Not when this
     // graph holds lists from an earlier count (they will be kept again), nor under a set window size
     // (the caller's bound is then on all the lists that are held).
@@ -582,6 +960,7 @@ int count_triangles(rtr_graph* g)
             if (pr->end) cudaEventDestroy(pr->end);
         }
     } side_guard{g, &pr};
+    HeavyRuns runs{nullptr, 0, n, nullptr, nullptr};
     if (rs.tab) {  // heavy edges in the order of the sets they probe
         unsigned nh = 0;
         if (const int rc = read_words(g, &nh, nheavy, sizeof(unsigned))) return rc;
@@ -600,6 +979,8 @@ int count_triangles(rtr_graph* g)
             unsigned npri = 0;
             if (const int rc = read_words(g, &npri, nheavy + 1, sizeof npri)) return rc;
             pr.edges = npri;
+            runs.keys = sorted;
+            runs.wbits = nbits;
             k_heavy_order<<<grid_for(nh, 256), 256, 0, s>>>(sorted, nh, heavy_list);
             g->launches += 2 + take_primitive_launches();
         }
@@ -610,6 +991,8 @@ int count_triangles(rtr_graph* g)
     std::unique_ptr<Scratch> msc;
     int64_t* moff = nullptr;
     uint32_t* masks = nullptr;
+    longlong2* pieces = nullptr;
+    int64_t np[2] = {0, 0};  // pieces of the priority rows' runs, of the others
     if (rs.tab) {
         unsigned nh = 0;
         if (const int rc = read_words(g, &nh, nheavy, sizeof(unsigned))) return rc;
@@ -627,6 +1010,10 @@ int count_triangles(rtr_graph* g)
             exclusive_scan_i64(wcount, moff, nh + 1, nullptr, wtmp, s);
             int64_t words = 0;
             if (const int rc = read_words(g, &words, moff + nh, sizeof(int64_t))) return rc;
+            if (runs.keys && n <= (1ll << kMaxBits)) {
+                const int rc = cut_runs(g, *msc, rs, nh, moff, &runs, &pieces, np);
+                if (rc) return rc;
+            }
             const int64_t bytes = (int64_t)sizeof(uint32_t) * (words + 1);
             if (g->rows_masks_cap >= bytes)
                 masks = (uint32_t*)g->rows_masks;
@@ -641,19 +1028,19 @@ int count_triangles(rtr_graph* g)
         }
     }
     ktime_begin(g, KT_EDGE_HEAVY);
+    const HeavyArgs ha{g->offsets, g->nbors, g->esrc, g->deg, g->fwd, g->partner, heavy_list, g->tune_gallop, rs, g->sup,
+                       cnt, cgt, heavy_pe ? g->pe : nullptr, g->ctr, moff, masks};
     if (pr.count > 0 && pr.edges > 0) {
-        k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->fwd, g->partner,
-                                                          heavy_list, 0, pr.edges, nheavy, g->tune_gallop, rs, g->sup,
-                                                          cnt, cgt, heavy_pe ? g->pe : nullptr, g->ctr, moff, masks, hq);
+        if (const int rc = launch_bits(g, ha, runs, pieces, np[0], hq + 2)) return rc;
+        k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(ha, runs, 0, pr.edges, nheavy, hq);
         g->launches += 1;
         const int rc = fold_priority_rows(g, sc, rs, &pr, cgt, heavy_list, moff, masks);
         if (rc) return rc;
     }
-    k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->fwd, g->partner,
-                                                      heavy_list, pr.count > 0 ? pr.edges : 0, -1, nheavy,
-                                                      g->tune_gallop, rs, g->sup, cnt, cgt,
-                                                      heavy_pe ? g->pe : nullptr, g->ctr, moff, masks, hq + 1);
+    if (const int rc = launch_bits(g, ha, runs, pieces + np[0], np[1], hq + 3)) return rc;
+    k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(ha, runs, pr.count > 0 ? pr.edges : 0, -1, nheavy, hq + 1);
     ktime_end(g, KT_EDGE_HEAVY);
+    if (rs.tab) light(nullptr);
     ktime_end(g, KT_EDGE_FOLD);
     exclusive_scan_i64(cnt, g->tl_off, m2 + 1, (int64_t*)(g->ctr + 4), tmp, s);
     g->launches += 2 + take_primitive_launches();
@@ -685,9 +1072,14 @@ int count_triangles(rtr_graph* g)
                 set_error("device allocation failed (count scratch)");
                 return RTR_ERR_CUDA;
             }
-            k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->fwd,
-                                                              g->partner, heavy_list, 0, -1, nheavy, g->tune_gallop, rs,
-                                                              g->sup, cnt, nullptr, g->pe, junk, nullptr, nullptr, hq + 2);
+            HeavyArgs again = ha;
+            again.cgt = nullptr;
+            again.pe = g->pe;
+            again.total = junk;
+            again.moff = nullptr;
+            again.masks = nullptr;
+            k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(again, HeavyRuns{nullptr, 0, n, nullptr, nullptr}, 0, -1, nheavy,
+                                                              hq + 4);
             g->launches += 1;
         }
         // cnt (scanned into tl_off above) is free: it takes the lists' offsets

@@ -674,9 +674,11 @@ int build_row_sets(rtr_graph* g, Scratch& sc, int min_deg, RowSets* out)
 // fill it ran for 21 of R-MAT scale 19's 61 ms and 147 of scale 22's 637.
 // So up to 32 rows, the largest, of at least 2,048 neighbours, go ahead: their
 // edges are counted and their lists filled first, and their chains run beside
-// the rest.  Count, rows layout, with 0 / 16 / 32 rows ahead: scale 19 60.7 / 54.2 /
-// 50.5 ms, 20 136 / 123 / 120, 22 637 / 603 / 607.  The blocks keep to two an SM's
-// shared memory (kBlockFoldSmem): given an SM each, they slowed the count beside them.
+// the rest.  Count, rows layout, with 1 / 16 / 32 / 64 / 128 rows ahead: scale 19
+// 41.1 / 41.4 / 38.2 / 38.4 / 39.1 ms, scale 20 96 / 98 / 96 / 97 / 101 (before,
+// with the count itself slower, none ahead: 60.7 and 136 for 50.5 and 120 with 32;
+// scale 22 637 for 607).  The blocks keep to two an SM's shared memory
+// (kBlockFoldSmem): given an SM each, scale 19 takes 39.5 ms.
 constexpr int kPriRows = 32;
 constexpr int kPriDegree = 2048;
 
