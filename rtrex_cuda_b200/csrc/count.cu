@@ -140,6 +140,12 @@ __global__ void __launch_bounds__(kBlock)
 // (the same left fold over z ascending as the thread path).
 constexpr int kHeavyEdgeBlock = 128;
 
+// Lists layout: the count leaves, for the first m / 2 + 1 heavy edges, the hits
+// before each lane's part of the intersection, so that k_tri_fill_heavy need not
+// intersect twice (R-MAT, 500,000 edges: 1.43 -> 0.92 ms); 64 bytes an edge, in 16
+// bits, so edges of more triangles than kPartsMax are intersected twice all the same.
+constexpr int64_t kPartsMax = 65535;
+
 struct HeavyArgs {
     const int64_t* off;
     const int32_t* nb;
@@ -158,6 +164,8 @@ struct HeavyArgs {
     unsigned long long* total;
     const int64_t* moff;  // hit masks, for the rows layout's list fill (may be null)
     uint32_t* masks;
+    uint16_t* parts;  // for k_tri_fill_heavy (kPartsMax)
+    int64_t nparts;
 };
 
 // Heavy edges in the order of their longer row w (k_heavy_keys): a run is the
@@ -334,6 +342,15 @@ __global__ void __launch_bounds__(kHeavyEdgeBlock, 6)
                 e.above += (z > e.v) ? 1u : 0u;
                 e.above_u += (z > e.u) ? 1u : 0u;
             });
+            if (hh < a.nparts) {
+                unsigned incl = e.c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                a.parts[hh * 32 + lane] = (uint16_t)(incl - e.c);  // read only when the sum fits
+            }
         }
         finish_edge(a, e, hb, i, lane, tri);
     }
@@ -604,24 +621,33 @@ __global__ void __launch_bounds__(kHeavyEdgeBlock)
                      const int32_t* __restrict__ deg, const int32_t* __restrict__ partner,
                      const int32_t* __restrict__ fwd, const int32_t* __restrict__ frank,
                      const int32_t* __restrict__ heavy_list, const unsigned* __restrict__ nheavy, int gallop,
-                     const int64_t* __restrict__ tl_off, TriEntry* __restrict__ tl)
+                     const uint16_t* __restrict__ parts, int64_t nparts, const int64_t* __restrict__ tl_off,
+                     TriEntry* __restrict__ tl, unsigned long long* __restrict__ next)
 {
     const int lane = threadIdx.x & 31;
     const int64_t nh = *nheavy;
-    const int64_t nwarps = (int64_t)gridDim.x * (kHeavyEdgeBlock / 32);
-    for (int64_t h = (int64_t)blockIdx.x * (kHeavyEdgeBlock / 32) + (threadIdx.x >> 5); h < nh; h += nwarps) {
+    const int64_t take = heavy_take(nh);
+    int64_t hq = 0, hend = 0;
+    while (true) {
+        if (hq >= hend && !next_heavy(next, 0, nh, take, hq, hend)) break;
+        const int64_t h = hq++;
         const int64_t i = fwd[heavy_list[h]];
         const int32_t u = esrc[i], v = nb[i];
         const int64_t duv = (int64_t)deg[u] * (int64_t)deg[v];
-        unsigned c = 0;
-        warp_intersect_part(nb, off[u], off[u + 1], off[v], off[v + 1], gallop, lane,
-                            [&](int32_t, int64_t, int64_t) { ++c; });
-        unsigned incl = c;  // inclusive prefix over lanes
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
+        int64_t w = tl_off[i];
+        if (h < nparts && tl_off[i + 1] - w <= kPartsMax) {
+            w += parts[h * 32 + lane];
+        } else {
+            unsigned c = 0;
+            warp_intersect_part(nb, off[u], off[u + 1], off[v], off[v + 1], gallop, lane,
+                                [&](int32_t, int64_t, int64_t) { ++c; });
+            unsigned incl = c;  // inclusive prefix over lanes
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            w += incl - c;
         }
-        int64_t w = tl_off[i] + (int64_t)(incl - c);
         warp_intersect_part(nb, off[u], off[u + 1], off[v], off[v + 1], gallop, lane,
                             [&](int32_t z, int64_t pu, int64_t pv) {
                                 TriEntry t;
@@ -672,10 +698,19 @@ __global__ void __launch_bounds__(kHeavyEdgeBlock)
 // thread, k_fold_terms_heavy one of more per warp (fold_run.cuh).  Vertices are
 // dealt by id modulo the warp count (power-law generators put hubs at
 // neighbouring ids).
-//   R-MAT, 500,009 edges, 6.1 M triangles: 5.58 -> 0.92 ms; 203,311 edges, 2.0 M
+// [lo, hi): the degrees taken.  From kAheadEdges heavy edges on, the vertices whose
+// edges are all heavy (those of tune_edge neighbours and more) are gathered and
+// folded as soon as the heavy lists are there, on the second stream, all of them a
+// warp each, beside the light lists and the other vertices: the longest chain, 0.79
+// ms of R-MAT 500,009 edges, no longer runs alone at the end.  Count of that graph
+// (162,000 heavy edges) 3.75 -> 3.12 ms, of 203,311 edges (30,000 heavy) 2.03 -> 1.69,
+// of 40,000 (1,100 heavy) 0.05 ms less -- below the 0.1 ms that making the stream
+// costs a new graph.
+//   R-MAT, 500,009 edges, 6.1 M triangles, in one go: 5.58 -> 0.92 ms; 203,311 edges, 2.0 M
 //   triangles: 3.37 -> 0.57 ms (before: a binary search per slot for its first
 //   entry, and per 32 terms a search, a gather and the adds, none overlapped).
 constexpr int kFoldWarp = 64;
+constexpr unsigned kAheadEdges = 16384;
 // The gather visits every slot: it pays from one term per this many slots on
 // (4,152 terms over 10,000 slots 0.023 against 0.050 ms folded from the lists,
 // 358,398 over 1.85 M 0.11 against 0.13; but 23,409 over 400,000 0.038 against 0.029).
@@ -683,15 +718,17 @@ constexpr int64_t kSlotsPerTerm = 8;
 
 __global__ void __launch_bounds__(kBlock)
     k_fold_gather(const int32_t* __restrict__ esrc, const int32_t* __restrict__ nb, const int32_t* __restrict__ partner,
-                  int64_t m2, const int64_t* __restrict__ cgt, const int64_t* __restrict__ lpos,
-                  const int64_t* __restrict__ tl_off, const TriEntry* __restrict__ tl, double* __restrict__ terms)
+                  const int32_t* __restrict__ deg, int lo, int hi, int64_t m2, const int64_t* __restrict__ cgt,
+                  const int64_t* __restrict__ lpos, const int64_t* __restrict__ tl_off,
+                  const TriEntry* __restrict__ tl, double* __restrict__ terms)
 {
     const int sub = threadIdx.x & 7;
     for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3; i < m2;
          i += ((int64_t)gridDim.x * blockDim.x) >> 3) {
         const int64_t len = cgt[i];
-        if (len == 0) continue;
-        const int64_t c = esrc[i] < nb[i] ? i : (int64_t)partner[i];
+        const int32_t x = esrc[i], d = deg[x];
+        if (len == 0 || d < lo || d >= hi) continue;
+        const int64_t c = x < nb[i] ? i : (int64_t)partner[i];
         const TriEntry* from = tl + (tl_off[c + 1] - len);
         double* to = terms + lpos[i];
         for (int64_t j = sub; j < len; j += 8) to[j] = from[j].wgt;
@@ -699,12 +736,12 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 __global__ void __launch_bounds__(kBlock)
-    k_fold_terms_light(const int64_t* __restrict__ off, const int64_t* __restrict__ lpos, int64_t n,
+    k_fold_terms_light(const int64_t* __restrict__ off, const int64_t* __restrict__ lpos, int64_t n, int hi,
                        const double* __restrict__ terms, double* __restrict__ pv)
 {
     for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
         const int64_t p0 = lpos[off[x]], p1 = lpos[off[x + 1]];
-        if (p1 - p0 >= kFoldWarp) continue;
+        if (p1 - p0 >= kFoldWarp || off[x + 1] - off[x] >= hi) continue;
         double acc = 0.0;
         for (int64_t p = p0; p < p1; ++p) acc += terms[p];
         pv[x] = acc;
@@ -713,7 +750,7 @@ __global__ void __launch_bounds__(kBlock)
 
 constexpr int kHeavyBlock = 128;
 __global__ void __launch_bounds__(kHeavyBlock)
-    k_fold_terms_heavy(const int64_t* __restrict__ off, const int64_t* __restrict__ lpos, int64_t n,
+    k_fold_terms_heavy(const int64_t* __restrict__ off, const int64_t* __restrict__ lpos, int64_t n, int lo, int hi,
                        const double* __restrict__ terms, double* __restrict__ pv)
 {
     __shared__ __align__(16) double s_w[kHeavyBlock / 32][kFoldStep];
@@ -721,7 +758,8 @@ __global__ void __launch_bounds__(kHeavyBlock)
     const int64_t nwarps = (int64_t)gridDim.x * (kHeavyBlock / 32);
     for (int64_t x = (int64_t)blockIdx.x * (kHeavyBlock / 32) + wib; x < n; x += nwarps) {
         const int64_t p0 = lpos[off[x]], p1 = lpos[off[x + 1]];
-        if (p1 - p0 < kFoldWarp) continue;
+        const int64_t d = off[x + 1] - off[x];
+        if ((p1 - p0 < kFoldWarp && lo == 0) || d < lo || d >= hi) continue;
         const double acc = fold_run<false>(terms + p0, p1 - p0, 0.0, s_w[wib]);
         if (lane == 0) pv[x] = acc;
     }
@@ -953,9 +991,11 @@ int count_triangles(rtr_graph* g)
     struct SideGuard {  // the second stream is done with the scratch before it is released
         rtr_graph* g;
         PriorityRows* pr;
+        cudaEvent_t lists = nullptr;
         ~SideGuard()
         {
-            if (pr->folding && g->side) cudaStreamSynchronize(g->side);
+            if ((pr->folding || lists) && g->side) cudaStreamSynchronize(g->side);
+            if (lists) cudaEventDestroy(lists);
             if (pr->begin) cudaEventDestroy(pr->begin);
             if (pr->end) cudaEventDestroy(pr->end);
         }
@@ -1028,8 +1068,13 @@ int count_triangles(rtr_graph* g)
         }
     }
     ktime_begin(g, KT_EDGE_HEAVY);
+    uint16_t* parts = nullptr;
+    if (!rs.tab && !heavy_pe) {
+        parts = (uint16_t*)sc.get(sizeof(uint16_t) * 32 * (size_t)(m / 2 + 1));
+        if (!parts) cudaGetLastError();  // no room: the fill intersects twice
+    }
     const HeavyArgs ha{g->offsets, g->nbors, g->esrc, g->deg, g->fwd, g->partner, heavy_list, g->tune_gallop, rs, g->sup,
-                       cnt, cgt, heavy_pe ? g->pe : nullptr, g->ctr, moff, masks};
+                       cnt, cgt, heavy_pe ? g->pe : nullptr, g->ctr, moff, masks, parts, parts ? m / 2 + 1 : 0};
     if (pr.count > 0 && pr.edges > 0) {
         if (const int rc = launch_bits(g, ha, runs, pieces, np[0], hq + 2)) return rc;
         k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(ha, runs, 0, pr.edges, nheavy, hq);
@@ -1078,6 +1123,7 @@ int count_triangles(rtr_graph* g)
             again.total = junk;
             again.moff = nullptr;
             again.masks = nullptr;
+            again.nparts = 0;
             k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(again, HeavyRuns{nullptr, 0, n, nullptr, nullptr}, 0, -1, nheavy,
                                                               hq + 4);
             g->launches += 1;
@@ -1116,27 +1162,58 @@ int count_triangles(rtr_graph* g)
     }
     g->tl_len = tl_len;
     g->lists = true;
-    ktime_begin(g, KT_TRI_FILL);
-    k_tri_fill<<<ge, kBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->partner, g->fwd, g->frank, m,
-                                     g->tl_off, g->tl, g->tune_gallop, g->tune_edge);
-    if (heavy) k_tri_fill_heavy<<<gh, kHeavyEdgeBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->partner, g->fwd,
-                                                    g->frank, heavy_list, nheavy, g->tune_gallop, g->tl_off, g->tl);
-    if (heavy) k_pe_fold_heavy<<<gh, kHeavyEdgeBlock, 0, s>>>(g->fwd, heavy_list, nheavy, g->tl_off, g->tl, g->pe);
-    ktime_end(g, KT_TRI_FILL);
-    ktime_begin(g, KT_VERTEX_FOLD);
     double* terms = nullptr;
     if (kSlotsPerTerm * tl_len >= m2 && tl_len > 0) {
         terms = (double*)sc.get(sizeof(double) * (size_t)tl_len);
         if (!terms) cudaGetLastError();  // no room: the folds read the lists
     }
+    const bool ahead = terms && (unsigned)words[1] >= kAheadEdges;
+    cudaStream_t hs = s;  // the heavy lists'
+    ktime_begin(g, KT_TRI_FILL);
+    // cnt (scanned into tl_off above) is free: it takes the terms' offsets
+    if (terms) exclusive_scan_i64(cgt, cnt, m2 + 1, nullptr, tmp, s);
+    auto gather = [&](int lo, int hi, cudaStream_t st) {
+        k_fold_gather<<<grid_for(8 * m2, kBlock), kBlock, 0, st>>>(g->esrc, g->nbors, g->partner, g->deg, lo, hi, m2,
+                                                                   cgt, cnt, g->tl_off, g->tl, terms);
+    };
+    auto fold = [&](int lo, int hi, cudaStream_t st) {
+        k_fold_terms_heavy<<<grid_for(1ll << 40, kHeavyBlock, 16), kHeavyBlock, 0, st>>>(g->offsets, cnt, n, lo, hi,
+                                                                                         terms, g->pv);
+    };
+    const int top = INT32_MAX, cut = ahead ? g->tune_edge : top;
+    cudaEvent_t filled = nullptr;
+    if (ahead) {
+        if (!g->side) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking));
+        hs = g->side;
+        RTR_CUDA_TRY(cudaEventCreateWithFlags(&filled, cudaEventDisableTiming));
+        side_guard.lists = filled;
+        RTR_CUDA_TRY(cudaEventRecord(filled, s));
+        RTR_CUDA_TRY(cudaStreamWaitEvent(hs, filled, 0));
+    }
+    if (heavy)
+        k_tri_fill_heavy<<<gh, kHeavyEdgeBlock, 0, hs>>>(g->offsets, g->nbors, g->esrc, g->deg, g->partner, g->fwd,
+                                                         g->frank, heavy_list, nheavy, g->tune_gallop, parts,
+                                                         ha.nparts, g->tl_off, g->tl, hq);
+    if (ahead) {
+        RTR_CUDA_TRY(cudaEventRecord(filled, hs));
+        gather(cut, top, hs);
+        fold(cut, top, hs);
+        g->launches += 2;
+    }
+    k_tri_fill<<<ge, kBlock, 0, s>>>(g->offsets, g->nbors, g->esrc, g->deg, g->partner, g->fwd, g->frank, m,
+                                     g->tl_off, g->tl, g->tune_gallop, g->tune_edge);
+    if (ahead) RTR_CUDA_TRY(cudaStreamWaitEvent(s, filled, 0));
+    if (heavy) k_pe_fold_heavy<<<gh, kHeavyEdgeBlock, 0, s>>>(g->fwd, heavy_list, nheavy, g->tl_off, g->tl, g->pe);
+    ktime_end(g, KT_TRI_FILL);
+    ktime_begin(g, KT_VERTEX_FOLD);
     if (terms) {
-        // cnt (scanned into tl_off above) is free: it takes the terms' offsets
-        exclusive_scan_i64(cgt, cnt, m2 + 1, nullptr, tmp, s);
-        k_fold_gather<<<grid_for(8 * m2, kBlock), kBlock, 0, s>>>(g->esrc, g->nbors, g->partner, m2, cgt, cnt,
-                                                                  g->tl_off, g->tl, terms);
-        k_fold_terms_light<<<grid_for(n, kBlock), kBlock, 0, s>>>(g->offsets, cnt, n, terms, g->pv);
-        k_fold_terms_heavy<<<grid_for(1ll << 40, kHeavyBlock, 16), kHeavyBlock, 0, s>>>(g->offsets, cnt, n, terms,
-                                                                                        g->pv);
+        gather(0, cut, s);
+        k_fold_terms_light<<<grid_for(n, kBlock), kBlock, 0, s>>>(g->offsets, cnt, n, cut, terms, g->pv);
+        fold(0, cut, s);
+        if (ahead) {
+            RTR_CUDA_TRY(cudaEventRecord(filled, hs));
+            RTR_CUDA_TRY(cudaStreamWaitEvent(s, filled, 0));
+        }
         g->launches += 3 + take_primitive_launches();
     } else {
         k_vertex_fold_light<<<grid_for(n, kBlock), kBlock, 0, s>>>(g->offsets, g->nbors, g->deg, g->partner, n, cgt,
