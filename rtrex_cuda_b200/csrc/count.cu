@@ -145,6 +145,11 @@ constexpr int kHeavyEdgeBlock = 128;
 // intersect twice (R-MAT, 500,000 edges: 1.43 -> 0.92 ms); 64 bytes an edge, in 16
 // bits, so edges of more triangles than kPartsMax are intersected twice all the same.
 constexpr int64_t kPartsMax = 65535;
+// Edges from which the host learns the number of heavy ones first (15 us) and
+// allocates no more than they need: half of 926,000 edges' notes were 30 MB that a
+// graph of 2,500 heavy edges left unused, and made the pool map new memory now and
+// then (a new graph's pass 22 ms, but up to 50).
+constexpr int64_t kListFirst = 1ll << 18;
 
 struct HeavyArgs {
     const int64_t* off;
@@ -973,11 +978,21 @@ int count_triangles(rtr_graph* g)
                                           g->sup, cnt, cgt, g->ctr, g->tune_gallop, g->tune_edge, list, nheavy);
         ktime_end(g, KT_EDGE_LIGHT);
     };
-    if (rs.tab) {
+    int64_t nparts = 0;  // heavy edges noted for k_tri_fill_heavy
+    if (rs.tab || (!heavy_pe && m >= kListFirst)) {
         k_heavy_list<<<ge, kBlock, 0, s>>>(g->esrc, g->nbors, g->deg, g->fwd, m, g->tune_edge, heavy_list, nheavy);
         g->launches += 1;
     } else {
         light(heavy_list);
+    }
+    if (!rs.tab && !heavy_pe) {
+        nparts = m / 2 + 1;
+        if (m >= kListFirst) {
+            unsigned nh = 0;
+            if (const int rc = read_words(g, &nh, nheavy, sizeof nh)) return rc;
+            nparts = std::min<int64_t>(nparts, nh);
+            light(nullptr);
+        }
     }
     // the longest perVertex chains ahead of the rest, where the rows layout is likely.  Not when this
     // graph holds lists from an earlier count (they will be kept again), nor under a set window size
@@ -1069,12 +1084,12 @@ int count_triangles(rtr_graph* g)
     }
     ktime_begin(g, KT_EDGE_HEAVY);
     uint16_t* parts = nullptr;
-    if (!rs.tab && !heavy_pe) {
-        parts = (uint16_t*)sc.get(sizeof(uint16_t) * 32 * (size_t)(m / 2 + 1));
+    if (nparts > 0) {
+        parts = (uint16_t*)sc.get(sizeof(uint16_t) * 32 * (size_t)nparts);
         if (!parts) cudaGetLastError();  // no room: the fill intersects twice
     }
     const HeavyArgs ha{g->offsets, g->nbors, g->esrc, g->deg, g->fwd, g->partner, heavy_list, g->tune_gallop, rs, g->sup,
-                       cnt, cgt, heavy_pe ? g->pe : nullptr, g->ctr, moff, masks, parts, parts ? m / 2 + 1 : 0};
+                       cnt, cgt, heavy_pe ? g->pe : nullptr, g->ctr, moff, masks, parts, parts ? nparts : 0};
     if (pr.count > 0 && pr.edges > 0) {
         if (const int rc = launch_bits(g, ha, runs, pieces, np[0], hq + 2)) return rc;
         k_edge_count_heavy<<<gc, kHeavyEdgeBlock, 0, s>>>(ha, runs, 0, pr.edges, nheavy, hq);

@@ -43,3 +43,12 @@ def test_long_lists(pages):
     u = np.concatenate([[0], np.zeros(pages, np.int64), np.ones(pages, np.int64), 2 + 3 * r])
     v = np.concatenate([[1], p, p, 3 + 3 * r])
     _check(2 + pages, u.astype(np.int64), v.astype(np.int64), (1024, 1 << 30))
+
+
+@pytest.mark.parametrize("m", [(1 << 18) - 1, 1 << 18])
+def test_heavy_edges_counted_first(m):
+    """Around the number of edges from which the host asks for the heavy ones first: none, some, all."""
+    n, u, v = graphgen.rmat(scale=15, edge_factor=12, seed=5)
+    keep = np.sort(np.random.Generator(np.random.PCG64(m)).permutation(u.size)[:m])
+    assert keep.size == m
+    _check(n, u[keep], v[keep], (1, 300, 1024, 1 << 30))
