@@ -35,13 +35,13 @@
 // subtract each vertex's weights in that order.
 //
 // What bounds it: a round is one dependent chain (window, entries, records,
-// table, fold, commit; 4 barriers) of ~4,300 cycles, of which the memory is a
-// quarter and the rest instruction latency, and every item that pushes ends a
+// table, fold, commit; 4 barriers) of ~4,000 cycles, of which the memory is a
+// fifth and the rest instruction latency, and every item that pushes ends a
 // round.  On the 926,000-edge co-purchase graph (B200, eps 0.3) the giant
-// unit's 41,000 pops take 7,100 rounds, 15.4 ms; reserving cells and letting
+// unit's 41,000 pops take 7,100 rounds, 14.4 ms; reserving cells and letting
 // only conflict-free items commit (with the sequence as a linked list, ranked
 // afterwards) took 25.0 ms, one warp per unit 38.5 ms.  On the 203,311-edge R-MAT
-// graph (mean list 31) 162,000 pops take 39,600 rounds, 116 ms against 235 ms one
+// graph (mean list 31) 162,000 pops take 39,600 rounds, 111 ms against 235 ms one
 // warp per unit.  Measured and slower: a warp replaying single items from lists
 // brought into L1 by helper warps (19.7 / 203 ms), one thread per edge folding all
 // items' subtractions (18.9 / 148 ms), one warp walking the window's items in
@@ -130,6 +130,29 @@ __device__ __forceinline__ void load_state(const EdgeRec* p, EdgeRec& r)
 // A cut value: the window ends with item `last`, which pushes (2 * last) or
 // after which the later items may not be taken (2 * last + 1).
 __device__ __forceinline__ int cut_after(int last) { return 2 * (last > 0 ? last : 0) + 1; }
+
+// The first 16 entries of a list that a later round reads: into L1 as soon as an
+// edge is seen to fall (its push is likely the next round's first item), into L2
+// when a seed enters the ring.  Co-purchase graph 15.6 -> 14.8 with the first, 14.4
+// ms with both; R-MAT 203,311 edges 117.3 -> 112.5 -> 111.5, 40,000 20.3 -> 19.5 -> 19.5.
+// (Whole lists by bulk prefetch at the push: 112 and 15.2 ms, but 21.0 for 40,000
+// edges -- issuing one costs the round 200 cycles.  In k_clean_units, where one warp
+// issues everything, the same prefetches cost 3 to 11%.)
+constexpr int kTouch = 4;  // lines of 4 entries
+
+__device__ __forceinline__ void touch_list(const TriEntry* p, int32_t cnt)
+{
+#pragma unroll
+    for (int k = 0; k < kTouch; ++k)
+        if (4 * k < cnt) asm volatile("prefetch.global.L1 [%0];" ::"l"(p + 4 * k));
+}
+
+__device__ __forceinline__ void ask_list(const TriEntry* p, int32_t cnt)
+{
+#pragma unroll
+    for (int k = 0; k < kTouch; ++k)
+        if (4 * k < cnt) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 4 * k));
+}
 
 constexpr int kSpareBits = 7;
 __device__ __forceinline__ int spare_hash(unsigned cell) { return (int)((cell * 2654435761u) >> (32 - kSpareBits)); }
@@ -257,7 +280,10 @@ __global__ void __launch_bounds__(32 * NW) k_clean_rounds(RoundArgs a)
                 __syncthreads();
                 const int x = lane < NW ? S.wlive[lane] : 0;
                 const int below = __reduce_add_sync(kFull, lane < wid ? x : 0);
-                if (kept) S.ring[(bot - 1 - below - __popc(bal & lt)) & M] = se;
+                if (kept) {
+                    ask_list(a.tl + se.t0, se.cnt);
+                    S.ring[(bot - 1 - below - __popc(bal & lt)) & M] = se;
+                }
                 sp -= k;
                 bot -= __reduce_add_sync(kFull, x);
             }
@@ -450,6 +476,8 @@ __global__ void __launch_bounds__(32 * NW) k_clean_rounds(RoundArgs a)
             f1 = c1 != SS_S && x1 < r1.thr;
             f2 = c2 != SS_S && x2 < r2.thr;
             if ((f1 || f2) && 2 * item < cut) cut = 2 * item;
+            if (f1) touch_list(a.tl + a.rec[rlw].t0, (int32_t)r1.cnt);
+            if (f2) touch_list(a.tl + a.rec[rhw].t0, (int32_t)r2.cnt);
         }
         cut = __reduce_min_sync(kFull, cut);
         if (lane == 0 && cut < cut_after(W)) atomicMin(&S.cut[par], cut);
