@@ -16,6 +16,7 @@
 //   std::sort candidates        -> introsort restatement (stl_order.cuh)
 //   std::stack deletion stack   -> array stack
 // Cluster creation order is the global rank of each cluster's seed.
+#include "block_prims.cuh"
 #include "primitives.cuh"
 #include "rtr_graph.cuh"
 #include "stl_order.cuh"
@@ -48,20 +49,30 @@ __device__ __forceinline__ int64_t find_slot(const int64_t* __restrict__ off, co
     return -1;
 }
 
-__global__ void k_iota_key_deg(const int32_t* __restrict__ deg, int64_t n, int B, uint64_t* __restrict__ keys)
+__device__ __forceinline__ void iota_key_deg(const int32_t* deg, int64_t n, int B, uint64_t* keys)
 {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
         keys[v] = ((uint64_t)deg[v] << B) | (uint64_t)v;
 }
 
-__global__ void k_rank(const uint64_t* __restrict__ sorted, int64_t n, uint64_t mask, int32_t* __restrict__ rank,
-                       int32_t* __restrict__ by_rank)
+__global__ void k_iota_key_deg(const int32_t* __restrict__ deg, int64_t n, int B, uint64_t* __restrict__ keys)
+{
+    iota_key_deg(deg, n, B, keys);
+}
+
+__device__ __forceinline__ void set_rank(const uint64_t* sorted, int64_t n, uint64_t mask, int32_t* rank, int32_t* by_rank)
 {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
         const int32_t v = (int32_t)(sorted[j] & mask);
         rank[v] = (int32_t)j;
         by_rank[j] = v;
     }
+}
+
+__global__ void k_set_rank(const uint64_t* __restrict__ sorted, int64_t n, uint64_t mask, int32_t* __restrict__ rank,
+                       int32_t* __restrict__ by_rank)
+{
+    set_rank(sorted, n, mask, rank, by_rank);
 }
 
 __global__ void k_uf_init(int32_t* __restrict__ p, int64_t n)
@@ -97,21 +108,31 @@ __global__ void k_alive_count(const int32_t* __restrict__ esrc, const int32_t* _
     }
 }
 
-__global__ void k_comp_keys(const int32_t* __restrict__ root, const int32_t* __restrict__ rank, int64_t n, int R,
-                            uint64_t* __restrict__ keys)
+__device__ __forceinline__ void comp_keys(const int32_t* root, const int32_t* rank, int64_t n, int R, uint64_t* keys)
 {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
         keys[v] = ((uint64_t)root[v] << R) | (uint64_t)rank[v];
 }
 
-__global__ void k_comp_heads(const uint64_t* __restrict__ keys, int64_t n, int R, const int32_t* __restrict__ by_rank,
-                             uint32_t* __restrict__ head, int32_t* __restrict__ vlist)
+__global__ void k_comp_keys(const int32_t* __restrict__ root, const int32_t* __restrict__ rank, int64_t n, int R,
+                            uint64_t* __restrict__ keys)
+{
+    comp_keys(root, rank, n, R, keys);
+}
+
+__device__ __forceinline__ void comp_heads(const uint64_t* keys, int64_t n, int R, const int32_t* by_rank, uint32_t* head, int32_t* vlist)
 {
     const uint64_t mask = (1ull << R) - 1;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
         head[j] = (j == 0 || (keys[j] >> R) != (keys[j - 1] >> R)) ? 1u : 0u;
         vlist[j] = by_rank[keys[j] & mask];
     }
+}
+
+__global__ void k_comp_heads(const uint64_t* __restrict__ keys, int64_t n, int R, const int32_t* __restrict__ by_rank,
+                             uint32_t* __restrict__ head, int32_t* __restrict__ vlist)
+{
+    comp_heads(keys, n, R, by_rank, head, vlist);
 }
 
 struct CompDesc {
@@ -122,16 +143,19 @@ struct CompDesc {
     int64_t scap;
 };
 
-__global__ void k_comp_begin(const uint64_t* __restrict__ keys, int64_t n, int R, const uint32_t* __restrict__ head,
-                             const uint32_t* __restrict__ hpos, CompDesc* __restrict__ comps)
+__device__ __forceinline__ void comp_begin(const uint64_t* keys, int64_t n, int R, const uint32_t* head, const uint32_t* hpos, CompDesc* comps)
 {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x)
         if (head[j]) comps[hpos[j]].vbegin = j;
 }
 
-__global__ void k_comp_sizes(CompDesc* __restrict__ comps, int64_t nc, int64_t n, const uint64_t* __restrict__ keys,
-                             int R, const uint32_t* __restrict__ acount, int64_t* __restrict__ bneed,
-                             int64_t* __restrict__ sneed)
+__global__ void k_comp_begin(const uint64_t* __restrict__ keys, int64_t n, int R, const uint32_t* __restrict__ head,
+                             const uint32_t* __restrict__ hpos, CompDesc* __restrict__ comps)
+{
+    comp_begin(keys, n, R, head, hpos, comps);
+}
+
+__device__ __forceinline__ void comp_sizes(CompDesc* comps, int64_t nc, int64_t n, const uint64_t* keys, int R, const uint32_t* acount, int64_t* bneed, int64_t* sneed)
 {
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
         const int64_t b = comps[c].vbegin;
@@ -142,9 +166,14 @@ __global__ void k_comp_sizes(CompDesc* __restrict__ comps, int64_t nc, int64_t n
     }
 }
 
-__global__ void k_comp_finish(CompDesc* __restrict__ comps, int64_t nc, const int64_t* __restrict__ boff,
-                              const int64_t* __restrict__ soff, const int64_t* __restrict__ sneed,
-                              uint64_t* __restrict__ order_keys, int64_t big_thr)
+__global__ void k_comp_sizes(CompDesc* __restrict__ comps, int64_t nc, int64_t n, const uint64_t* __restrict__ keys,
+                             int R, const uint32_t* __restrict__ acount, int64_t* __restrict__ bneed,
+                             int64_t* __restrict__ sneed)
+{
+    comp_sizes(comps, nc, n, keys, R, acount, bneed, sneed);
+}
+
+__device__ __forceinline__ void comp_finish(CompDesc* comps, int64_t nc, const int64_t* boff, const int64_t* soff, const int64_t* sneed, uint64_t* order_keys, int64_t big_thr)
 {
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
         comps[c].bbase = boff[c];
@@ -157,6 +186,87 @@ __global__ void k_comp_finish(CompDesc* __restrict__ comps, int64_t nc, const in
         const uint64_t small = comps[c].vcount >= big_thr ? 0u : 1u;
         order_keys[c] = (small << 63) | ((uint64_t)(0x7fffffffu - (uint32_t)w) << 32) | (uint64_t)c;
     }
+}
+
+__global__ void k_comp_finish(CompDesc* __restrict__ comps, int64_t nc, const int64_t* __restrict__ boff,
+                              const int64_t* __restrict__ soff, const int64_t* __restrict__ sneed,
+                              uint64_t* __restrict__ order_keys, int64_t big_thr)
+{
+    comp_finish(comps, nc, boff, soff, sneed, order_keys, big_thr);
+}
+
+// Components of at least `thr` vertices (the block kernel's) and the largest vertex count among them.
+__device__ __forceinline__ void big_count(const CompDesc* comps, int64_t nc, int64_t thr, unsigned* nbig, unsigned long long* maxv)
+{
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x)
+        if (comps[c].vcount >= thr) {
+            atomicAdd(nbig, 1u);
+            atomicMax(maxv, (unsigned long long)comps[c].vcount);
+        }
+}
+
+__global__ void k_big_count(const CompDesc* __restrict__ comps, int64_t nc, int64_t thr, unsigned* __restrict__ nbig,
+                            unsigned long long* __restrict__ maxv)
+{
+    big_count(comps, nc, thr, nbig, maxv);
+}
+
+// Up to kSmallSetup vertices: the set-up of the extraction in two launches of one
+// block around the union-find over the edges, instead of 16 and a wait.
+//   1,003 edges: the extraction but its replay 0.22 -> 0.11 ms, 20,000 0.28 -> 0.17, 60,000 0.36 -> 0.30.
+constexpr int64_t kSmallSetup = kSortOne;
+
+__global__ void __launch_bounds__(kOneBlock) k_order_small(const int32_t* deg, int64_t n, int B, int bits, uint64_t* k1,
+                                                         uint64_t* k2, int32_t* rank, int32_t* by_rank, int32_t* root,
+                                                         uint32_t* acount)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    iota_key_deg(deg, n, B, k1);
+    for (int64_t v = threadIdx.x; v <= n; v += blockDim.x) {
+        acount[v] = 0;
+        if (v < n) root[v] = (int32_t)v;
+    }
+    __syncthreads();
+    sort_one(*reinterpret_cast<SortOneSmem*>(smem_raw), k1, k2, (int)n, 0, bits);
+    __syncthreads();
+    set_rank(k2, n, (1ull << B) - 1, rank, by_rank);
+}
+
+// out: the components, and what the host sizes its buffers by (bucket and stack
+// entries, big components and the largest one's vertices).
+__global__ void __launch_bounds__(kOneBlock)
+    k_comps_small(const int32_t* root, const int32_t* rank, const int32_t* by_rank, int64_t n, int B,
+                  const uint32_t* acount, int64_t big_thr, uint64_t* k1, uint64_t* k2, uint32_t* head, uint32_t* hpos,
+                  int32_t* vlist, CompDesc* comps, int64_t* bneed, int64_t* sneed, int64_t* boff, int64_t* soff,
+                  uint64_t* okeys, uint64_t* order, int64_t* out)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SortOneSmem& S = *reinterpret_cast<SortOneSmem*>(smem_raw);
+    __shared__ uint32_t s_warp32[32], s_nc;
+    __shared__ int64_t s_warp64[32];
+    if (threadIdx.x < 5) out[threadIdx.x] = 0;
+    comp_keys(root, rank, n, B, k1);
+    __syncthreads();
+    sort_one(S, k1, k2, (int)n, 0, 2 * B);
+    __syncthreads();
+    comp_heads(k2, n, B, by_rank, head, vlist);
+    __syncthreads();
+    scan_one(head, hpos, (int)n, &s_nc, s_warp32);
+    __syncthreads();
+    const int nc = (int)s_nc;
+    comp_begin(k2, n, B, head, hpos, comps);
+    __syncthreads();
+    comp_sizes(comps, nc, n, k2, B, acount, bneed, sneed);
+    __syncthreads();
+    big_count(comps, nc, big_thr, (unsigned*)(out + 3), (unsigned long long*)(out + 4));
+    scan_one(bneed, boff, nc, out + 1, s_warp64);
+    __syncthreads();
+    scan_one(sneed, soff, nc, out + 2, s_warp64);
+    __syncthreads();
+    comp_finish(comps, nc, boff, soff, sneed, okeys, big_thr);
+    __syncthreads();
+    sort_one(S, okeys, order, nc, 32, 64);
+    if (threadIdx.x == 0) out[0] = nc;
 }
 
 struct Cand {
@@ -825,9 +935,7 @@ __global__ void __launch_bounds__(kBigBlock) k_extract_big(ExtractArgs a, const 
     }
 }
 
-__global__ void k_cluster_keys(const CompDesc* __restrict__ comps, int64_t nc, const int32_t* __restrict__ ncl,
-                               const int64_t* __restrict__ cpos, const int32_t* __restrict__ hdr_seed,
-                               const int32_t* __restrict__ rank, int B, uint64_t* __restrict__ keys)
+__device__ __forceinline__ void cluster_keys(const CompDesc* comps, int64_t nc, const int32_t* ncl, const int64_t* cpos, const int32_t* hdr_seed, const int32_t* rank, int B, uint64_t* keys)
 {
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
         const int64_t vb = comps[c].vbegin;
@@ -836,9 +944,14 @@ __global__ void k_cluster_keys(const CompDesc* __restrict__ comps, int64_t nc, c
     }
 }
 
-__global__ void k_cluster_gather(const uint64_t* __restrict__ sorted, int64_t ncl, uint64_t mask,
-                                 const int32_t* __restrict__ hdr_seed, const int32_t* __restrict__ hdr_size,
-                                 int32_t* __restrict__ cl_seed, int64_t* __restrict__ size64)
+__global__ void k_cluster_keys(const CompDesc* __restrict__ comps, int64_t nc, const int32_t* __restrict__ ncl,
+                               const int64_t* __restrict__ cpos, const int32_t* __restrict__ hdr_seed,
+                               const int32_t* __restrict__ rank, int B, uint64_t* __restrict__ keys)
+{
+    cluster_keys(comps, nc, ncl, cpos, hdr_seed, rank, B, keys);
+}
+
+__device__ __forceinline__ void cluster_gather(const uint64_t* sorted, int64_t ncl, uint64_t mask, const int32_t* hdr_seed, const int32_t* hdr_size, int32_t* cl_seed, int64_t* size64)
 {
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ncl; g += (int64_t)gridDim.x * blockDim.x) {
         const int64_t h = (int64_t)(sorted[g] & mask);
@@ -847,10 +960,14 @@ __global__ void k_cluster_gather(const uint64_t* __restrict__ sorted, int64_t nc
     }
 }
 
-__global__ void k_cluster_members(const uint64_t* __restrict__ sorted, int64_t ncl, int64_t n, uint64_t mask,
-                                  const int64_t* __restrict__ hdr_start, const int64_t* __restrict__ cl_off,
-                                  const int32_t* __restrict__ out_vert, int32_t* __restrict__ cl_vert,
-                                  int32_t* __restrict__ cluster_of)
+__global__ void k_cluster_gather(const uint64_t* __restrict__ sorted, int64_t ncl, uint64_t mask,
+                                 const int32_t* __restrict__ hdr_seed, const int32_t* __restrict__ hdr_size,
+                                 int32_t* __restrict__ cl_seed, int64_t* __restrict__ size64)
+{
+    cluster_gather(sorted, ncl, mask, hdr_seed, hdr_size, cl_seed, size64);
+}
+
+__device__ __forceinline__ void cluster_members(const uint64_t* sorted, int64_t ncl, int64_t n, uint64_t mask, const int64_t* hdr_start, const int64_t* cl_off, const int32_t* out_vert, int32_t* cl_vert, int32_t* cluster_of)
 {
     if (cl_off[ncl] != n) return;  // reported by the host
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ncl; g += (int64_t)gridDim.x * blockDim.x) {
@@ -861,6 +978,62 @@ __global__ void k_cluster_members(const uint64_t* __restrict__ sorted, int64_t n
             cl_vert[p] = v;
             cluster_of[v] = (int32_t)g;
         }
+    }
+}
+
+__global__ void k_cluster_members(const uint64_t* __restrict__ sorted, int64_t ncl, int64_t n, uint64_t mask,
+                                  const int64_t* __restrict__ hdr_start, const int64_t* __restrict__ cl_off,
+                                  const int32_t* __restrict__ out_vert, int32_t* __restrict__ cl_vert,
+                                  int32_t* __restrict__ cluster_of)
+{
+    cluster_members(sorted, ncl, n, mask, hdr_start, cl_off, out_vert, cl_vert, cluster_of);
+}
+
+__device__ __forceinline__ void widen(const int32_t* in, int64_t* out, int64_t k)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < k; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = in[i];
+}
+
+__global__ void k_widen(const int32_t* __restrict__ in, int64_t* __restrict__ out, int64_t k)
+{
+    widen(in, out, k);
+}
+
+// The set-up's size rule again: the clusters in creation order, their seeds, offsets
+// and members in one block's launch instead of eight.  out: the clusters and their
+// members, both 0 when the extraction failed.
+__global__ void __launch_bounds__(kOneBlock)
+    k_clusters_small(const unsigned* err, const CompDesc* comps, int nc, int64_t n, const int32_t* ncl, int B,
+                     const int32_t* rank, const int32_t* hdr_seed, const int64_t* hdr_start, const int32_t* hdr_size,
+                     const int32_t* out_vert, int64_t* ncl64, int64_t* cpos, uint64_t* keys, uint64_t* sorted,
+                     int64_t* size64, int32_t* cl_seed, int64_t* cl_off, int64_t* cl_ne, int64_t* cl_cut,
+                     int32_t* cl_vert, int32_t* cluster_of, int64_t* out)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int64_t s_warp[32], s_total;
+    if (*err) return;
+    widen(ncl, ncl64, nc);
+    __syncthreads();
+    scan_one(ncl64, cpos, nc, &s_total, s_warp);
+    __syncthreads();
+    const int64_t k = s_total;
+    if (k > n) return;  // reported by the host
+    const uint64_t mask = (1ull << B) - 1;
+    cluster_keys(comps, nc, ncl, cpos, hdr_seed, rank, B, keys);
+    __syncthreads();
+    sort_one(*reinterpret_cast<SortOneSmem*>(smem_raw), keys, sorted, (int)k, 0, 2 * B);
+    __syncthreads();
+    cluster_gather(sorted, k, mask, hdr_seed, hdr_size, cl_seed, size64);
+    if (threadIdx.x == 0) size64[k] = 0;
+    for (int64_t c = threadIdx.x; c <= k; c += blockDim.x) cl_ne[c] = cl_cut[c] = 0;
+    __syncthreads();
+    scan_one(size64, cl_off, (int)k + 1, &s_total, s_warp);
+    __syncthreads();
+    cluster_members(sorted, k, n, mask, hdr_start, cl_off, out_vert, cl_vert, cluster_of);
+    if (threadIdx.x == 0) {
+        out[0] = k;
+        out[1] = s_total;
     }
 }
 
@@ -882,28 +1055,10 @@ __global__ void k_cluster_stats(const int64_t* __restrict__ off, const int32_t* 
     }
 }
 
-__global__ void k_widen(const int32_t* __restrict__ in, int64_t* __restrict__ out, int64_t k)
+// Internal edges were counted from both ends.
+__global__ void k_halve(int64_t* __restrict__ ne, const int64_t* __restrict__ clusters)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < k; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = in[i];
-}
-
-// Components of at least `thr` vertices (the block kernel's) and the largest vertex count among them.
-__global__ void k_big_count(const CompDesc* __restrict__ comps, int64_t nc, int64_t thr, unsigned* __restrict__ nbig,
-                            unsigned long long* __restrict__ maxv)
-{
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x)
-        if (comps[c].vcount >= thr) {
-            atomicAdd(nbig, 1u);
-            atomicMax(maxv, (unsigned long long)comps[c].vcount);
-        }
-}
-
-// Internal edges were counted from both ends; `members` takes the cluster sizes' sum.
-__global__ void k_halve(int64_t* __restrict__ ne, int64_t ncl, const int64_t* __restrict__ off,
-                        unsigned long long* __restrict__ members)
-{
-    if (blockIdx.x == 0 && threadIdx.x == 0) *members = (unsigned long long)off[ncl];
+    const int64_t ncl = *clusters;
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ncl; g += (int64_t)gridDim.x * blockDim.x)
         ne[g] /= 2;
 }
@@ -947,7 +1102,7 @@ int extract_clusters(rtr_graph* g)
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
-    RTR_CUDA_TRY(cudaMemsetAsync(g->ctr + 1, 0, 2 * sizeof(unsigned long long), s));
+    RTR_CUDA_TRY(cudaMemsetAsync(g->ctr + 1, 0, 5 * sizeof(unsigned long long), s));
 
     const int B = bits_for((uint64_t)(n - 1));
     const uint64_t bmask = (1ull << B) - 1;
@@ -970,33 +1125,49 @@ int extract_clusters(rtr_graph* g)
         set_error("device allocation failed (extract setup)");
         return RTR_ERR_CUDA;
     }
-    k_iota_key_deg<<<gn, kBlock, 0, s>>>(g->deg, n, B, k1);
-    uint64_t* sorted = radix_sort_u64(k1, k2, n, B + bits_for((uint64_t)m2), rtmp, s);
-    k_rank<<<gn, kBlock, 0, s>>>(sorted, n, bmask, rank, by_rank);
+    const bool small = n <= kSmallSetup;
+    const int dbits = B + bits_for((uint64_t)m2);
+    uint64_t* sorted = k2;
+    if (small) {
+        RTR_CUDA_TRY(cudaFuncSetAttribute(k_order_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)sizeof(SortOneSmem)));
+        k_order_small<<<1, kOneBlock, sizeof(SortOneSmem), s>>>(g->deg, n, B, dbits, k1, k2, rank, by_rank, root,
+                                                                acount);
+        g->launches += 1;
+    } else {
+        k_iota_key_deg<<<gn, kBlock, 0, s>>>(g->deg, n, B, k1);
+        sorted = radix_sort_u64(k1, k2, n, dbits, rtmp, s);
+        k_set_rank<<<gn, kBlock, 0, s>>>(sorted, n, bmask, rank, by_rank);
+        k_uf_init<<<gn, kBlock, 0, s>>>(root, n);
+        RTR_CUDA_TRY(cudaMemsetAsync(acount, 0, sizeof(uint32_t) * (n + 1), s));
+        g->launches += 3 + take_primitive_launches();
+    }
     // components of the alive graph
-    k_uf_init<<<gn, kBlock, 0, s>>>(root, n);
     k_uf_hook_alive<<<gm, kBlock, 0, s>>>(g->esrc, g->nbors, g->fwd, m, g->st, root);
     k_uf_flatten<<<gn, kBlock, 0, s>>>(root, n);
-    RTR_CUDA_TRY(cudaMemsetAsync(acount, 0, sizeof(uint32_t) * (n + 1), s));
     k_alive_count<<<gm, kBlock, 0, s>>>(g->esrc, g->fwd, m, g->st, root, acount);
-    k_comp_keys<<<gn, kBlock, 0, s>>>(root, rank, n, B, k1 == sorted ? k2 : k1);
-    uint64_t* ck = (k1 == sorted) ? k2 : k1;
-    uint64_t* calt = sorted;  // rank/by_rank already captured; reuse as ping-pong
-    uint64_t* csorted = radix_sort_u64(ck, calt, n, 2 * B, rtmp, s);
-    k_comp_heads<<<gn, kBlock, 0, s>>>(csorted, n, B, by_rank, head, vlist);
-    exclusive_scan_u32(head, hpos, n, d_nc, htmp, s);
-    g->launches += 8 + take_primitive_launches();
-    RTR_CUDA_TRY(cudaGetLastError());
-    uint32_t nc = 0;
-    if (const int rc = read_words(g, &nc, d_nc, sizeof(uint32_t))) return rc;
+    g->launches += 3;
+    uint64_t* csorted = k2;
+    uint32_t nc = small ? (uint32_t)n : 0;  // the buffers' bound, then the number
+    if (!small) {
+        k_comp_keys<<<gn, kBlock, 0, s>>>(root, rank, n, B, k1 == sorted ? k2 : k1);
+        uint64_t* ck = (k1 == sorted) ? k2 : k1;
+        uint64_t* calt = sorted;  // rank/by_rank already captured; reuse as ping-pong
+        csorted = radix_sort_u64(ck, calt, n, 2 * B, rtmp, s);
+        k_comp_heads<<<gn, kBlock, 0, s>>>(csorted, n, B, by_rank, head, vlist);
+        exclusive_scan_u32(head, hpos, n, d_nc, htmp, s);
+        g->launches += 2 + take_primitive_launches();
+        RTR_CUDA_TRY(cudaGetLastError());
+        if (const int rc = read_words(g, &nc, d_nc, sizeof(uint32_t))) return rc;
+    }
 
     CompDesc* comps = (CompDesc*)sc.get(sizeof(CompDesc) * (nc + 1));
     int64_t* bneed = (int64_t*)sc.get(sizeof(int64_t) * (nc + 1));
     int64_t* sneed = (int64_t*)sc.get(sizeof(int64_t) * (nc + 1));
     int64_t* boff = (int64_t*)sc.get(sizeof(int64_t) * (nc + 1));
     int64_t* soff = (int64_t*)sc.get(sizeof(int64_t) * (nc + 1));
-    int64_t* ltmp = (int64_t*)sc.get(sizeof(int64_t) * scan_temp_elems(nc + 1));
-    int64_t* d_tot = (int64_t*)sc.get(sizeof(int64_t) * 4);  // buckets, stack entries, big components, the largest
+    int64_t* ltmp = (int64_t*)sc.get(sizeof(int64_t) * scan_temp_elems(n + 1));
+    int64_t* d_tot = (int64_t*)sc.get(sizeof(int64_t) * 5);  // components, then as in k_comps_small
     uint64_t* okeys = (uint64_t*)sc.get(sizeof(uint64_t) * (nc + 1));
     uint64_t* oalt = (uint64_t*)sc.get(sizeof(uint64_t) * (nc + 1));
     void* otmp = sc.get(radix_temp_bytes(nc));
@@ -1004,20 +1175,34 @@ int extract_clusters(rtr_graph* g)
         set_error("device allocation failed (extract components)");
         return RTR_ERR_CUDA;
     }
-    k_comp_begin<<<gn, kBlock, 0, s>>>(csorted, n, B, head, hpos, comps);
+    uint64_t* order = oalt;
+    int64_t tots[5] = {0, 0, 0, 0, 0};
+    if (small) {
+        RTR_CUDA_TRY(cudaFuncSetAttribute(k_comps_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)sizeof(SortOneSmem)));
+        k_comps_small<<<1, kOneBlock, sizeof(SortOneSmem), s>>>(root, rank, by_rank, n, B, acount, g->extract_big, k1,
+                                                                k2, head, hpos, vlist, comps, bneed, sneed, boff, soff,
+                                                                okeys, oalt, d_tot);
+        g->launches += 1;
+        RTR_CUDA_TRY(cudaGetLastError());
+        if (const int rc = read_words(g, tots, d_tot, sizeof tots)) return rc;
+        nc = (uint32_t)tots[0];
+    }
     const int gc = grid_for(nc, kBlock);
-    k_comp_sizes<<<gc, kBlock, 0, s>>>(comps, nc, n, csorted, B, acount, bneed, sneed);
-    RTR_CUDA_TRY(cudaMemsetAsync(d_tot + 2, 0, sizeof(int64_t) * 2, s));
-    k_big_count<<<gc, kBlock, 0, s>>>(comps, nc, g->extract_big, (unsigned*)(d_tot + 2),
-                                      (unsigned long long*)(d_tot + 3));
-    exclusive_scan_i64(bneed, boff, nc, d_tot, ltmp, s);
-    exclusive_scan_i64(sneed, soff, nc, d_tot + 1, ltmp, s);
-    k_comp_finish<<<gc, kBlock, 0, s>>>(comps, nc, boff, soff, sneed, okeys, g->extract_big);
-    // components ascend in the keys' low half already
-    uint64_t* order = radix_sort_bits_u64(okeys, oalt, nc, 32, 64, otmp, s);
-    g->launches += 4 + take_primitive_launches();
-    int64_t tots[4] = {0, 0, 0, 0};
-    if (const int rc = read_words(g, tots, d_tot, sizeof tots)) return rc;
+    if (!small) {
+        k_comp_begin<<<gn, kBlock, 0, s>>>(csorted, n, B, head, hpos, comps);
+        k_comp_sizes<<<gc, kBlock, 0, s>>>(comps, nc, n, csorted, B, acount, bneed, sneed);
+        RTR_CUDA_TRY(cudaMemsetAsync(d_tot, 0, sizeof(int64_t) * 5, s));
+        k_big_count<<<gc, kBlock, 0, s>>>(comps, nc, g->extract_big, (unsigned*)(d_tot + 3),
+                                          (unsigned long long*)(d_tot + 4));
+        exclusive_scan_i64(bneed, boff, nc, d_tot + 1, ltmp, s);
+        exclusive_scan_i64(sneed, soff, nc, d_tot + 2, ltmp, s);
+        k_comp_finish<<<gc, kBlock, 0, s>>>(comps, nc, boff, soff, sneed, okeys, g->extract_big);
+        // components ascend in the keys' low half already
+        order = radix_sort_bits_u64(okeys, oalt, nc, 32, 64, otmp, s);
+        g->launches += 4 + take_primitive_launches();
+        if (const int rc = read_words(g, tots, d_tot, sizeof tots)) return rc;
+    }
 
     ExtractArgs a;
     a.vbase = g->vbase;
@@ -1041,10 +1226,10 @@ int extract_clusters(rtr_graph* g)
     a.triwgt = (double*)sc.get(sizeof(double) * (n + 1));
     a.ukey = (int32_t*)sc.get(sizeof(int32_t) * (n + 1));
     a.unext = (int32_t*)sc.get(sizeof(int32_t) * (n + 1));
-    a.ubucket = (int32_t*)sc.get(sizeof(int32_t) * (tots[0] + 1));
+    a.ubucket = (int32_t*)sc.get(sizeof(int32_t) * (tots[1] + 1));
     a.twohop = (int32_t*)sc.get(sizeof(int32_t) * (n + 1));
     a.cand = (Cand*)sc.get(sizeof(Cand) * (n + 1));
-    a.dstack = (DelEntry*)sc.get(sizeof(DelEntry) * (tots[1] + 1));
+    a.dstack = (DelEntry*)sc.get(sizeof(DelEntry) * (tots[2] + 1));
     a.hdr_seed = (int32_t*)sc.get(sizeof(int32_t) * (n + 1));
     a.hdr_start = (int64_t*)sc.get(sizeof(int64_t) * (n + 1));
     a.hdr_size = (int32_t*)sc.get(sizeof(int32_t) * (n + 1));
@@ -1066,8 +1251,8 @@ int extract_clusters(rtr_graph* g)
     RTR_CUDA_TRY(cudaMemsetAsync(next_comp, 0, sizeof(unsigned) * 2, s));
     // components of at least extract_big vertices: a thread block each, on the side
     // stream while the others (if any) take a warp each here
-    const unsigned nbig = (unsigned)tots[2];
-    const int64_t maxv = tots[3], warps = (int64_t)nc - nbig;
+    const unsigned nbig = (unsigned)tots[3];
+    const int64_t maxv = tots[4], warps = (int64_t)nc - nbig;
     ktime_begin(g, KT_EXTRACT);
     SideJoin side_join;  // an early return waits for the side stream before scratch is freed
     if (nbig > 0) {
@@ -1115,16 +1300,21 @@ int extract_clusters(rtr_graph* g)
         set_error("device allocation failed (cluster order)");
         return RTR_ERR_CUDA;
     }
-    k_widen<<<gc, kBlock, 0, s>>>(a.ncl, ncl64, nc);
-    exclusive_scan_i64(ncl64, cpos, nc, (int64_t*)(g->ctr + 4), ltmp, s);
-    unsigned long long h[5];
-    if (const int rc = read_words(g, h, g->ctr, sizeof h, true)) return rc;
-    if (h[1] != 0) {
+    unsigned long long h[6];
+    auto failed = [&]() {
+        if (h[1] == 0) return false;
         set_error("device error word 0x%llx during extraction", h[1]);
-        return RTR_ERR_DEVICE;
+        return true;
+    };
+    int64_t ncl = n;  // the buffers' bound, then the number
+    if (!small) {
+        k_widen<<<gc, kBlock, 0, s>>>(a.ncl, ncl64, nc);
+        exclusive_scan_i64(ncl64, cpos, nc, (int64_t*)(g->ctr + 4), ltmp, s);
+        g->launches += 1 + take_primitive_launches();
+        if (const int rc = read_words(g, h, g->ctr, sizeof h, true)) return rc;
+        if (failed()) return RTR_ERR_DEVICE;
+        ncl = (int64_t)h[4];
     }
-    g->diag_residual += (long long)h[2];
-    const int64_t ncl = (int64_t)h[4];
     uint64_t* ckeys = (uint64_t*)sc.get(sizeof(uint64_t) * (ncl + 1));
     uint64_t* calt2 = (uint64_t*)sc.get(sizeof(uint64_t) * (ncl + 1));
     void* ctmp = sc.get(radix_temp_bytes(ncl));
@@ -1133,11 +1323,12 @@ int extract_clusters(rtr_graph* g)
         set_error("device allocation failed (cluster keys)");
         return RTR_ERR_CUDA;
     }
-    if (!g->cl_seed || g->ncl < ncl) {
+    if (!g->cl_seed || g->cl_cap < ncl) {
         g->cl_seed = (int32_t*)dev_alloc(g, sizeof(int32_t) * (ncl + 1));
         g->cl_off = (int64_t*)dev_alloc(g, sizeof(int64_t) * (ncl + 2));
         g->cl_ne = (int64_t*)dev_alloc(g, sizeof(int64_t) * (ncl + 1));
         g->cl_cut = (int64_t*)dev_alloc(g, sizeof(int64_t) * (ncl + 1));
+        g->cl_cap = ncl;
     }
     if (!g->cl_vert) {
         g->cl_vert = (int32_t*)dev_alloc(g, sizeof(int32_t) * (n + 1));
@@ -1147,34 +1338,46 @@ int extract_clusters(rtr_graph* g)
         set_error("device allocation failed (cluster outputs)");
         return RTR_ERR_CUDA;
     }
-    g->ncl = ncl;
-    RTR_CUDA_TRY(cudaMemsetAsync(size64, 0, sizeof(int64_t) * (ncl + 1), s));
-    k_cluster_keys<<<gc, kBlock, 0, s>>>(comps, nc, a.ncl, cpos, a.hdr_seed, rank, B, ckeys);
-    uint64_t* csort = radix_sort_u64(ckeys, calt2, ncl, 2 * B, ctmp, s);
     const int gk = grid_for(ncl, kBlock);
-    k_cluster_gather<<<gk, kBlock, 0, s>>>(csort, ncl, bmask, a.hdr_seed, a.hdr_size, g->cl_seed, size64);
-    exclusive_scan_i64(size64, g->cl_off, ncl + 1, nullptr, ltmp, s);
-    k_cluster_members<<<gk, kBlock, 0, s>>>(csort, ncl, n, bmask, a.hdr_start, g->cl_off, a.out_vert, g->cl_vert,
-                                            g->cluster_of);
-    RTR_CUDA_TRY(cudaMemsetAsync(g->cl_ne, 0, sizeof(int64_t) * (ncl + 1), s));
-    RTR_CUDA_TRY(cudaMemsetAsync(g->cl_cut, 0, sizeof(int64_t) * (ncl + 1), s));
-    k_cluster_stats<<<gn, kBlock, 0, s>>>(g->offsets, g->nbors, n, g->cluster_of, g->cl_off + ncl,
+    int64_t* counts = (int64_t*)(g->ctr + 4);  // the clusters, their members
+    if (small) {
+        RTR_CUDA_TRY(cudaFuncSetAttribute(k_clusters_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)sizeof(SortOneSmem)));
+        k_clusters_small<<<1, kOneBlock, sizeof(SortOneSmem), s>>>(
+            a.err, comps, (int)nc, n, a.ncl, B, rank, a.hdr_seed, a.hdr_start, a.hdr_size, a.out_vert, ncl64, cpos, ckeys,
+            calt2, size64, g->cl_seed, g->cl_off, g->cl_ne, g->cl_cut, g->cl_vert, g->cluster_of, counts);
+        g->launches += 1;
+    } else {
+        RTR_CUDA_TRY(cudaMemsetAsync(size64, 0, sizeof(int64_t) * (ncl + 1), s));
+        k_cluster_keys<<<gc, kBlock, 0, s>>>(comps, nc, a.ncl, cpos, a.hdr_seed, rank, B, ckeys);
+        uint64_t* csort = radix_sort_u64(ckeys, calt2, ncl, 2 * B, ctmp, s);
+        k_cluster_gather<<<gk, kBlock, 0, s>>>(csort, ncl, bmask, a.hdr_seed, a.hdr_size, g->cl_seed, size64);
+        exclusive_scan_i64(size64, g->cl_off, ncl + 1, counts + 1, ltmp, s);
+        k_cluster_members<<<gk, kBlock, 0, s>>>(csort, ncl, n, bmask, a.hdr_start, g->cl_off, a.out_vert, g->cl_vert,
+                                                g->cluster_of);
+        RTR_CUDA_TRY(cudaMemsetAsync(g->cl_ne, 0, sizeof(int64_t) * (ncl + 1), s));
+        RTR_CUDA_TRY(cudaMemsetAsync(g->cl_cut, 0, sizeof(int64_t) * (ncl + 1), s));
+        g->launches += 3 + take_primitive_launches();
+    }
+    k_cluster_stats<<<gn, kBlock, 0, s>>>(g->offsets, g->nbors, n, g->cluster_of, counts + 1,
                                           (unsigned long long*)g->cl_ne, (unsigned long long*)g->cl_cut);
-    k_halve<<<gk, kBlock, 0, s>>>(g->cl_ne, ncl, g->cl_off, g->ctr + 5);
-    g->launches += 6 + take_primitive_launches();
+    k_halve<<<gk, kBlock, 0, s>>>(g->cl_ne, counts);
+    g->launches += 2;
     RTR_CUDA_TRY(cudaGetLastError());
     cudaEventRecord(e1, s);
-    unsigned long long members = 0;
-    if (const int rc = read_words(g, &members, g->ctr + 5, sizeof members)) return rc;
+    if (const int rc = read_words(g, h, g->ctr, sizeof h, small)) return rc;
     cudaEventElapsedTime(&g->ms_extract, e0, e1);
     ktime_read(g, KT_EXTRACT);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    if (failed()) return RTR_ERR_DEVICE;
+    g->diag_residual += (long long)h[2];
     // the clusters must partition the vertex set
-    if ((int64_t)members != n) {
-        set_error("extraction produced %lld cluster members for %lld vertices", (long long)members, (long long)n);
+    if ((int64_t)h[5] != n) {
+        set_error("extraction produced %lld cluster members for %lld vertices", (long long)h[5], (long long)n);
         return RTR_ERR_DEVICE;
     }
+    g->ncl = (int64_t)h[4];
     g->stage = 4;
     return RTR_OK;
 }

@@ -43,6 +43,7 @@ struct rtr_graph {
 
     // extraction results: clusters in creation order
     int64_t ncl = 0;
+    int64_t cl_cap = 0;            // clusters that the arrays hold
     int32_t* cl_seed = nullptr;    // [ncl]
     int64_t* cl_off = nullptr;     // [ncl+1] into cl_vert
     int32_t* cl_vert = nullptr;    // [n] members, in set-iteration order
