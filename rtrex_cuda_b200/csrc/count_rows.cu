@@ -24,7 +24,10 @@
 //             (the intersection again); k_fill_heavy: a warp per heavy edge,
 //             which reads the count's hit masks (one 32-bit word per 32
 //             elements of the shorter row) instead of repeating the lookups,
-//             hits ranked by ballot.
+//             a lane per hit.  What bounds it: the gathers of nb and deg
+//             and the 4-byte stores of the hits (a lane per element of a
+//             word with hits, 7 of 32 at work: R-MAT scale 19 7.0 -> 5.8
+//             ms, scale 20 17.8 -> 14.6, 22 105 -> 81).
 //   fold      perVertex[x] = the left fold of x's slots' lists in slot order
 //             (y ascending), each in z order -- exactly commonNbr's order.
 //             k_vfold_thread: a thread per vertex of fewer than warp_min terms;
@@ -126,7 +129,7 @@ __global__ void __launch_bounds__(kHeavyBlock, 8) k_fill_heavy(FillArgs a, const
         const int64_t i = a.fwd[heavy_list[h]];
         const int32_t u = a.esrc[i], v = a.nb[i];
         const int64_t r = a.partner[i];
-        const bool wi = kPri ? a.rank[u] >= 0 : in_window(a, i), wr = kPri ? a.rank[v] >= 0 : in_window(a, r);
+        bool wi = kPri ? a.rank[u] >= 0 : in_window(a, i), wr = kPri ? a.rank[v] >= 0 : in_window(a, r);
         if (!wi && !wr) continue;  // uniform across the warp
         int64_t qi = 0, qr = 0, qi1 = 0, qr1 = 0;  // the writes stay inside each list
         if (wi) {
@@ -139,6 +142,9 @@ __global__ void __launch_bounds__(kHeavyBlock, 8) k_fill_heavy(FillArgs a, const
             qr = a.lpos[lr] - a.e0;
             qr1 = a.lpos[lr + 1] - a.e0;
         }
+        wi = wi && qi1 > qi;  // an empty list (a row folded ahead has none here) wants nothing
+        wr = wr && qr1 > qr;
+        if (!wi && !wr) continue;
         const int32_t from = wr ? u + 1 : v + 1;
         const int64_t u0 = a.off[u], u1 = a.off[u + 1], v0 = a.off[v], v1 = a.off[v + 1];
         const bool u_short = u1 - u0 <= v1 - v0;
@@ -156,43 +162,50 @@ __global__ void __launch_bounds__(kHeavyBlock, 8) k_fill_heavy(FillArgs a, const
         };
         const int32_t t = rs_table(a.rs, u_short ? v : u);
         if (t >= 0 && a.masks) {
-            // the count's hit masks: only chunks with hits are read, no lookups
+            // The count's hit masks, 32 words at a time, a lane per hit: its word by a search over
+            // the words' running counts, its bit by halving.  Hit g of the edge is entry g of slot
+            // r's list; slot i's list (z > v) is the last of them.
             const int64_t w0 = a.moff[h], nw = a.moff[h + 1] - w0;
             const int64_t sa = u_short ? u0 : v0;  // where the count's walk began
-            for (int64_t cb = (s0 - sa) / 32; cb < nw; cb += 32) {
-                const int64_t cc = cb + lane;
-                const uint32_t mw = cc < nw ? __ldg(a.masks + w0 + cc) : 0u;
-                unsigned nz = __ballot_sync(0xffffffffu, mw != 0u);
-                while (nz) {  // uniform across the warp
-                    // up to four chunks with hits at a time: their element loads, then their
-                    // degree loads, in flight together; emitted in chunk order
-                    constexpr int Q = 4;
-                    int js[Q];
-                    uint32_t ms[Q];
+            const int64_t all = wr ? qr1 - qr : qi1 - qi, gi0 = all - (qi1 - qi), c0 = (s0 - sa) / 32;
+            int64_t done = 0;
+            for (int64_t cb = c0; cb < nw && done < all; cb += 32) {
+                uint32_t mw = cb + lane < nw ? __ldg(a.masks + w0 + cb + lane) : 0u;
+                if (cb == c0 && lane == 0) mw &= 0xffffffffu << (int)((s0 - sa) & 31);  // before s0: z < from
+                const int cw = __popc(mw);
+                int incl = cw;
 #pragma unroll
-                    for (int q = 0; q < Q; ++q) {
-                        js[q] = -1;
-                        ms[q] = 0u;
-                        if (nz) {
-                            js[q] = __ffs(nz) - 1;
-                            nz &= nz - 1u;
-                            ms[q] = __shfl_sync(0xffffffffu, mw, js[q]);
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                const int tot = __shfl_sync(0xffffffffu, incl, 31);
+                for (int b = 0; b < tot; b += 32) {
+                    const int gl = b + lane;
+                    int j = 0;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        const int y = __shfl_sync(0xffffffffu, incl, j + o - 1);
+                        if (y <= gl) j += o;
+                    }
+                    const uint32_t word = __shfl_sync(0xffffffffu, mw, j);
+                    int k = gl - __shfl_sync(0xffffffffu, incl - cw, j), bit = 0;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        const int y = __popc((word >> bit) & ((1u << o) - 1u));
+                        if (y <= k) {
+                            k -= y;
+                            bit += o;
                         }
                     }
-                    bool hit[Q];
-                    int32_t z[Q], dz[Q];
-#pragma unroll
-                    for (int q = 0; q < Q; ++q) {
-                        const int64_t p = sa + (cb + js[q]) * 32 + lane;
-                        hit[q] = js[q] >= 0 && ((ms[q] >> lane) & 1u) && p >= s0;  // before s0: z < from
-                        z[q] = hit[q] ? a.nb[p] : 0;
+                    if (gl < tot) {
+                        const int64_t g = done + gl;
+                        const int32_t dz = a.deg[a.nb[sa + (cb + j) * 32 + bit]];
+                        if (wr && qr + g < qr1) a.lists[qr + g] = dz;
+                        if (wi && g >= gi0 && qi + (g - gi0) < qi1) a.lists[qi + (g - gi0)] = dz;
                     }
-#pragma unroll
-                    for (int q = 0; q < Q; ++q) dz[q] = hit[q] ? a.deg[z[q]] : 0;
-#pragma unroll
-                    for (int q = 0; q < Q; ++q)
-                        if (js[q] >= 0) emit(hit[q], z[q], dz[q]);
                 }
+                done += tot;
             }
         } else if (t >= 0) {
             constexpr int B = 4;  // 4 chunks per step, their lookups (then degrees) in flight together
