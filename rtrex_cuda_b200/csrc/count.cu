@@ -183,6 +183,13 @@ struct HeavyArgs {
 // 94 for scale 20.  More vertices than fit one block's shared memory keep the hash
 // sets: bits shared by several ids, with the hits looked up, took three times as
 // long (scale 22: 950 ms for the heavy edges against 332).
+// Heavy edges from which this pays, and from which the longest rows go ahead of the
+// rest (count_rows.cu): each costs a few launches and waits.  R-MAT scales 15 / 16 /
+// 17 / 18 (168,000 / 338,000 / 1.1 M / 2.2 M heavy edges), whole count: neither 4.48 /
+// 6.81 / 13.5 / 27.6 ms, bits alone 5.02 / 6.72 / 12.4 / 24.1, both 5.33 / 6.72 / 11.4 /
+// 18.7.
+constexpr unsigned kBitsEdges = 1u << 18;
+constexpr unsigned kAheadRows = 1u << 19;
 constexpr int64_t kRunWords = 256;
 constexpr int64_t kPieceWords = 8192;
 constexpr int kMaxBits = 20;  // of the shared-memory row: 128 KB, a block an SM; below, two blocks
@@ -998,7 +1005,10 @@ int count_triangles(rtr_graph* g)
     // graph holds lists from an earlier count (they will be kept again), nor under a set window size
     // (the caller's bound is then on all the lists that are held).
     PriorityRows pr;
-    if (rs.tab && !g->tl && g->rows_window_cap == 0) {
+    unsigned nh = 0;  // heavy edges, where the sets are built
+    if (rs.tab)
+        if (const int rc = read_words(g, &nh, nheavy, sizeof(unsigned))) return rc;
+    if (rs.tab && !g->tl && g->rows_window_cap == 0 && nh >= kAheadRows) {
         const int rc = pick_priority_rows(g, sc, &pr);
         if (rc) return rc;
     }
@@ -1017,8 +1027,6 @@ int count_triangles(rtr_graph* g)
     } side_guard{g, &pr};
     HeavyRuns runs{nullptr, 0, n, nullptr, nullptr};
     if (rs.tab) {  // heavy edges in the order of the sets they probe
-        unsigned nh = 0;
-        if (const int rc = read_words(g, &nh, nheavy, sizeof(unsigned))) return rc;
         if (nh > 1) {
             uint64_t* hkeys = (uint64_t*)sc.get(sizeof(uint64_t) * (nh + 1));
             uint64_t* halt = (uint64_t*)sc.get(sizeof(uint64_t) * (nh + 1));
@@ -1049,8 +1057,6 @@ int count_triangles(rtr_graph* g)
     longlong2* pieces = nullptr;
     int64_t np[2] = {0, 0};  // pieces of the priority rows' runs, of the others
     if (rs.tab) {
-        unsigned nh = 0;
-        if (const int rc = read_words(g, &nh, nheavy, sizeof(unsigned))) return rc;
         if (nh > 0) {
             msc.reset(new Scratch(g));
             int64_t* wcount = (int64_t*)msc->get(sizeof(int64_t) * (nh + 1));
@@ -1065,7 +1071,7 @@ int count_triangles(rtr_graph* g)
             exclusive_scan_i64(wcount, moff, nh + 1, nullptr, wtmp, s);
             int64_t words = 0;
             if (const int rc = read_words(g, &words, moff + nh, sizeof(int64_t))) return rc;
-            if (runs.keys && n <= (1ll << kMaxBits)) {
+            if (runs.keys && n <= (1ll << kMaxBits) && nh >= kBitsEdges) {
                 const int rc = cut_runs(g, *msc, rs, nh, moff, &runs, &pieces, np);
                 if (rc) return rc;
             }

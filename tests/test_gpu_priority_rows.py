@@ -1,8 +1,9 @@
 """The rows layout's longest rows, counted and folded ahead of the rest: hubs of
 2,047 to 2,049 neighbours (the least such row has 2,048) and more than 32 of them
 (the most taken), with the degree from which an edge is a heavy one above and
-below; counted again in the same graph, in windows, and with lists, against the
-oracle bit for bit."""
+below; counted again in the same graph, in windows, and with lists, beside a
+complete bipartite graph that brings the heavy edges to the number from which rows
+are taken ahead (2^19), against the oracle bit for bit."""
 import numpy as np
 import pytest
 
@@ -45,6 +46,9 @@ CASES = {
 @pytest.mark.parametrize("edge", [1, 1024, 2049, 6000])
 def test_hubs(name, edge):
     n, u, v = _hubs(CASES[name], 5)
+    a, b = np.meshgrid(np.arange(512), np.arange(1024))
+    u, v = np.concatenate([u, n + a.ravel()]), np.concatenate([v, n + 512 + b.ravel()])
+    n += 1536
     c = oracle.build_csr(n, u, v)
     assert sorted(np.diff(c.offsets)[: len(CASES[name])]) == sorted(CASES[name])
     s = oracle.count(c)
