@@ -39,7 +39,7 @@
 //             add chain -- the one sequential part (~10^8 dependent adds for
 //             the largest R-MAT scale-24 vertex).  Vertices are dealt from
 //             queues in descending term count.
-//   ahead     the rows of the most neighbours (up to 32) go before all others:
+//   ahead     on large graphs the rows of the most neighbours (up to 32) go first:
 //             pick_priority_rows names them, count.cu counts their edges first,
 //             and fold_priority_rows fills their lists and runs their chains on
 //             the second stream beside the rest of the count and the fill.
