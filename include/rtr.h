@@ -135,6 +135,12 @@ int rtr_get_tuning(const rtr_graph* g, int* gallop_ratio, int* heavy_degree, int
  * (RTRex_Sequential/Escape/Decomposition.h:42-117). */
 int rtr_set_count_mode(rtr_graph* g, int mode, int hub_degree);
 int rtr_get_count_mode(const rtr_graph* g, int* mode, int* hub_degree, int* lists_kept);
+/* Directed slots (2m) from which a count in mode 0 prepares for the rows layout
+ * before it knows whether the lists fit: hash sets of the long rows, the heavy
+ * edges in their order, the longest perVertex chains ahead of the rest.  Default
+ * 2^25; lowered, small graphs take the same path.  Results are the same bits for
+ * every setting.  No counterpart in the reference. */
+int rtr_set_count_sets(rtr_graph* g, int64_t min_slots);
 /* Rows layout of the last rtr_count: the windows of whole rows its per-slot
  * lists were filled and folded in (1 when they all fit in free device memory)
  * and their total entries (3 per triangle); both 0 when the lists were kept.

@@ -107,6 +107,7 @@ def lib():
     L.rtr_set_count_mode.argtypes = [_vp, ctypes.c_int, ctypes.c_int]
     L.rtr_get_count_mode.argtypes = [_vp, P(ctypes.c_int), P(ctypes.c_int), P(ctypes.c_int)]
     L.rtr_get_count_windows.argtypes = [_vp, P(ctypes.c_int64), P(ctypes.c_int64)]
+    L.rtr_set_count_sets.argtypes = [_vp, ctypes.c_int64]
     L.rtr_set_count_window.argtypes = [_vp, ctypes.c_int64]
     L.rtr_graph_create_rmat.argtypes = [ctypes.c_int, _i64, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                         ctypes.c_uint64, ctypes.c_int, P(_vp)]
@@ -365,6 +366,10 @@ class Graph:
         a, b, c = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
         _check(lib().rtr_get_count_mode(self._h, ctypes.byref(a), ctypes.byref(b), ctypes.byref(c)))
         return int(a.value), int(b.value), bool(c.value)
+
+    def set_count_sets(self, min_slots: int):
+        """Directed slots from which mode 0 prepares for the rows layout (same bits)."""
+        _check(lib().rtr_set_count_sets(self._h, int(min_slots)))
 
     def set_count_window(self, max_entries: int):
         """Rows layout: at most max_entries list entries per window (0: as many as fit)."""

@@ -489,6 +489,16 @@ int rtr_get_count_mode(const rtr_graph* g, int* mode, int* hub_degree, int* list
     return RTR_OK;
 }
 
+int rtr_set_count_sets(rtr_graph* g, int64_t min_slots)
+{
+    if (!g || min_slots < 0) {
+        set_error("rtr_set_count_sets: null graph or negative slot count");
+        return RTR_ERR_ARG;
+    }
+    g->count_sets = min_slots;
+    return RTR_OK;
+}
+
 int rtr_set_count_window(rtr_graph* g, int64_t max_entries)
 {
     if (!g || max_entries < 0) {

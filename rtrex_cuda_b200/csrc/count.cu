@@ -943,7 +943,9 @@ int count_triangles(rtr_graph* g)
     int64_t* tmp = (int64_t*)sc.get(sizeof(int64_t) * scan_temp_elems(m2 + 1));
     int32_t* heavy_list = (int32_t*)sc.get(sizeof(int32_t) * (m + 1));
     unsigned* nheavy = (unsigned*)(g->ctr + 5);  // heavy edges; those of the priority rows
-    unsigned long long* hq = (unsigned long long*)sc.get(sizeof(unsigned long long) * 5);  // the heavy counts' queues
+    // a queue word for each launch that deals the heavy edges: the counts', then the list fill's
+    constexpr int kQueues = 6;
+    unsigned long long* hq = (unsigned long long*)sc.get(sizeof(unsigned long long) * kQueues);
     if (!cnt || !tmp || !heavy_list || !hq) {
         set_error("device allocation failed (count scratch)");
         return RTR_ERR_CUDA;
@@ -959,12 +961,12 @@ int count_triangles(rtr_graph* g)
     const int ge = grid_for(m, kBlock);
     const int gh = grid_for(1ll << 40, kHeavyEdgeBlock, 16);
     const int gc = grid_for(1ll << 40, kHeavyEdgeBlock, 6);  // k_edge_count_heavy: the resident blocks
-    RTR_CUDA_TRY(cudaMemsetAsync(hq, 0, sizeof(unsigned long long) * 5, s));
+    RTR_CUDA_TRY(cudaMemsetAsync(hq, 0, sizeof(unsigned long long) * kQueues, s));
     ktime_begin(g, KT_EDGE_FOLD);
     // Hash sets of the long rows, for the heavy-edge count and the rows layout:
-    // built when the rows layout is asked for, or may be chosen (2m >= 2^25).
+    // built when the rows layout is asked for, or may be chosen (2m >= count_sets).
     RowSets rs{nullptr, nullptr, nullptr, nullptr};
-    if (g->count_mode == 2 || (g->count_mode == 0 && m2 >= (1ll << 25))) {
+    if (g->count_mode == 2 || (g->count_mode == 0 && m2 >= g->count_sets)) {
         const int rc = build_row_sets(g, sc, kSetDegree, &rs);
         if (rc) return rc;
     }
@@ -1214,7 +1216,7 @@ int count_triangles(rtr_graph* g)
     if (heavy)
         k_tri_fill_heavy<<<gh, kHeavyEdgeBlock, 0, hs>>>(g->offsets, g->nbors, g->esrc, g->deg, g->partner, g->fwd,
                                                          g->frank, heavy_list, nheavy, g->tune_gallop, parts,
-                                                         ha.nparts, g->tl_off, g->tl, hq);
+                                                         ha.nparts, g->tl_off, g->tl, hq + 5);
     if (ahead) {
         RTR_CUDA_TRY(cudaEventRecord(filled, hs));
         gather(cut, top, hs);

@@ -88,6 +88,8 @@ struct rtr_graph {
     // 1 always keep them, 2 never (rows layout: folds straight from the CSR);
     // count_hub: perVertex terms from which the rows layout folds a vertex with a warp
     int count_mode = 0;
+    // directed slots from which mode 0 prepares for the rows layout (rtr_set_count_sets)
+    int64_t count_sets = 1ll << 25;
     int64_t rows_window_cap = 0;  // rows layout: list entries per window at most (0: as many as fit)
     int64_t rows_windows = 0;  // rows layout: windows the last count took, and its list entries
     int64_t rows_entries = 0;
