@@ -164,6 +164,13 @@ int rtr_set_count_window(rtr_graph* g, int64_t max_entries);
 int rtr_set_clean_split(rtr_graph* g, int64_t min_seeds, double max_mean_list);
 int rtr_get_clean_split(const rtr_graph* g, int64_t* min_seeds, double* max_mean_list);
 
+/* Device bytes that the window replay's log may take: about 85 for each triangle
+ * of the units it replays, beside the lists' 96.  -1 (the default): what the
+ * device has, less 1 GiB.  When the log does not fit, those units replay one warp
+ * each as well, which is slower and needs no log.  Results are the same bits for
+ * every setting.  No counterpart in the reference. */
+int rtr_set_clean_log(rtr_graph* g, int64_t max_bytes);
+
 /* Split of the extraction: components of the cleaned graph with at least
  * min_vertices vertices (default 512) replay their seed loop in a whole thread
  * block -- the two-hop scan's pairs worked out by seven warps ahead of the warp

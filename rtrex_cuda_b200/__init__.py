@@ -112,6 +112,7 @@ def lib():
     L.rtr_graph_create_rmat.argtypes = [ctypes.c_int, _i64, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                         ctypes.c_uint64, ctypes.c_int, P(_vp)]
     L.rtr_set_clean_split.argtypes = [_vp, _i64, ctypes.c_double]
+    L.rtr_set_clean_log.argtypes = [_vp, _i64]
     L.rtr_set_clean_checks.argtypes = [_vp, _i64, _i64]
     L.rtr_set_extract_split.argtypes = [_vp, _i64]
     L.rtr_nucleus.argtypes = [_vp, P(_i64)]
@@ -386,6 +387,11 @@ class Graph:
         most `max_mean_list` entries on average replay a window of pops at a
         time (one thread block each), the others one warp per unit (same bits)."""
         _check(lib().rtr_set_clean_split(self._h, int(min_seeds), float(max_mean_list)))
+
+    def set_clean_log(self, max_bytes: int = -1):
+        """Device bytes that the window replay's log may take (-1: what the device has,
+        less 1 GiB); units whose log does not fit replay one warp each (same bits)."""
+        _check(lib().rtr_set_clean_log(self._h, int(max_bytes)))
 
     def nucleus(self) -> int:
         """The nucleus (truss-hierarchy) path; returns the number of clusters."""

@@ -543,6 +543,16 @@ int rtr_set_clean_checks(rtr_graph* g, int64_t first_wait_rounds, int64_t stack_
     return RTR_OK;
 }
 
+int rtr_set_clean_log(rtr_graph* g, int64_t max_bytes)
+{
+    if (!g || max_bytes < -1) {
+        set_error("rtr_set_clean_log: null graph or byte count below -1");
+        return RTR_ERR_ARG;
+    }
+    g->clean_log_limit = max_bytes;
+    return RTR_OK;
+}
+
 int rtr_set_extract_split(rtr_graph* g, int64_t min_vertices)
 {
     if (!g || min_vertices < 2) {

@@ -44,6 +44,7 @@
 #include "unionfind.cuh"
 
 #include <algorithm>
+#include <memory>
 #include <vector>
 
 namespace rtr {
@@ -862,18 +863,26 @@ int initial_clean(rtr_graph* g, double eps)
         if (const int rc = read_words(g, tot, d_tot, sizeof tot)) return rc;
         if (small) nu = (uint32_t)tot[4];
         const unsigned* nc = (const unsigned*)(tot + 2);
-        const int64_t nwide = nc[UNIT_WIDE], nnarrow = nc[UNIT_NARROW], nbig = nwide + nnarrow;
+        int64_t nwide = nc[UNIT_WIDE], nnarrow = nc[UNIT_NARROW];
         StackEntry* stacks = (StackEntry*)sc.get(sizeof(StackEntry) * (tot[0] + 1));
         if (!stacks) {
             set_error("device allocation failed (clean stacks)");
             return RTR_ERR_CUDA;
         }
+        // The window replay's log, reserved before anything is replayed: without room for it every
+        // unit replays one warp each.  Freed after the side streams are waited for.
+        std::unique_ptr<Scratch> log(new Scratch(g));
+        RoundReplay rr;
+        if (nwide + nnarrow > 0 && !clean_rounds_reserve(g, *log, tot[0], tot[1], &rr)) {
+            log.reset();
+            nwide = nnarrow = 0;
+        }
+        const int64_t nbig = nwide + nnarrow;
         ktime_begin(g, KT_CLEAN_UNITS);
         // The units order[0, nbig) take the window replay, the others replay one warp
         // per unit; each of the three kinds that exists takes a stream of its own, the
         // first the graph's (a side stream costs 0.1 ms to make and to destroy, a third
         // of what a graph of 1,000 edges spends in this stage).
-        RoundReplay rr;
         SideWait side_wait, side_wait2;  // an early return waits for the side streams before scratch is freed
         const bool has_small = nbig < (int64_t)nu;
         cudaStream_t wide_st = s, narrow_st = s;
@@ -887,8 +896,8 @@ int initial_clean(rtr_graph* g, double eps)
             narrow_st = side_wait2.st = st;
         }
         if (nbig > 0) {
-            const int rc = clean_rounds_launch(g, sc, wide_st, narrow_st, rec, seeds, units, order, nwide, nnarrow,
-                                               tot[0], tot[1], stacks, &rr);
+            const int rc = clean_rounds_launch(g, wide_st, narrow_st, rec, seeds, units, order, nwide, nnarrow, stacks,
+                                               &rr);
             if (rc) return rc;
         }
         if (has_small) {
@@ -915,7 +924,7 @@ int initial_clean(rtr_graph* g, double eps)
                 cudaStreamWaitEvent(s, joined, 0);
                 cudaEventDestroy(joined);
             }
-            const int rc = clean_rounds_finish(g, sc, &rr);
+            const int rc = clean_rounds_finish(g, &rr);
             if (rc) return rc;
         }
         ktime_end(g, KT_CLEAN_UNITS);

@@ -695,22 +695,61 @@ int launch_rounds(rtr_graph* g, RoundArgs ra, int64_t units, cudaStream_t st)
 
 }  // namespace
 
-int clean_rounds_launch(rtr_graph* g, Scratch& sc, cudaStream_t wide_st, cudaStream_t narrow_st, EdgeRec* rec,
+// A log of up to this size is simply asked for (the device's free memory takes 64 us
+// to learn); a larger one must leave this much of it to others.
+constexpr int64_t kLogSmall = 256ll << 20;
+constexpr int64_t kLogMargin = 1ll << 30;
+
+bool clean_rounds_reserve(rtr_graph* g, Scratch& sc, int64_t stack_entries, int64_t log_entries, RoundReplay* rr)
+{
+    const int64_t pops = stack_entries, logs = log_entries, cnt = 3 * logs;
+    const size_t sizes[] = {sizeof(PopLog) * ((size_t)pops + 1),
+                            (size_t)g->tl_len + 16,
+                            sizeof(uint32_t) * ((size_t)pops + 1),
+                            sizeof(uint32_t) * ((size_t)pops + 1),
+                            sizeof(uint32_t) * (size_t)scan_temp_elems(pops + 1),
+                            sizeof(double) * ((size_t)logs + 1),
+                            sizeof(uint64_t) * ((size_t)cnt + 1),
+                            sizeof(uint64_t) * ((size_t)cnt + 1),
+                            radix_temp_bytes(cnt),
+                            sizeof(double) * ((size_t)cnt + 1),
+                            sizeof(longlong2) * ((size_t)(cnt / kLongRun) + 2),
+                            sizeof(unsigned) * 2};
+    constexpr int kParts = sizeof sizes / sizeof sizes[0];
+    int64_t need = 0;
+    for (const size_t b : sizes) need += (int64_t)b;
+    if (g->clean_log_limit >= 0 && need > g->clean_log_limit) return false;
+    if (need > kLogSmall && need + kLogMargin > (int64_t)device_avail_bytes(g)) return false;
+    void* part[kParts];
+    for (int k = 0; k < kParts; ++k)
+        if (!(part[k] = sc.get(sizes[k]))) {
+            cudaGetLastError();  // the units replay without the log
+            return false;
+        }
+    rr->pops_cap = pops;
+    rr->logs_cap = logs;
+    rr->plog = (PopLog*)part[0];
+    rr->live8 = (uint8_t*)part[1];
+    rr->pcnt = (uint32_t*)part[2];
+    rr->poff = (uint32_t*)part[3];
+    rr->ptmp = (uint32_t*)part[4];
+    rr->wlog = (double*)part[5];
+    rr->keys = (uint64_t*)part[6];
+    rr->alt = (uint64_t*)part[7];
+    rr->rtmp = part[8];
+    rr->ws = (double*)part[9];
+    rr->runs = (longlong2*)part[10];
+    rr->nruns = (unsigned*)part[11];
+    return true;
+}
+
+int clean_rounds_launch(rtr_graph* g, cudaStream_t wide_st, cudaStream_t narrow_st, EdgeRec* rec,
                         const StackEntry* seeds, const UnitDesc* units, const uint64_t* order, int64_t nwide,
-                        int64_t nnarrow, int64_t stack_entries, int64_t log_entries, StackEntry* stacks,
-                        RoundReplay* rr)
+                        int64_t nnarrow, StackEntry* stacks, RoundReplay* rr)
 {
     rr->rec = rec;
-    rr->pops_cap = stack_entries;
-    rr->logs_cap = log_entries;
-    rr->plog = (PopLog*)sc.get(sizeof(PopLog) * (stack_entries + 1));
-    rr->live8 = (uint8_t*)sc.get((size_t)g->tl_len + 16);
-    if (!rr->plog || !rr->live8) {
-        set_error("device allocation failed (clean rounds)");
-        return RTR_ERR_CUDA;
-    }
     cudaStream_t s = g->stream;
-    RTR_CUDA_TRY(cudaMemsetAsync(rr->plog, 0xff, sizeof(PopLog) * (stack_entries + 1), s));
+    RTR_CUDA_TRY(cudaMemsetAsync(rr->plog, 0xff, sizeof(PopLog) * ((size_t)rr->pops_cap + 1), s));
     RTR_CUDA_TRY(cudaMemsetAsync(rr->live8, 0, (size_t)g->tl_len + 16, s));
     // the replays on side streams run after everything above
     if (wide_st != s || narrow_st != s) {
@@ -735,39 +774,26 @@ int clean_rounds_launch(rtr_graph* g, Scratch& sc, cudaStream_t wide_st, cudaStr
     return RTR_OK;
 }
 
-int clean_rounds_finish(rtr_graph* g, Scratch& sc, RoundReplay* rr)
+int clean_rounds_finish(rtr_graph* g, RoundReplay* rr)
 {
     cudaStream_t s = g->stream;
     const int64_t pops = rr->pops_cap, logs = rr->logs_cap, cnt = 3 * logs;
     if (logs == 0) return RTR_OK;
     const int lb = bits_for((uint64_t)logs);
     const int vb = bits_for((uint64_t)g->n);
-    uint32_t* pcnt = (uint32_t*)sc.get(sizeof(uint32_t) * (pops + 1));
-    uint32_t* poff = (uint32_t*)sc.get(sizeof(uint32_t) * (pops + 1));
-    uint32_t* ptmp = (uint32_t*)sc.get(sizeof(uint32_t) * scan_temp_elems(pops + 1));
-    uint64_t* keys = (uint64_t*)sc.get(sizeof(uint64_t) * ((size_t)cnt + 1));
-    uint64_t* alt = (uint64_t*)sc.get(sizeof(uint64_t) * ((size_t)cnt + 1));
-    void* rtmp = sc.get(radix_temp_bytes(cnt));
-    double* wlog = (double*)sc.get(sizeof(double) * ((size_t)logs + 1));
-    double* ws = (double*)sc.get(sizeof(double) * ((size_t)cnt + 1));
-    longlong2* runs = (longlong2*)sc.get(sizeof(longlong2) * ((size_t)(cnt / kLongRun) + 2));
-    unsigned* nruns = (unsigned*)sc.get(sizeof(unsigned) * 2);
-    if (!pcnt || !poff || !ptmp || !keys || !alt || !rtmp || !wlog || !ws || !runs || !nruns) {
-        set_error("device allocation failed (clean rounds log)");
-        return RTR_ERR_CUDA;
-    }
-    RTR_CUDA_TRY(cudaMemsetAsync(nruns, 0, sizeof(unsigned) * 2, s));
+    RTR_CUDA_TRY(cudaMemsetAsync(rr->nruns, 0, sizeof(unsigned) * 2, s));
     // an unused key keeps a vertex past the last
-    RTR_CUDA_TRY(cudaMemsetAsync(keys, 0xff, sizeof(uint64_t) * (size_t)cnt, s));
-    k_pop_counts<<<grid_for(pops, kBlock), kBlock, 0, s>>>(rr->plog, pops, pcnt);
-    exclusive_scan_u32(pcnt, poff, pops, nullptr, ptmp, s);
-    k_log_keys<<<grid_for(8 * pops, kBlock), kBlock, 0, s>>>(rr->rec, rr->plog, poff, pops, g->tl, rr->live8, g->fwd,
-                                                             g->esrc, g->nbors, 1 / (double)g->n, lb, keys, wlog,
-                                                             (unsigned*)(g->ctr + 1), g->ctr + 2);
+    RTR_CUDA_TRY(cudaMemsetAsync(rr->keys, 0xff, sizeof(uint64_t) * (size_t)cnt, s));
+    k_pop_counts<<<grid_for(pops, kBlock), kBlock, 0, s>>>(rr->plog, pops, rr->pcnt);
+    exclusive_scan_u32(rr->pcnt, rr->poff, pops, nullptr, rr->ptmp, s);
+    k_log_keys<<<grid_for(8 * pops, kBlock), kBlock, 0, s>>>(rr->rec, rr->plog, rr->poff, pops, g->tl, rr->live8,
+                                                             g->fwd, g->esrc, g->nbors, 1 / (double)g->n, lb,
+                                                             rr->keys, rr->wlog, (unsigned*)(g->ctr + 1), g->ctr + 2);
     // the keys come in log order, so a stable sort on the vertex bits suffices
-    uint64_t* sorted = radix_sort_bits_u64(keys, alt, cnt, lb, lb + vb, rtmp, s);
-    k_log_gather<<<grid_for(cnt, kBlock), kBlock, 0, s>>>(sorted, cnt, g->n, lb, wlog, ws, g->pv, runs, nruns);
-    k_fold_long_runs<<<grid_for(1ll << 40, 128, 8), 128, 0, s>>>(runs, nruns, sorted, lb, ws, g->pv);
+    uint64_t* sorted = radix_sort_bits_u64(rr->keys, rr->alt, cnt, lb, lb + vb, rr->rtmp, s);
+    k_log_gather<<<grid_for(cnt, kBlock), kBlock, 0, s>>>(sorted, cnt, g->n, lb, rr->wlog, rr->ws, g->pv, rr->runs,
+                                                          rr->nruns);
+    k_fold_long_runs<<<grid_for(1ll << 40, 128, 8), 128, 0, s>>>(rr->runs, rr->nruns, sorted, lb, rr->ws, g->pv);
     g->launches += 4 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     return RTR_OK;

@@ -80,11 +80,23 @@ struct RoundReplay {
     int64_t pops_cap = 0, logs_cap = 0;
     PopLog* plog = nullptr;
     uint8_t* live8 = nullptr;  // per list entry: its triangle was removed by the pop of its list's edge
+    // the fold's: per pop, per removed triangle, per subtraction
+    uint32_t *pcnt = nullptr, *poff = nullptr, *ptmp = nullptr;
+    double* wlog = nullptr;
+    uint64_t *keys = nullptr, *alt = nullptr;
+    void* rtmp = nullptr;
+    double* ws = nullptr;
+    longlong2* runs = nullptr;
+    unsigned* nruns = nullptr;
 };
-int clean_rounds_launch(rtr_graph* g, Scratch& sc, cudaStream_t wide_st, cudaStream_t narrow_st, EdgeRec* rec,
+// The memory of all that, before anything is replayed: about 85 bytes for each
+// triangle of the units, beside the lists' 96.  False when it does not fit: the
+// units then replay one warp each, which needs none of it (the lists are kept
+// without regard to the log, so no graph loses its clean to it).
+bool clean_rounds_reserve(rtr_graph* g, Scratch& sc, int64_t stack_entries, int64_t log_entries, RoundReplay* rr);
+int clean_rounds_launch(rtr_graph* g, cudaStream_t wide_st, cudaStream_t narrow_st, EdgeRec* rec,
                         const StackEntry* seeds, const UnitDesc* units, const uint64_t* order, int64_t nwide,
-                        int64_t nnarrow, int64_t stack_entries, int64_t log_entries, StackEntry* stacks,
-                        RoundReplay* rr);
-int clean_rounds_finish(rtr_graph* g, Scratch& sc, RoundReplay* rr);
+                        int64_t nnarrow, StackEntry* stacks, RoundReplay* rr);
+int clean_rounds_finish(rtr_graph* g, RoundReplay* rr);
 
 }  // namespace rtr
