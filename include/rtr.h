@@ -189,6 +189,12 @@ int rtr_set_extract_split(rtr_graph* g, int64_t min_vertices);
  * the graph's results are then incomplete but the device stays usable. */
 int rtr_set_clean_checks(rtr_graph* g, int64_t first_wait_rounds, int64_t stack_entries);
 
+/* A smaller device, to test what calls do on a full one (no counterpart in the
+ * reference): the rules that ask how much device memory is available take the
+ * graph to have graph_bytes for all it holds, and a single allocation of more than
+ * max_alloc bytes fails.  0, the default of both: the device's own limits. */
+int rtr_set_device_limits(rtr_graph* g, int64_t graph_bytes, int64_t max_alloc);
+
 /* Autotuner: times the counting pass on this graph for gallop ratios
  * {4,8,16,32,64}, then heavy degrees {8,16,32,64,128}, then heavy-edge degree
  * sums {128,256,512,1024,4096,off} (coordinate descent, each candidate timed by

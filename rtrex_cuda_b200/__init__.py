@@ -113,6 +113,7 @@ def lib():
                                         ctypes.c_uint64, ctypes.c_int, P(_vp)]
     L.rtr_set_clean_split.argtypes = [_vp, _i64, ctypes.c_double]
     L.rtr_set_clean_log.argtypes = [_vp, _i64]
+    L.rtr_set_device_limits.argtypes = [_vp, _i64, _i64]
     L.rtr_set_clean_checks.argtypes = [_vp, _i64, _i64]
     L.rtr_set_extract_split.argtypes = [_vp, _i64]
     L.rtr_nucleus.argtypes = [_vp, P(_i64)]
@@ -392,6 +393,10 @@ class Graph:
         """Device bytes that the window replay's log may take (-1: what the device has,
         less 1 GiB); units whose log does not fit replay one warp each (same bits)."""
         _check(lib().rtr_set_clean_log(self._h, int(max_bytes)))
+
+    def set_device_limits(self, graph_bytes: int = 0, max_alloc: int = 0):
+        """Take the device to be smaller (0: as it is), to test what calls do on a full one."""
+        _check(lib().rtr_set_device_limits(self._h, int(graph_bytes), int(max_alloc)))
 
     def nucleus(self) -> int:
         """The nucleus (truss-hierarchy) path; returns the number of clusters."""

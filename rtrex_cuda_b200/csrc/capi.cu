@@ -543,6 +543,17 @@ int rtr_set_clean_checks(rtr_graph* g, int64_t first_wait_rounds, int64_t stack_
     return RTR_OK;
 }
 
+int rtr_set_device_limits(rtr_graph* g, int64_t graph_bytes, int64_t max_alloc)
+{
+    if (!g || graph_bytes < 0 || max_alloc < 0) {
+        set_error("rtr_set_device_limits: null graph or negative byte count");
+        return RTR_ERR_ARG;
+    }
+    g->device_limit = graph_bytes > 0 ? graph_bytes : INT64_MAX;
+    g->alloc_limit = max_alloc > 0 ? max_alloc : INT64_MAX;
+    return RTR_OK;
+}
+
 int rtr_set_clean_log(rtr_graph* g, int64_t max_bytes)
 {
     if (!g || max_bytes < -1) {

@@ -150,6 +150,9 @@ constexpr int64_t kPartsMax = 65535;
 // graph of 2,500 heavy edges left unused, and made the pool map new memory now and
 // then (a new graph's pass 22 ms, but up to 50).
 constexpr int64_t kListFirst = 1ll << 18;
+// Lists (with the clean's records) of up to this size may take the pool's cached
+// blocks without leaving a margin to others.
+constexpr double kListsSmall = 256.0 * (1ll << 20);
 
 struct HeavyArgs {
     const int64_t* off;
@@ -1125,10 +1128,37 @@ int count_triangles(rtr_graph* g)
         // later allocation reuses) and this graph's own rows-layout buffers
         const double use = (double)sizeof(TriEntry) * (double)(tl_len + 1) + 64.0 * (double)(m + 1);
         const double own = (double)(g->rows_masks_cap + g->rows_lists_cap + g->rows_ahead_cap);
-        // the pool's cached blocks alone may do; only then the device is not asked for its free
-        // memory, which takes 64 us, as long as the rest of a small graph's count
-        keep_lists = use <= (double)pool_cached_bytes(g) ||
-                     use + (double)(1ll << 30) <= (double)device_avail_bytes(g) + own;
+        const double margin = (double)(1ll << 30);
+        // small lists may come from the pool's cached blocks alone: the device is not asked for its
+        // free memory, which takes 64 us, as long as the rest of a small graph's count
+        keep_lists = (use <= kListsSmall && use <= (double)pool_cached_bytes(g)) ||
+                     use + margin <= (double)device_avail_bytes(g) + own;
+    }
+    if (keep_lists) {
+        if (pr.folding) {  // the lists are kept after all: they fold every vertex
+            RTR_CUDA_TRY(cudaStreamSynchronize(g->side));
+            pr.folding = false;
+        }
+        // the rows layout's buffers are not needed with lists
+        msc.reset();
+        moff = nullptr;
+        masks = nullptr;
+        release_owned(g, &g->rows_masks, &g->rows_masks_cap);
+        release_owned(g, &g->rows_lists, &g->rows_lists_cap);
+        release_owned(g, &g->rows_ahead, &g->rows_ahead_cap);
+        if (tl_len > g->tl_len || !g->tl) {
+            // grow-only buffer owned by the graph
+            TriEntry* tl = (TriEntry*)dev_alloc(g, sizeof(TriEntry) * (size_t)(tl_len + 1));
+            if (tl) {
+                g->tl = tl;
+            } else if (g->count_mode == 0) {
+                cudaGetLastError();  // less room than it looked: cached blocks in pieces, or taken by others
+                keep_lists = false;
+            } else {
+                set_error("device allocation failed for %lld triangle-list entries", (long long)tl_len);
+                return RTR_ERR_CUDA;
+            }
+        }
     }
     if (!keep_lists) {
         // rows layout: perVertex and heavy-edge perEdge straight from the CSR rows
@@ -1165,23 +1195,6 @@ int count_triangles(rtr_graph* g)
         cudaEventDestroy(e1);
         g->stage = 2;
         return RTR_OK;
-    }
-    if (pr.folding) {  // the lists are kept after all: they fold every vertex
-        RTR_CUDA_TRY(cudaStreamSynchronize(g->side));
-        pr.folding = false;
-    }
-    msc.reset();
-    // the rows layout's buffers are not needed with lists
-    release_owned(g, &g->rows_masks, &g->rows_masks_cap);
-    release_owned(g, &g->rows_lists, &g->rows_lists_cap);
-    release_owned(g, &g->rows_ahead, &g->rows_ahead_cap);
-    if (tl_len > g->tl_len || !g->tl) {
-        // grow-only buffer owned by the graph
-        g->tl = (TriEntry*)dev_alloc(g, sizeof(TriEntry) * (tl_len + 1));
-        if (!g->tl) {
-            set_error("device allocation failed for %lld triangle-list entries", (long long)tl_len);
-            return RTR_ERR_CUDA;
-        }
     }
     g->tl_len = tl_len;
     g->lists = true;

@@ -10,6 +10,7 @@
 #include "primitives.cuh"
 #include "rtr_graph.cuh"
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -44,6 +45,7 @@ void* dev_alloc(rtr_graph* g, size_t bytes)
 {
     void* p = nullptr;
     if (bytes == 0) bytes = 16;
+    if (bytes > (size_t)g->alloc_limit) return nullptr;
     if (cudaMallocAsync(&p, bytes, g->stream) != cudaSuccess) return nullptr;
     g->owned.push_back(p);
     g->owned_bytes += (int64_t)bytes;
@@ -69,6 +71,7 @@ void* Scratch::get(size_t bytes)
 {
     void* p = nullptr;
     if (bytes == 0) bytes = 16;
+    if (bytes > (size_t)g->alloc_limit) return nullptr;
     if (cudaMallocAsync(&p, bytes, g->stream) != cudaSuccess) return nullptr;
     ptrs.push_back(p);
     this->bytes += (int64_t)bytes;
@@ -102,7 +105,10 @@ size_t device_avail_bytes(rtr_graph* g)
 {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
-    return free_b + pool_cached_bytes(g);
+    const size_t avail = free_b + pool_cached_bytes(g);
+    if (g->device_limit == INT64_MAX) return avail;
+    const int64_t left = g->device_limit - g->owned_bytes - g->scratch_bytes;
+    return std::min(avail, (size_t)std::max<int64_t>(left, 0));
 }
 
 void release_owned(rtr_graph* g, void** buf, int64_t* cap)

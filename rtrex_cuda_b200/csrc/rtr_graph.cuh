@@ -138,6 +138,8 @@ struct rtr_graph {
     long long diag_residual = 0;
     long long diag_bad_status = 0;
 
+    // bytes of one device allocation, and of all that the graph holds, at most: lowered only in tests
+    int64_t alloc_limit = INT64_MAX, device_limit = INT64_MAX;
     std::vector<void*> owned;  // device allocations released by rtr_graph_destroy
     // device bytes: held by the graph (owned), and temporary scratch now / at most
     int64_t owned_bytes = 0;
