@@ -51,6 +51,8 @@
 #include "rowsets.cuh"
 #include "rtr_graph.cuh"
 
+#include <algorithm>
+
 namespace rtr {
 
 namespace {
@@ -692,6 +694,7 @@ int build_row_sets(rtr_graph* g, Scratch& sc, int min_deg, RowSets* out)
 // with the count itself slower, none ahead: 60.7 and 136 for 50.5 and 120 with 32;
 // scale 22 637 for 607).  The blocks keep to two an SM's shared memory
 // (kBlockFoldSmem): given an SM each, scale 19 takes 39.5 ms.
+constexpr int64_t kListsMargin = 1ll << 30;  // device memory that the rows layout's lists leave
 constexpr int kPriRows = 32;
 constexpr int kPriDegree = 2048;
 
@@ -775,10 +778,13 @@ int fold_priority_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, PriorityRow
     RTR_CUDA_TRY(cudaMemcpyAsync(&entries, lpos + S, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     if (const int rc = read_words(g, &nseg, segoff + k, sizeof(int64_t))) return rc;
     g->launches += 2 + take_primitive_launches();
-    // a graph-owned buffer (reused by later counts) of at most an eighth of the free memory: a
-    // smaller row's list then fits in what is left
+    // a graph-owned buffer (reused by later counts) of at most an eighth of the free memory, beside
+    // which any other row's list (a term is an edge: at most m) and its count's scratch still fit
     const int64_t bytes = (int64_t)sizeof(int32_t) * (entries + 1);
-    if (g->rows_ahead_cap < bytes && bytes > (int64_t)((device_avail_bytes(g) + g->rows_ahead_cap) / 8)) {
+    const int64_t avail = (int64_t)device_avail_bytes(g) + g->rows_ahead_cap;
+    const int64_t rest = kListsMargin + (int64_t)sizeof(int32_t) * (g->m + 1) + 64 * g->n + (16ll << 20);
+    if ((g->rows_ahead_cap < bytes && bytes > avail / 8) ||
+        std::max(bytes, g->rows_ahead_cap) + rest > avail + g->rows_lists_cap) {
         release_owned(g, &g->rows_ahead, &g->rows_ahead_cap);
         return RTR_OK;
     }
@@ -892,7 +898,7 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const PriorityRows&
     }
     // the lists: all of them when they fit in the free HBM (less 1 GiB), else windows of whole
     // rows; a graph-owned buffer, reused by later counts of the graph
-    const int64_t margin = 1ll << 30;
+    const int64_t margin = kListsMargin;
     int64_t room = 0;
     int32_t* lists = nullptr;
     if (g->rows_lists_cap >= (int64_t)sizeof(int32_t) * (want + 1)) {
