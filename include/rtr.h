@@ -195,6 +195,15 @@ int rtr_set_clean_checks(rtr_graph* g, int64_t first_wait_rounds, int64_t stack_
  * max_alloc bytes fails.  0, the default of both: the device's own limits. */
 int rtr_set_device_limits(rtr_graph* g, int64_t graph_bytes, int64_t max_alloc);
 
+/* The library's device sort on keys[n], stably by bits [lo, hi) into out[n], to
+ * test its forms (no counterpart in the reference).  wait_limit is the polls of an
+ * earlier tile before its keys are counted instead, one_region_from and wide_from
+ * the key counts from which the passes share one region of status words and those
+ * words are 64 bits; -1 leaves each as it is.  Bits above hi that share its last
+ * digit of 8 (from lo) must be zero. */
+int rtr_sort_keys(const uint64_t* keys, int64_t n, int lo, int hi, int64_t wait_limit, int64_t one_region_from,
+                  int64_t wide_from, int device, uint64_t* out);
+
 /* Autotuner: times the counting pass on this graph for gallop ratios
  * {4,8,16,32,64}, then heavy degrees {8,16,32,64,128}, then heavy-edge degree
  * sums {128,256,512,1024,4096,off} (coordinate descent, each candidate timed by

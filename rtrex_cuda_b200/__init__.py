@@ -112,6 +112,7 @@ def lib():
     L.rtr_graph_create_rmat.argtypes = [ctypes.c_int, _i64, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                         ctypes.c_uint64, ctypes.c_int, P(_vp)]
     L.rtr_set_clean_split.argtypes = [_vp, _i64, ctypes.c_double]
+    L.rtr_sort_keys.argtypes = [_vp, _i64, ctypes.c_int, ctypes.c_int, _i64, _i64, _i64, ctypes.c_int, _vp]
     L.rtr_set_clean_log.argtypes = [_vp, _i64]
     L.rtr_set_device_limits.argtypes = [_vp, _i64, _i64]
     L.rtr_set_clean_checks.argtypes = [_vp, _i64, _i64]

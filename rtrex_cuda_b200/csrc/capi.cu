@@ -543,6 +543,42 @@ int rtr_set_clean_checks(rtr_graph* g, int64_t first_wait_rounds, int64_t stack_
     return RTR_OK;
 }
 
+int rtr_sort_keys(const uint64_t* keys, int64_t n, int lo, int hi, int64_t wait_limit, int64_t one_region_from,
+                  int64_t wide_from, int device, uint64_t* out)
+{
+    if (n < 0 || (n > 0 && (!keys || !out)) || lo < 0 || hi < lo || hi > 64 || wait_limit < -1 ||
+        one_region_from < -1 || wide_from < -1) {
+        set_error("rtr_sort_keys: null array, bits outside 0..64 or a limit below -1");
+        return RTR_ERR_ARG;
+    }
+    rtr_graph* g = nullptr;
+    int rc = make_graph(1, device, &g);  // its stream
+    if (rc) return rc;
+    {
+        SortForms forms;
+        if (wait_limit >= 0) forms.wait_limit = (long)wait_limit;
+        if (one_region_from >= 0) forms.one_region_from = one_region_from;
+        if (wide_from >= 0) forms.wide_from = wide_from;
+        Scratch sc(g);
+        uint64_t* k1 = (uint64_t*)sc.get(sizeof(uint64_t) * (size_t)n);
+        uint64_t* k2 = (uint64_t*)sc.get(sizeof(uint64_t) * (size_t)n);
+        void* tmp = sc.get(radix_temp_bytes(n, forms));
+        auto sorted = [&]() -> int {
+            if (!k1 || !k2 || !tmp) {
+                set_error("device allocation failed (sort)");
+                return RTR_ERR_CUDA;
+            }
+            RTR_CUDA_TRY(cudaMemcpyAsync(k1, keys, sizeof(uint64_t) * (size_t)n, cudaMemcpyHostToDevice, g->stream));
+            const uint64_t* s = radix_sort_bits_u64(k1, k2, n, lo, hi, tmp, g->stream, forms);
+            RTR_CUDA_TRY(cudaGetLastError());
+            return read_words(g, out, s, sizeof(uint64_t) * (size_t)n);
+        };
+        if (n > 0) rc = sorted();
+    }
+    rtr_graph_destroy(g);
+    return rc;
+}
+
 int rtr_set_device_limits(rtr_graph* g, int64_t graph_bytes, int64_t max_alloc)
 {
     if (!g || graph_bytes < 0 || max_alloc < 0) {

@@ -160,7 +160,9 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_sort_one(const uint64_t* __
 constexpr int kMaxDigits = 8;
 constexpr int kPassItems = 16;
 constexpr int kPassTile = kBlock * kPassItems;  // 4096 keys per tile of a digit's pass
-constexpr long kLookbackLimit = 1l << 28;       // polls of an earlier tile before the wait is given up
+constexpr long kLookbackLimit = 1l << 21;       // polls of an earlier tile (a second) before it is counted instead
+constexpr int64_t kOneRegionFrom = (1ll << 24) + 1;  // keys from which the passes share one region of status words
+constexpr int64_t kWideFrom = 1ll << 30;             // keys from which a status word is 64 bits
 
 // Every digit's histogram in one read of the keys.
 __global__ void __launch_bounds__(kBlock) k_radix_hist(const uint64_t* __restrict__ keys, int64_t n, int lo,
@@ -184,13 +186,15 @@ __global__ void __launch_bounds__(kBlock) k_radix_hist(const uint64_t* __restric
 // keys are ranked by warp, its digit counts published, and each digit's offset
 // found by looking back over the earlier tiles (status word: 0 not yet, 1 the
 // tile's own count, 2 the count through the tile, in the top two bits).  A tile
-// only waits for tiles taken before it, whose blocks are running.
+// only waits for tiles taken before it, whose blocks are running; should a wait
+// run out all the same (wait_limit polls), the thread counts its digit in that
+// tile's keys itself and goes on, so that no wait can end in a wrong place.
 template <typename S>
 __global__ void __launch_bounds__(kBlock) k_radix_pass(const uint64_t* __restrict__ keys, uint64_t* __restrict__ out,
                                                         int64_t n, int shift,
                                                         const unsigned long long* __restrict__ hist,
                                                         S* __restrict__ status, unsigned* __restrict__ next_tile,
-                                                        unsigned* __restrict__ err)
+                                                        long wait_limit)
 {
     constexpr int kWarps = kBlock / 32;
     constexpr int kShift = 8 * sizeof(S) - 2;
@@ -253,12 +257,13 @@ __global__ void __launch_bounds__(kBlock) k_radix_pass(const uint64_t* __restric
         const unsigned f = (unsigned)(x >> kShift);
         if (f == 0) {
             long spin = 0;
-            while ((st[p * kBins] >> kShift) == 0 && ++spin < kLookbackLimit) {
+            bool there = false;
+            while (spin++ < wait_limit && !(there = (st[p * kBins] >> kShift) != 0)) {
             }
-            if (spin >= kLookbackLimit) {
-                atomicExch(err, 1u);
-                break;
-            }
+            if (there) continue;
+            const uint64_t* k0 = keys + p * kPassTile;  // an earlier tile is a whole one
+            for (int i = 0; i < kPassTile; ++i) before += ((k0[i] >> shift) & (kBins - 1)) == (uint64_t)t ? 1 : 0;
+            --p;
             continue;
         }
         before += x & kMask;
@@ -291,13 +296,13 @@ struct RadixPlan {
     int64_t tiles, words;
     bool wide;  // 64-bit words: counts of 2^30 and more
     int64_t regions;
-    explicit RadixPlan(int64_t n)
-        : tiles((n + kPassTile - 1) / kPassTile), words(tiles * kBins), wide(n >= (1ll << 30)),
-          regions(n <= (1ll << 24) ? kMaxDigits : 1)
+    RadixPlan(int64_t n, const SortForms& f)
+        : tiles((n + kPassTile - 1) / kPassTile), words(tiles * kBins), wide(n >= std::min(f.wide_from, kWideFrom)),
+          regions(n < f.one_region_from ? kMaxDigits : 1)
     {
     }
     size_t region_bytes() const { return (size_t)words * (wide ? 8 : 4); }
-    // histograms, tile counters and the error word, then the regions
+    // histograms and tile counters, then the regions
     static constexpr size_t kHead = sizeof(unsigned long long) * kMaxDigits * kBins + sizeof(unsigned) * 64;
     size_t bytes() const { return kHead + region_bytes() * (size_t)regions; }
 };
@@ -321,12 +326,14 @@ int exclusive_scan_i64(const int64_t* d_in, int64_t* d_out, int64_t n, int64_t* 
     return scan_impl<int64_t>(d_in, d_out, n, d_total, temp, s);
 }
 
-size_t radix_temp_bytes(int64_t n)
+SortForms::SortForms() : wait_limit(kLookbackLimit), one_region_from(kOneRegionFrom), wide_from(kWideFrom) {}
+
+size_t radix_temp_bytes(int64_t n, const SortForms& forms)
 {
     // enough for any smaller n too
     if (n <= kSortOne) return 16;
-    const size_t b = RadixPlan(n).bytes();
-    return n > (1ll << 24) ? std::max(b, RadixPlan(1ll << 24).bytes()) : b;
+    const size_t b = RadixPlan(n, forms).bytes();
+    return n >= forms.one_region_from ? std::max(b, RadixPlan(forms.one_region_from - 1, forms).bytes()) : b;
 }
 
 uint64_t* radix_sort_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int nbits, void* temp, cudaStream_t s)
@@ -342,7 +349,7 @@ int64_t take_primitive_launches()
 }
 
 uint64_t* radix_sort_bits_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int lo, int hi, void* temp,
-                              cudaStream_t s)
+                              cudaStream_t s, const SortForms& forms)
 {
     if (n <= 1 || hi <= lo) return d_keys;
     if (n <= kSortOne) {
@@ -352,11 +359,10 @@ uint64_t* radix_sort_bits_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int 
         t_launches += 1;
         return d_alt;
     }
-    const RadixPlan plan(n);
+    const RadixPlan plan(n, forms);
     const int digits = (hi - lo + kRadixBits - 1) / kRadixBits;
     unsigned long long* hist = (unsigned long long*)temp;
     unsigned* next = (unsigned*)(hist + kMaxDigits * kBins);
-    unsigned* err = next + kMaxDigits;
     unsigned char* status = (unsigned char*)temp + RadixPlan::kHead;
     const bool own = plan.regions > 1;
     cudaMemsetAsync(temp, 0, RadixPlan::kHead + (own ? plan.region_bytes() * (size_t)digits : 0), s);
@@ -369,10 +375,10 @@ uint64_t* radix_sort_bits_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int 
         const int shift = lo + d * kRadixBits;
         if (plan.wide)
             k_radix_pass<unsigned long long><<<(unsigned)plan.tiles, kBlock, 0, s>>>(
-                src, dst, n, shift, hist + d * kBins, (unsigned long long*)st, next + d, err);
+                src, dst, n, shift, hist + d * kBins, (unsigned long long*)st, next + d, forms.wait_limit);
         else
             k_radix_pass<uint32_t><<<(unsigned)plan.tiles, kBlock, 0, s>>>(src, dst, n, shift, hist + d * kBins,
-                                                                           (uint32_t*)st, next + d, err);
+                                                                           (uint32_t*)st, next + d, forms.wait_limit);
         std::swap(src, dst);
     }
     t_launches += 1 + digits;

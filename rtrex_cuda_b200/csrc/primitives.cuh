@@ -18,13 +18,21 @@ int exclusive_scan_i64(const int64_t* d_in, int64_t* d_out, int64_t n, int64_t* 
 // Stable LSD radix sort of n uint64 keys over bits [0, nbits).  Uses d_alt as
 // the ping-pong buffer; returns the buffer that holds the sorted keys
 // (d_keys or d_alt).  temp must hold radix_temp_bytes(n) bytes.
-size_t radix_temp_bytes(int64_t n);
+//
+// The tiled sort's forms (primitives.cu): their lines as they are, or lowered to
+// reach each form with few keys.
+struct SortForms {
+    long wait_limit;
+    int64_t one_region_from, wide_from;
+    SortForms();
+};
+size_t radix_temp_bytes(int64_t n, const SortForms& forms = SortForms());
 uint64_t* radix_sort_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int nbits, void* temp,
                          cudaStream_t s);
 
 // The same over bits [lo, hi) only.
 uint64_t* radix_sort_bits_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int lo, int hi, void* temp,
-                              cudaStream_t s);
+                              cudaStream_t s, const SortForms& forms = SortForms());
 
 // Kernels that the calling thread's scans and sorts have launched since it last asked.
 int64_t take_primitive_launches();
