@@ -5,7 +5,7 @@ every CUDA / C++ source under ``csrc/`` with nvcc for ``sm_100a`` and links
 ``rtrex_cuda_b200/librtr.so`` plus the ``rtrex_cuda_b200/rtrex_b200`` binary.
 Objects go to ``rtrex_cuda_b200/_build/``.  Floating-point contraction is
 disabled (``-fmad=false``) so every add / multiply rounds as the reference's
-x86-64 SSE2 code does.
+x86-64 SSE2 code does.  A scan or sort whose status the caller drops is an error.
 """
 from __future__ import annotations
 
@@ -23,7 +23,7 @@ LIB = os.path.join(HERE, "librtr.so")
 CLI = os.path.join(HERE, "rtrex_b200")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVFLAGS = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC,-O2",
+NVFLAGS = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC,-O2,-Werror=unused-result",
            "-I" + os.path.join(ROOT, "include")]
 SOURCES = ["primitives.cu", "graph.cu", "count.cu", "count_rows.cu", "clean.cu", "clean_rounds.cu", "extract.cu", "capi.cu", "io.cpp", "noalloc.cu", "components.cu", "expand.cu", "escape.cu", "serve.cpp", "gen.cu", "nucleus.cu"]
 

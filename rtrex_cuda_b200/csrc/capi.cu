@@ -569,8 +569,8 @@ int rtr_sort_keys(const uint64_t* keys, int64_t n, int lo, int hi, int64_t wait_
                 return RTR_ERR_CUDA;
             }
             RTR_CUDA_TRY(cudaMemcpyAsync(k1, keys, sizeof(uint64_t) * (size_t)n, cudaMemcpyHostToDevice, g->stream));
-            const uint64_t* s = radix_sort_bits_u64(k1, k2, n, lo, hi, tmp, g->stream, forms);
-            RTR_CUDA_TRY(cudaGetLastError());
+            uint64_t* s = nullptr;
+            RTR_TRY(radix_sort_bits_u64(k1, k2, n, lo, hi, tmp, g->stream, &s, forms));
             return read_words(g, out, s, sizeof(uint64_t) * (size_t)n);
         };
         if (n > 0) rc = sorted();

@@ -780,7 +780,7 @@ int initial_clean(rtr_graph* g, double eps)
     RTR_CUDA_TRY(cudaMemsetAsync(ecount, 0, sizeof(uint32_t) * (n + 1), s));
     RTR_CUDA_TRY(cudaMemsetAsync(tsum, 0, sizeof(unsigned long long) * (n + 1), s));
     k_unit_edges<<<gm, kBlock, 0, s>>>(g->esrc, g->fwd, m, g->sup, root, ecount, tsum);
-    exclusive_scan_u32(is_seed, spos, m, d_ns, stmp, s);
+    RTR_TRY(exclusive_scan_u32(is_seed, spos, m, d_ns, stmp, s));
     g->launches += 5 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     uint32_t ns = 0;
@@ -812,9 +812,9 @@ int initial_clean(rtr_graph* g, double eps)
         uint32_t nu = ns;  // the buffers' bound, then the number
         g->launches += 1;
         if (!small) {
-            sorted = radix_sort_u64(keys, alt, ns, kbits, rtmp, s);
+            RTR_TRY(radix_sort_u64(keys, alt, ns, kbits, rtmp, s, &sorted));
             k_unit_heads<<<gs, kBlock, 0, s>>>(sorted, ns, rbits, head);
-            exclusive_scan_u32(head, hpos, ns, d_ns + 1, htmp, s);
+            RTR_TRY(exclusive_scan_u32(head, hpos, ns, d_ns + 1, htmp, s));
             k_seed_info<<<gs, kBlock, 0, s>>>(sorted, ns, rmask, g->fwd, g->esrc, g->nbors, g->deg, rec, seeds);
             g->launches += 2 + take_primitive_launches();
             if (const int rc = read_words(g, &nu, d_ns + 1, sizeof(uint32_t))) return rc;
@@ -851,11 +851,11 @@ int initial_clean(rtr_graph* g, double eps)
             k_unit_class<<<grid_for(nu, kBlock), kBlock, 0, s>>>(units, nu, ns, ecount, tsum, rule, cls,
                                                                  (unsigned long long*)(d_tot + 1),
                                                                  (unsigned*)(d_tot + 2));
-            exclusive_scan_i64(cap, capoff, nu, d_tot, ctmp, s);
+            RTR_TRY(exclusive_scan_i64(cap, capoff, nu, d_tot, ctmp, s));
             k_unit_finish<<<grid_for(nu, kBlock), kBlock, 0, s>>>(units, cap, capoff, nu, cls, okeys,
                                                                   g->clean_stack_limit);
             // units ascend in the keys' low half already
-            order = radix_sort_bits_u64(okeys, oalt, nu, 32, 64, otmp, s);
+            RTR_TRY(radix_sort_bits_u64(okeys, oalt, nu, 32, 64, otmp, s, &order));
             g->launches += 3 + take_primitive_launches();
         }
         RTR_CUDA_TRY(cudaGetLastError());

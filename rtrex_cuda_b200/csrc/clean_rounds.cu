@@ -785,12 +785,13 @@ int clean_rounds_finish(rtr_graph* g, RoundReplay* rr)
     // an unused key keeps a vertex past the last
     RTR_CUDA_TRY(cudaMemsetAsync(rr->keys, 0xff, sizeof(uint64_t) * (size_t)cnt, s));
     k_pop_counts<<<grid_for(pops, kBlock), kBlock, 0, s>>>(rr->plog, pops, rr->pcnt);
-    exclusive_scan_u32(rr->pcnt, rr->poff, pops, nullptr, rr->ptmp, s);
+    RTR_TRY(exclusive_scan_u32(rr->pcnt, rr->poff, pops, nullptr, rr->ptmp, s));
     k_log_keys<<<grid_for(8 * pops, kBlock), kBlock, 0, s>>>(rr->rec, rr->plog, rr->poff, pops, g->tl, rr->live8,
                                                              g->fwd, g->esrc, g->nbors, 1 / (double)g->n, lb,
                                                              rr->keys, rr->wlog, (unsigned*)(g->ctr + 1), g->ctr + 2);
     // the keys come in log order, so a stable sort on the vertex bits suffices
-    uint64_t* sorted = radix_sort_bits_u64(rr->keys, rr->alt, cnt, lb, lb + vb, rr->rtmp, s);
+    uint64_t* sorted = nullptr;
+    RTR_TRY(radix_sort_bits_u64(rr->keys, rr->alt, cnt, lb, lb + vb, rr->rtmp, s, &sorted));
     k_log_gather<<<grid_for(cnt, kBlock), kBlock, 0, s>>>(sorted, cnt, g->n, lb, rr->wlog, rr->ws, g->pv, rr->runs,
                                                           rr->nruns);
     k_fold_long_runs<<<grid_for(1ll << 40, 128, 8), 128, 0, s>>>(rr->runs, rr->nruns, sorted, lb, rr->ws, g->pv);

@@ -209,7 +209,7 @@ int connected_components(rtr_graph* g)
     k_cc_init<<<gn, kBlock, 0, s>>>(root, key, vis, n);
     k_cc_hook<<<gm, kBlock, 0, s>>>(g->esrc, g->nbors, g->fwd, m, root);
     k_cc_flatten<<<gn, kBlock, 0, s>>>(root, n, is_root);
-    exclusive_scan_u32(is_root, pos, n, d_cnt, tmp, s);
+    RTR_TRY(exclusive_scan_u32(is_root, pos, n, d_cnt, tmp, s));
     k_cc_roots<<<gn, kBlock, 0, s>>>(is_root, pos, n, fa, vis, seq);
     g->launches += 4 + take_primitive_launches();
     uint32_t ncomp = 0;
@@ -222,7 +222,7 @@ int connected_components(rtr_graph* g)
         const int gf = grid_for(nf, kBlock);
         k_cc_offer<<<gf, kBlock, 0, s>>>(cur, nf, g->offsets, g->nbors, vis, key);
         k_cc_count<<<gf, kBlock, 0, s>>>(cur, nf, g->offsets, g->nbors, vis, key, cnt);
-        exclusive_scan_u32(cnt, base, nf, d_cnt + 1, tmp, s);
+        RTR_TRY(exclusive_scan_u32(cnt, base, nf, d_cnt + 1, tmp, s));
         k_cc_write<<<gf, kBlock, 0, s>>>(cur, nf, g->offsets, g->nbors, vis, key, base, nxt);
         g->launches += 3 + take_primitive_launches();
         uint32_t nn = 0;
@@ -260,9 +260,10 @@ int connected_components(rtr_graph* g)
     }
     k_cc_keys<<<gn, kBlock, 0, s>>>(root, seq, n, B, k1);
     k_cc_by_seq<<<gn, kBlock, 0, s>>>(seq, n, by_seq);
-    uint64_t* sorted = radix_sort_u64(k1, k2, n, 2 * B, rtmp, s);
+    uint64_t* sorted = nullptr;
+    RTR_TRY(radix_sort_u64(k1, k2, n, 2 * B, rtmp, s, &sorted));
     k_cc_unpack<<<gn, kBlock, 0, s>>>(sorted, n, B, by_seq, g->cc_vert, is_root);
-    exclusive_scan_u32(is_root, pos, n, nullptr, tmp, s);
+    RTR_TRY(exclusive_scan_u32(is_root, pos, n, nullptr, tmp, s));
     k_cc_offsets<<<gn, kBlock, 0, s>>>(is_root, pos, n, g->cc_off);
     RTR_CUDA_TRY(cudaMemcpyAsync(g->cc_off + ncomp, &n, sizeof(int64_t), cudaMemcpyHostToDevice, s));
     g->launches += 4 + take_primitive_launches();

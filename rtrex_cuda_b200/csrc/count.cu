@@ -884,7 +884,7 @@ int cut_runs(rtr_graph* g, Scratch& sc, const RowSets& rs, int64_t nh, const int
     k_fwd_start<<<grid_for(n, 256), 256, 0, s>>>(g->offsets, g->nbors, n, fstart);
     k_run_ends<<<grid_for(nh, 256), 256, 0, s>>>(*runs, nh, first, last);
     k_piece_counts<<<grid_for(2 * n + 1, 256), 256, 0, s>>>(first, last, pre, rs, n, pcnt);
-    exclusive_scan_i64(pcnt, poff, 2 * n + 1, nullptr, tmp, s);
+    RTR_TRY(exclusive_scan_i64(pcnt, poff, 2 * n + 1, nullptr, tmp, s));
     g->launches += 3 + take_primitive_launches();
     int64_t all = 0;
     if (const int rc = read_words(g, &np[0], poff + n, sizeof(int64_t))) return rc;
@@ -1043,7 +1043,8 @@ int count_triangles(rtr_graph* g)
             const int nbits = bits_for((uint64_t)(n > 0 ? n - 1 : 0));
             k_heavy_keys<<<grid_for(nh, 256), 256, 0, s>>>(g->offsets, g->esrc, g->nbors, g->fwd, heavy_list, nh,
                                                             pr.rank, nbits, hkeys, nheavy + 1);
-            const uint64_t* sorted = radix_sort_u64(hkeys, halt, nh, nbits + (pr.count > 0 ? 1 : 0), htmp, s);
+            uint64_t* sorted = nullptr;
+            RTR_TRY(radix_sort_u64(hkeys, halt, nh, nbits + (pr.count > 0 ? 1 : 0), htmp, s, &sorted));
             unsigned npri = 0;
             if (const int rc = read_words(g, &npri, nheavy + 1, sizeof npri)) return rc;
             pr.edges = npri;
@@ -1073,7 +1074,7 @@ int count_triangles(rtr_graph* g)
             }
             k_mask_words<<<grid_for(nh + 1, 256), 256, 0, s>>>(g->offsets, g->esrc, g->nbors, g->fwd, heavy_list,
                                                                 nh, rs, wcount);
-            exclusive_scan_i64(wcount, moff, nh + 1, nullptr, wtmp, s);
+            RTR_TRY(exclusive_scan_i64(wcount, moff, nh + 1, nullptr, wtmp, s));
             int64_t words = 0;
             if (const int rc = read_words(g, &words, moff + nh, sizeof(int64_t))) return rc;
             if (runs.keys && n <= (1ll << kMaxBits) && nh >= kBitsEdges) {
@@ -1113,7 +1114,7 @@ int count_triangles(rtr_graph* g)
     ktime_end(g, KT_EDGE_HEAVY);
     if (rs.tab) light(nullptr);
     ktime_end(g, KT_EDGE_FOLD);
-    exclusive_scan_i64(cnt, g->tl_off, m2 + 1, (int64_t*)(g->ctr + 4), tmp, s);
+    RTR_TRY(exclusive_scan_i64(cnt, g->tl_off, m2 + 1, (int64_t*)(g->ctr + 4), tmp, s));
     g->launches += 2 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     unsigned long long words[2] = {0, 0};  // list entries, heavy edges (low half)
@@ -1207,7 +1208,7 @@ int count_triangles(rtr_graph* g)
     cudaStream_t hs = s;  // the heavy lists'
     ktime_begin(g, KT_TRI_FILL);
     // cnt (scanned into tl_off above) is free: it takes the terms' offsets
-    if (terms) exclusive_scan_i64(cgt, cnt, m2 + 1, nullptr, tmp, s);
+    if (terms) RTR_TRY(exclusive_scan_i64(cgt, cnt, m2 + 1, nullptr, tmp, s));
     auto gather = [&](int lo, int hi, cudaStream_t st) {
         k_fold_gather<<<grid_for(8 * m2, kBlock), kBlock, 0, st>>>(g->esrc, g->nbors, g->partner, g->deg, lo, hi, m2,
                                                                    cgt, cnt, g->tl_off, g->tl, terms);

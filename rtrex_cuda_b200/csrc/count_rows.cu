@@ -652,7 +652,7 @@ int build_row_sets(rtr_graph* g, Scratch& sc, int min_deg, RowSets* out)
         return RTR_ERR_CUDA;
     }
     k_rs_flags<<<grid_for(n + 1, 256), 256, 0, s>>>(g->deg, n, min_deg, flag);
-    exclusive_scan_i64(flag, num, n + 1, nullptr, tmp, s);
+    RTR_TRY(exclusive_scan_i64(flag, num, n + 1, nullptr, tmp, s));
     int64_t nt = 0;
     if (const int rc = read_words(g, &nt, num + n, sizeof(int64_t))) return rc;
     g->launches += 2;
@@ -668,7 +668,7 @@ int build_row_sets(rtr_graph* g, Scratch& sc, int min_deg, RowSets* out)
     }
     RTR_CUDA_TRY(cudaMemsetAsync(tsize + nt, 0, sizeof(int64_t), s));
     k_rs_sizes<<<grid_for(n, 256), 256, 0, s>>>(g->deg, n, num, tab, owner, tbits, tsize);
-    exclusive_scan_i64(tsize, toff, nt + 1, nullptr, ltmp, s);
+    RTR_TRY(exclusive_scan_i64(tsize, toff, nt + 1, nullptr, ltmp, s));
     int64_t total = 0;
     if (const int rc = read_words(g, &total, toff + nt, sizeof(int64_t))) return rc;
     int32_t* slot = (int32_t*)sc.get(sizeof(int32_t) * (total + 1));
@@ -723,7 +723,8 @@ int pick_priority_rows(rtr_graph* g, Scratch& sc, PriorityRows* pr)
         cudaGetLastError();  // no room: every row goes with the rest
         return RTR_OK;
     }
-    const uint64_t* sorted = radix_sort_u64(keys, alt, found, 64, rtmp, s);
+    uint64_t* sorted = nullptr;
+    RTR_TRY(radix_sort_u64(keys, alt, found, 64, rtmp, s, &sorted));
     const int64_t k = found < (unsigned)kPriRows ? found : kPriRows;
     uint64_t h[kPriRows];
     if (const int rc = read_words(g, h, sorted, sizeof(uint64_t) * k)) return rc;
@@ -771,9 +772,9 @@ int fold_priority_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, PriorityRow
     }
     k_pri_counts<<<(unsigned)k, 256, 0, s>>>(g->offsets, pr->rows, pr->base, k, const_cast<int64_t*>(cgt), false, cnt);
     RTR_CUDA_TRY(cudaMemsetAsync(cnt + S, 0, sizeof(int64_t), s));
-    exclusive_scan_i64(cnt, lpos, S + 1, nullptr, tmp, s);
+    RTR_TRY(exclusive_scan_i64(cnt, lpos, S + 1, nullptr, tmp, s));
     k_seg_counts<<<1, 64, 0, s>>>(g->offsets, lpos, pr->base, pr->rows, k, scnt);
-    exclusive_scan_i64(scnt, segoff, k + 1, nullptr, tmp, s);
+    RTR_TRY(exclusive_scan_i64(scnt, segoff, k + 1, nullptr, tmp, s));
     int64_t entries = 0, nseg = 0;
     RTR_CUDA_TRY(cudaMemcpyAsync(&entries, lpos + S, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     if (const int rc = read_words(g, &nseg, segoff + k, sizeof(int64_t))) return rc;
@@ -847,7 +848,7 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const PriorityRows&
         k_pri_counts<<<(unsigned)pr.count, 256, 0, s>>>(g->offsets, pr.rows, pr.base, pr.count, cgt, true, nullptr);
         g->launches += 1;
     }
-    exclusive_scan_i64(cgt, lpos, m2 + 1, nullptr, tmp, s);
+    RTR_TRY(exclusive_scan_i64(cgt, lpos, m2 + 1, nullptr, tmp, s));
     // a warp from warp_min terms, a thread block from 64 x warp_min
     const int64_t warp_min = g->count_hub;
     const int64_t block_min = 64 * warp_min;
@@ -868,7 +869,8 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const PriorityRows&
             set_error("device allocation failed (rows layout)");
             return RTR_ERR_CUDA;
         }
-        uint64_t* sorted = radix_sort_u64(keys, alt, nbig, 64, rtmp, s);
+        uint64_t* sorted = nullptr;
+        RTR_TRY(radix_sort_u64(keys, alt, nbig, 64, rtmp, s, &sorted));
         k_low_ids<<<grid_for(nbig, 256), 256, 0, s>>>(sorted, nbig, big);
         g->launches += 1 + take_primitive_launches();
     }
@@ -884,7 +886,7 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const PriorityRows&
             return RTR_ERR_CUDA;
         }
         k_seg_counts<<<grid_for(nhuge + 1, 256), 256, 0, s>>>(g->offsets, lpos, nullptr, big, nhuge, scnt);
-        exclusive_scan_i64(scnt, segoff, nhuge + 1, nullptr, stmp, s);
+        RTR_TRY(exclusive_scan_i64(scnt, segoff, nhuge + 1, nullptr, stmp, s));
         int64_t nseg = 0;
         if (const int rc = read_words(g, &nseg, segoff + nhuge, sizeof(int64_t))) return rc;
         segslot = (int32_t*)sc.get(sizeof(int32_t) * (nseg + 1));

@@ -227,7 +227,7 @@ int parse_escape_device(rtr_graph* g, Scratch& sc, const char* h_text, FILE* f, 
         return RTR_ERR_CUDA;
     }
     k_nl_count<<<(unsigned)tiles, kBlock, 0, s>>>(text, len, tile_cnt);
-    exclusive_scan_i64(tile_cnt, tile_off, tiles, tile_off + tiles, ltmp, s);
+    RTR_TRY(exclusive_scan_i64(tile_cnt, tile_off, tiles, tile_off + tiles, ltmp, s));
     int64_t nnl = 0;
     RTR_CUDA_TRY(cudaMemcpyAsync(&nnl, tile_off + tiles, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     RTR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -253,7 +253,7 @@ int parse_escape_device(rtr_graph* g, Scratch& sc, const char* h_text, FILE* f, 
     if (nnl) k_nl_write<<<(unsigned)tiles, kBlock, 0, s>>>(text, len, tile_off, nlpos);
     if (L) {
         k_lines<<<grid_for(L, kBlock), kBlock, 0, s>>>(text, len, nlpos, nnl, L, is_data, va, vb, first);
-        exclusive_scan_u32(is_data, rank, L, ndata, utmp, s);
+        RTR_TRY(exclusive_scan_u32(is_data, rank, L, ndata, utmp, s));
     }
     g->launches += 6;
     RTR_CUDA_TRY(cudaGetLastError());

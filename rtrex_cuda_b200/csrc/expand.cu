@@ -434,7 +434,7 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
     RTR_CUDA_TRY(cudaMemsetAsync(moved, 0, n + 16, s));
     RTR_CUDA_TRY(cudaMemsetAsync(d_cnt, 0, sizeof(uint32_t) * 4, s));
     k_singleton_flags<<<gk, kBlock, 0, s>>>(g->cl_off, ncl, flag);
-    exclusive_scan_u32(flag, fpos, ncl, d_cnt, utmp, s);
+    RTR_TRY(exclusive_scan_u32(flag, fpos, ncl, d_cnt, utmp, s));
     g->launches += 4;
     uint32_t S32 = 0;
     RTR_CUDA_TRY(cudaMemcpyAsync(&S32, d_cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -457,7 +457,7 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
     if (S > 0) {
         k_singleton_list<<<gk, kBlock, 0, s>>>(flag, fpos, ncl, g->cl_off, g->cl_vert, g->offsets, s_cluster,
                                                s_vertex, vs, s_tab);
-        exclusive_scan_i64(s_tab, s_toff, S, s_toff + S, ltmp, s);
+        RTR_TRY(exclusive_scan_i64(s_tab, s_toff, S, s_toff + S, ltmp, s));
         g->launches += 4;
     }
     int64_t tab_total = 0;
@@ -496,8 +496,8 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
     RTR_CUDA_TRY(cudaMemsetAsync(inbound, 0, sizeof(uint32_t) * (ncl + 1), s));
     if (S > 0) k_inbound<<<gs, kBlock, 0, s>>>(s_best, S, inbound);
     k_caps<<<gk, kBlock, 0, s>>>(g->cl_off, ncl, inbound, sequential ? 1 : 0, ncap, bcap);
-    exclusive_scan_i64(ncap, noff, ncl, noff + ncl, ltmp, s);
-    exclusive_scan_i64(bcap, boff, ncl, boff + ncl, ltmp, s);
+    RTR_TRY(exclusive_scan_i64(ncap, noff, ncl, noff + ncl, ltmp, s));
+    RTR_TRY(exclusive_scan_i64(bcap, boff, ncl, boff + ncl, ltmp, s));
     g->launches += 9;
     int64_t caps[2] = {0, 0};
     RTR_CUDA_TRY(cudaMemcpyAsync(&caps[0], noff + ncl, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
@@ -539,7 +539,8 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
         RTR_CUDA_TRY(cudaStreamSynchronize(s));
         if (nm > 0) {
             const int nbits = sbits + bits_for((uint64_t)ncl);
-            uint64_t* sorted = radix_sort_u64(mk, malt, nm, nbits, rtmp, s);
+            uint64_t* sorted = nullptr;
+            RTR_TRY(radix_sort_u64(mk, malt, nm, nbits, rtmp, s, &sorted));
             k_apply_parallel<<<grid_for(nm, kBlock), kBlock, 0, s>>>(st, sorted, nm, sbits, s_vertex, err);
             g->launches += 1 + take_primitive_launches();
         }
@@ -550,7 +551,7 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
     // new membership, statistics, scores
     int64_t* nsz = ncap;  // capacities are no longer needed
     k_new_sizes<<<gk, kBlock, 0, s>>>(st, g->cl_off, g->cl_vert, ncl, moved, nsz);
-    exclusive_scan_i64(nsz, g->x_off, ncl, g->x_off + ncl, ltmp, s);
+    RTR_TRY(exclusive_scan_i64(nsz, g->x_off, ncl, g->x_off + ncl, ltmp, s));
     RTR_CUDA_TRY(cudaMemsetAsync(g->x_cof, 0xff, sizeof(int32_t) * (n + 1), s));
     k_emit<<<gk, kBlock, 0, s>>>(st, g->cl_off, g->cl_vert, ncl, g->x_off, g->x_vert, g->x_cof);
     RTR_CUDA_TRY(cudaMemsetAsync(g->x_ne, 0, sizeof(int64_t) * (ncl + 1), s));
@@ -565,7 +566,7 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
         return RTR_ERR_CUDA;
     }
     k_u8_to_u32<<<gn, kBlock, 0, s>>>(moved, n, m32);
-    exclusive_scan_u32(m32, mpos, n, d_cnt + 2, utmp, s);
+    RTR_TRY(exclusive_scan_u32(m32, mpos, n, d_cnt + 2, utmp, s));
     k_scores<<<gn, kBlock, 0, s>>>(moved, mpos, n, vs, s_score, g->x_scv, g->x_scx);
     g->launches += 12;
     RTR_CUDA_TRY(cudaGetLastError());

@@ -1136,7 +1136,7 @@ int extract_clusters(rtr_graph* g)
         g->launches += 1;
     } else {
         k_iota_key_deg<<<gn, kBlock, 0, s>>>(g->deg, n, B, k1);
-        sorted = radix_sort_u64(k1, k2, n, dbits, rtmp, s);
+        RTR_TRY(radix_sort_u64(k1, k2, n, dbits, rtmp, s, &sorted));
         k_set_rank<<<gn, kBlock, 0, s>>>(sorted, n, bmask, rank, by_rank);
         k_uf_init<<<gn, kBlock, 0, s>>>(root, n);
         RTR_CUDA_TRY(cudaMemsetAsync(acount, 0, sizeof(uint32_t) * (n + 1), s));
@@ -1153,9 +1153,9 @@ int extract_clusters(rtr_graph* g)
         k_comp_keys<<<gn, kBlock, 0, s>>>(root, rank, n, B, k1 == sorted ? k2 : k1);
         uint64_t* ck = (k1 == sorted) ? k2 : k1;
         uint64_t* calt = sorted;  // rank/by_rank already captured; reuse as ping-pong
-        csorted = radix_sort_u64(ck, calt, n, 2 * B, rtmp, s);
+        RTR_TRY(radix_sort_u64(ck, calt, n, 2 * B, rtmp, s, &csorted));
         k_comp_heads<<<gn, kBlock, 0, s>>>(csorted, n, B, by_rank, head, vlist);
-        exclusive_scan_u32(head, hpos, n, d_nc, htmp, s);
+        RTR_TRY(exclusive_scan_u32(head, hpos, n, d_nc, htmp, s));
         g->launches += 2 + take_primitive_launches();
         RTR_CUDA_TRY(cudaGetLastError());
         if (const int rc = read_words(g, &nc, d_nc, sizeof(uint32_t))) return rc;
@@ -1195,11 +1195,11 @@ int extract_clusters(rtr_graph* g)
         RTR_CUDA_TRY(cudaMemsetAsync(d_tot, 0, sizeof(int64_t) * 5, s));
         k_big_count<<<gc, kBlock, 0, s>>>(comps, nc, g->extract_big, (unsigned*)(d_tot + 3),
                                           (unsigned long long*)(d_tot + 4));
-        exclusive_scan_i64(bneed, boff, nc, d_tot + 1, ltmp, s);
-        exclusive_scan_i64(sneed, soff, nc, d_tot + 2, ltmp, s);
+        RTR_TRY(exclusive_scan_i64(bneed, boff, nc, d_tot + 1, ltmp, s));
+        RTR_TRY(exclusive_scan_i64(sneed, soff, nc, d_tot + 2, ltmp, s));
         k_comp_finish<<<gc, kBlock, 0, s>>>(comps, nc, boff, soff, sneed, okeys, g->extract_big);
         // components ascend in the keys' low half already
-        order = radix_sort_bits_u64(okeys, oalt, nc, 32, 64, otmp, s);
+        RTR_TRY(radix_sort_bits_u64(okeys, oalt, nc, 32, 64, otmp, s, &order));
         g->launches += 4 + take_primitive_launches();
         if (const int rc = read_words(g, tots, d_tot, sizeof tots)) return rc;
     }
@@ -1309,7 +1309,7 @@ int extract_clusters(rtr_graph* g)
     int64_t ncl = n;  // the buffers' bound, then the number
     if (!small) {
         k_widen<<<gc, kBlock, 0, s>>>(a.ncl, ncl64, nc);
-        exclusive_scan_i64(ncl64, cpos, nc, (int64_t*)(g->ctr + 4), ltmp, s);
+        RTR_TRY(exclusive_scan_i64(ncl64, cpos, nc, (int64_t*)(g->ctr + 4), ltmp, s));
         g->launches += 1 + take_primitive_launches();
         if (const int rc = read_words(g, h, g->ctr, sizeof h, true)) return rc;
         if (failed()) return RTR_ERR_DEVICE;
@@ -1350,9 +1350,10 @@ int extract_clusters(rtr_graph* g)
     } else {
         RTR_CUDA_TRY(cudaMemsetAsync(size64, 0, sizeof(int64_t) * (ncl + 1), s));
         k_cluster_keys<<<gc, kBlock, 0, s>>>(comps, nc, a.ncl, cpos, a.hdr_seed, rank, B, ckeys);
-        uint64_t* csort = radix_sort_u64(ckeys, calt2, ncl, 2 * B, ctmp, s);
+        uint64_t* csort = nullptr;
+        RTR_TRY(radix_sort_u64(ckeys, calt2, ncl, 2 * B, ctmp, s, &csort));
         k_cluster_gather<<<gk, kBlock, 0, s>>>(csort, ncl, bmask, a.hdr_seed, a.hdr_size, g->cl_seed, size64);
-        exclusive_scan_i64(size64, g->cl_off, ncl + 1, counts + 1, ltmp, s);
+        RTR_TRY(exclusive_scan_i64(size64, g->cl_off, ncl + 1, counts + 1, ltmp, s));
         k_cluster_members<<<gk, kBlock, 0, s>>>(csort, ncl, n, bmask, a.hdr_start, g->cl_off, a.out_vert, g->cl_vert,
                                                 g->cluster_of);
         RTR_CUDA_TRY(cudaMemsetAsync(g->cl_ne, 0, sizeof(int64_t) * (ncl + 1), s));

@@ -306,7 +306,7 @@ int finish_csr(rtr_graph* g, unsigned long long* h_ctr)
         return RTR_ERR_CUDA;
     }
     k_fwd_flags<<<grid_for(m2, kBlock), kBlock, 0, s>>>(g->esrc, g->nbors, m2, flag);
-    exclusive_scan_u32(flag, pos, m2, nullptr, tmp, s);
+    RTR_TRY(exclusive_scan_u32(flag, pos, m2, nullptr, tmp, s));
     k_fwd_list<<<grid_for(m2, kBlock), kBlock, 0, s>>>(flag, pos, m2, g->fwd, g->frank);
     g->launches += 2 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
@@ -348,7 +348,8 @@ int build_csr(rtr_graph* g, const int64_t* d_u, const int64_t* d_v, int64_t m, b
     }
     RTR_CUDA_TRY(cudaMemsetAsync(g->ctr, 0, 8 * sizeof(unsigned long long), s));
     k_make_keys<<<grid_for(m, kBlock), kBlock, 0, s>>>(d_u, d_v, m, n, B, keys, g->ctr + 4);
-    uint64_t* sorted = radix_sort_u64(keys, alt, m2, 2 * B, rtmp, s);
+    uint64_t* sorted = nullptr;
+    RTR_TRY(radix_sort_u64(keys, alt, m2, 2 * B, rtmp, s, &sorted));
     g->launches += 1 + take_primitive_launches();
     uint32_t* keep = (uint32_t*)sc.get(sizeof(uint32_t) * (m2 + 1));
     if (!keep) {
@@ -374,7 +375,7 @@ int build_csr(rtr_graph* g, const int64_t* d_u, const int64_t* d_v, int64_t m, b
         uint32_t* tmp = (uint32_t*)sc.get(sizeof(uint32_t) * scan_temp_elems(m2));
         uint32_t* d_tot = (uint32_t*)sc.get(sizeof(uint32_t));
         uint64_t* out = (sorted == keys) ? alt : keys;
-        exclusive_scan_u32(keep, pos, m2, d_tot, tmp, s);
+        RTR_TRY(exclusive_scan_u32(keep, pos, m2, d_tot, tmp, s));
         k_compact_keys<<<grid_for(m2, kBlock), kBlock, 0, s>>>(sorted, keep, pos, m2, out);
         g->launches += 1 + take_primitive_launches();
         uint32_t tot = 0;

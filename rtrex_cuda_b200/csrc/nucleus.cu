@@ -521,7 +521,8 @@ int nucleus_run(rtr_graph* g)
         }
         const int gn = grid_for(n, kBlock);
         k_nuc_keys<<<gn, kBlock, 0, s>>>(g->deg, n, B, k1);
-        uint64_t* sorted = radix_sort_u64(k1, k2, n, B + bits_for((uint64_t)g->m2), rtmp, s);
+        uint64_t* sorted = nullptr;
+        RTR_TRY(radix_sort_u64(k1, k2, n, B + bits_for((uint64_t)g->m2), rtmp, s, &sorted));
         k_nuc_rank<<<gn, kBlock, 0, s>>>(sorted, n, mask, inv, newid);
         k_nuc_pairs<<<grid_for(m, kBlock), kBlock, 0, s>>>(g->fwd, g->esrc, g->nbors, newid, m, du, dv);
         g->launches += 3 + take_primitive_launches();
@@ -556,7 +557,7 @@ int nucleus_run(rtr_graph* g)
     if (!tc || !kappa || !comp || !carries || !cpos || !stmp || !next) return failed("edges");
     RTR_CUDA_TRY(cudaMemsetAsync(next, 0, sizeof(unsigned) * 8, rs));
     k_nuc_init<<<gm, kBlock, 0, rs>>>(r->fwd, r->sup, m, tc, kappa, comp, carries);
-    exclusive_scan_u32(carries, cpos, m, next + 4, stmp, rs);
+    RTR_TRY(exclusive_scan_u32(carries, cpos, m, next + 4, stmp, rs));
     k_nuc_unite<<<gm, kBlock, 0, rs>>>(r->fwd, r->nbors, r->tl_off, r->tl, m, comp);
     g->launches += 2 + take_primitive_launches();
     unsigned mc32 = 0;
@@ -581,10 +582,11 @@ int nucleus_run(rtr_graph* g)
     int64_t* ltmp = (int64_t*)sc.get(sizeof(int64_t) * scan_temp_elems(mc + 1));
     if (!k1 || !k2 || !rtmp || !list || !lsup || !psup || !head || !hpos || !ub || !ltmp) return failed("units");
     k_nuc_unit_keys<<<gm, kBlock, 0, rs>>>(carries, cpos, m, rb, comp, k1);
-    uint64_t* by_unit = radix_sort_u64(k1, k2, mc, 2 * rb, rtmp, rs);
+    uint64_t* by_unit = nullptr;
+    RTR_TRY(radix_sort_u64(k1, k2, mc, 2 * rb, rtmp, rs, &by_unit));
     k_nuc_unit_list<<<gc, kBlock, 0, rs>>>(by_unit, mc, rb, tc, list, lsup, head);
-    exclusive_scan_i64(lsup, psup, mc, psup + mc, ltmp, rs);
-    exclusive_scan_u32(head, hpos, mc, next + 5, stmp, rs);
+    RTR_TRY(exclusive_scan_i64(lsup, psup, mc, psup + mc, ltmp, rs));
+    RTR_TRY(exclusive_scan_u32(head, hpos, mc, next + 5, stmp, rs));
     k_nuc_unit_begin<<<gc, kBlock, 0, rs>>>(head, hpos, mc, ub);
     unsigned nu32 = 0;
     RTR_CUDA_TRY(cudaGetLastError());
@@ -612,12 +614,15 @@ int nucleus_run(rtr_graph* g)
     pa.next = next;
     if (!o1 || !o2 || !otmp || !pa.stack || !pa.del_edge || !pa.del_seed || !pa.del_level) return failed("peel");
     k_nuc_unit_order<<<grid_for(nu, kBlock), kBlock, 0, rs>>>(ub, nu, mc, o1);
-    pa.order = radix_sort_bits_u64(o1, o2, nu, 32, 64, otmp, rs);
+    uint64_t* by_size = nullptr;
+    RTR_TRY(radix_sort_bits_u64(o1, o2, nu, 32, 64, otmp, rs, &by_size));
+    pa.order = by_size;
     // the largest unit's chain bounds the peel
     k_nuc_peel<<<(int)std::min<int64_t>((nu + 3) / 4, grid_for(1ll << 40, 128, 16)), 128, 0, rs>>>(pa);
     // the deletion order
     k_nuc_seed_keys<<<gc, kBlock, 0, rs>>>(pa.del_seed, mc, m, pb, k1);
-    uint64_t* seq = radix_sort_bits_u64(k1, k2, mc, pb, pb + rb, rtmp, rs);
+    uint64_t* seq = nullptr;
+    RTR_TRY(radix_sort_bits_u64(k1, k2, mc, pb, pb + rb, rtmp, rs, &seq));
     g->launches += 6 + take_primitive_launches();
     unsigned pk[3] = {0, 0, 0};
     RTR_CUDA_TRY(cudaGetLastError());
@@ -634,7 +639,7 @@ int nucleus_run(rtr_graph* g)
     if (!hist || !ord || !dtime) return failed("order");
     RTR_CUDA_TRY(cudaMemsetAsync(hist, 0, sizeof(unsigned) * (max_c + 2), rs));
     k_nuc_level_keys<<<gc, kBlock, 0, rs>>>(seq, mc, pb, pa.del_level, hist);
-    seq = radix_sort_bits_u64(seq, seq == k1 ? k2 : k1, mc, pb, pb + bits_for((uint64_t)max_c), rtmp, rs);
+    RTR_TRY(radix_sort_bits_u64(seq, seq == k1 ? k2 : k1, mc, pb, pb + bits_for((uint64_t)max_c), rtmp, rs, &seq));
     k_nuc_deletions<<<gc, kBlock, 0, rs>>>(seq, mc, pb, pa.del_edge, ord, dtime);
     std::vector<unsigned> per_level((size_t)max_c + 2);
     RTR_CUDA_TRY(cudaMemcpyAsync(per_level.data(), hist, sizeof(unsigned) * (max_c + 2), cudaMemcpyDeviceToHost, rs));
@@ -687,12 +692,12 @@ int nucleus_run(rtr_graph* g)
         k_nuc_join<<<gl, kBlock, 0, rs>>>(la);
         k_nuc_comps<<<gl, kBlock, 0, rs>>>(la);
         k_nuc_roots<<<gl, kBlock, 0, rs>>>(la);
-        exclusive_scan_u32(la.is_start, hpos, la.cnt, next + 6, stmp, rs);
+        RTR_TRY(exclusive_scan_u32(la.is_start, hpos, la.cnt, next + 6, stmp, rs));
         k_nuc_clusters<<<gl, kBlock, 0, rs>>>(la, hpos, ncl, cl);
         RTR_CUDA_TRY(cudaMemsetAsync(d_tot, 0, sizeof(int64_t) * 2, rs));
         if (ncl > 0) {
             k_nuc_children<<<gk, kBlock, 0, rs>>>(la, ncl, cl, brings);
-            exclusive_scan_i64(brings, bat, ncl, d_tot, ltmp, rs);
+            RTR_TRY(exclusive_scan_i64(brings, bat, ncl, d_tot, ltmp, rs));
         }
         unsigned born = 0;
         int64_t brought = 0;
@@ -719,9 +724,10 @@ int nucleus_run(rtr_graph* g)
                                                                                mk + 2 * la.cnt);
             g->launches += 1;
         }
-        const uint64_t* ms = radix_sort_u64(mk, ma, cnt, B + bits_for((uint64_t)born), mt, rs);
+        uint64_t* ms = nullptr;
+        RTR_TRY(radix_sort_u64(mk, ma, cnt, B + bits_for((uint64_t)born), mt, rs, &ms));
         k_nuc_distinct<<<gq, kBlock, 0, rs>>>(ms, cnt, mflag);
-        exclusive_scan_u32(mflag, mpos, cnt, next + 7, mtmp, rs);
+        RTR_TRY(exclusive_scan_u32(mflag, mpos, cnt, next + 7, mtmp, rs));
         unsigned distinct = 0;
         RTR_CUDA_TRY(cudaMemcpyAsync(&distinct, next + 7, sizeof distinct, cudaMemcpyDeviceToHost, rs));
         RTR_CUDA_TRY(cudaStreamSynchronize(rs));

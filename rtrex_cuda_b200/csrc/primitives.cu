@@ -336,9 +336,10 @@ size_t radix_temp_bytes(int64_t n, const SortForms& forms)
     return n >= forms.one_region_from ? std::max(b, RadixPlan(forms.one_region_from - 1, forms).bytes()) : b;
 }
 
-uint64_t* radix_sort_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int nbits, void* temp, cudaStream_t s)
+int radix_sort_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int nbits, void* temp, cudaStream_t s,
+                   uint64_t** sorted)
 {
-    return radix_sort_bits_u64(d_keys, d_alt, n, 0, nbits, temp, s);
+    return radix_sort_bits_u64(d_keys, d_alt, n, 0, nbits, temp, s, sorted);
 }
 
 int64_t take_primitive_launches()
@@ -348,16 +349,19 @@ int64_t take_primitive_launches()
     return k;
 }
 
-uint64_t* radix_sort_bits_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int lo, int hi, void* temp,
-                              cudaStream_t s, const SortForms& forms)
+int radix_sort_bits_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int lo, int hi, void* temp, cudaStream_t s,
+                        uint64_t** sorted, const SortForms& forms)
 {
-    if (n <= 1 || hi <= lo) return d_keys;
+    *sorted = d_keys;
+    if (n <= 1 || hi <= lo) return RTR_OK;
     if (n <= kSortOne) {
         const size_t smem = sizeof(SortOneSmem);
-        cudaFuncSetAttribute(k_sort_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        RTR_CUDA_TRY(cudaFuncSetAttribute(k_sort_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k_sort_one<<<1, 32 * kSortWarps, smem, s>>>(d_keys, d_alt, (int)n, lo, hi);
         t_launches += 1;
-        return d_alt;
+        RTR_CUDA_TRY(cudaGetLastError());
+        *sorted = d_alt;
+        return RTR_OK;
     }
     const RadixPlan plan(n, forms);
     const int digits = (hi - lo + kRadixBits - 1) / kRadixBits;
@@ -365,13 +369,13 @@ uint64_t* radix_sort_bits_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int 
     unsigned* next = (unsigned*)(hist + kMaxDigits * kBins);
     unsigned char* status = (unsigned char*)temp + RadixPlan::kHead;
     const bool own = plan.regions > 1;
-    cudaMemsetAsync(temp, 0, RadixPlan::kHead + (own ? plan.region_bytes() * (size_t)digits : 0), s);
+    RTR_CUDA_TRY(cudaMemsetAsync(temp, 0, RadixPlan::kHead + (own ? plan.region_bytes() * (size_t)digits : 0), s));
     k_radix_hist<<<grid_for(n, kBlock, 8), kBlock, 0, s>>>(d_keys, n, lo, digits, hist);
     uint64_t* src = d_keys;
     uint64_t* dst = d_alt;
     for (int d = 0; d < digits; ++d) {
         unsigned char* st = status + (own ? plan.region_bytes() * (size_t)d : 0);
-        if (!own) cudaMemsetAsync(st, 0, plan.region_bytes(), s);
+        if (!own) RTR_CUDA_TRY(cudaMemsetAsync(st, 0, plan.region_bytes(), s));
         const int shift = lo + d * kRadixBits;
         if (plan.wide)
             k_radix_pass<unsigned long long><<<(unsigned)plan.tiles, kBlock, 0, s>>>(
@@ -382,7 +386,9 @@ uint64_t* radix_sort_bits_u64(uint64_t* d_keys, uint64_t* d_alt, int64_t n, int 
         std::swap(src, dst);
     }
     t_launches += 1 + digits;
-    return src;
+    RTR_CUDA_TRY(cudaGetLastError());
+    *sorted = src;
+    return RTR_OK;
 }
 
 int grid_for(int64_t work, int block, int blocks_per_sm)

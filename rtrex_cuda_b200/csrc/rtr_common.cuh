@@ -86,6 +86,13 @@ __host__ __device__ inline double tri_weight(int64_t a, int64_t b, int64_t c)
         if (e_ != cudaSuccess) return ::rtr::cuda_fail(e_, #expr, __FILE__, __LINE__); \
     } while (0)
 
+// A call that returns an rtr_status.
+#define RTR_TRY(expr)              \
+    do {                           \
+        const int rc_ = (expr);    \
+        if (rc_) return rc_;       \
+    } while (0)
+
 namespace rtr {
 int cuda_fail(cudaError_t e, const char* what, const char* file, int line);
 void set_error(const char* fmt, ...);
