@@ -173,6 +173,7 @@ int copy_i32_as_i64(rtr_graph* g, const int32_t* d, int64_t k, int64_t* h)
         return RTR_ERR_CUDA;
     }
     k_widen32<<<grid_for(k, 256), 256, 0, g->stream>>>(d, w, k);
+    g->launches += 1;
     RTR_CUDA_TRY(cudaMemcpyAsync(h, w, sizeof(int64_t) * k, cudaMemcpyDeviceToHost, g->stream));
     RTR_CUDA_TRY(cudaStreamSynchronize(g->stream));
     return RTR_OK;
@@ -879,6 +880,7 @@ int rtr_get_clusters(const rtr_graph* gc, int64_t* seed, int64_t* nv, int64_t* n
         }
         k_pack_clusters<<<grid_for(words, 256), 256, 0, s>>>(g->cl_off, g->cl_ne, g->cl_cut, g->cl_seed, g->cl_vert, k,
                                                              g->n, d);
+        g->launches += 1;
         RTR_CUDA_TRY(cudaGetLastError());
         RTR_CUDA_TRY(cudaMemcpyAsync(h.get(), d, sizeof(int64_t) * words, cudaMemcpyDeviceToHost, s));
         RTR_CUDA_TRY(cudaStreamSynchronize(s));

@@ -738,6 +738,7 @@ struct SideWait {
 
 int initial_clean(rtr_graph* g, double eps)
 {
+    take_primitive_launches();  // what a call that failed left uncounted is not this one's
     if (g->stage < 2) {
         set_error("clean called before count");
         return RTR_ERR_STATE;

@@ -182,6 +182,7 @@ __global__ void k_cc_offsets(const uint32_t* __restrict__ head, const uint32_t* 
 
 int connected_components(rtr_graph* g)
 {
+    take_primitive_launches();  // what a call that failed left uncounted is not this one's
     if (g->stage < 1) {
         set_error("components requested before the graph was built");
         return RTR_ERR_STATE;

@@ -924,6 +924,7 @@ int launch_bits(rtr_graph* g, const HeavyArgs& ha, const HeavyRuns& runs, const 
 
 int count_triangles(rtr_graph* g)
 {
+    take_primitive_launches();  // what a call that failed left uncounted is not this one's
     if (g->stage < 1) {
         set_error("count called before the graph was built");
         return RTR_ERR_STATE;

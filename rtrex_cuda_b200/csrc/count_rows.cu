@@ -655,7 +655,7 @@ int build_row_sets(rtr_graph* g, Scratch& sc, int min_deg, RowSets* out)
     RTR_TRY(exclusive_scan_i64(flag, num, n + 1, nullptr, tmp, s));
     int64_t nt = 0;
     if (const int rc = read_words(g, &nt, num + n, sizeof(int64_t))) return rc;
-    g->launches += 2;
+    g->launches += 1 + take_primitive_launches();
     if (nt == 0) return RTR_OK;
     int32_t* owner = (int32_t*)sc.get(sizeof(int32_t) * (nt + 1));
     int32_t* tbits = (int32_t*)sc.get(sizeof(int32_t) * (nt + 1));
@@ -678,7 +678,7 @@ int build_row_sets(rtr_graph* g, Scratch& sc, int min_deg, RowSets* out)
     }
     RTR_CUDA_TRY(cudaMemsetAsync(slot, 0xff, sizeof(int32_t) * (total + 1), s));
     k_rs_insert<<<grid_for(1ll << 40, 256, 8), 256, 0, s>>>(owner, nt, g->offsets, g->nbors, toff, tbits, slot);
-    g->launches += 3;
+    g->launches += 2 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     *out = RowSets{tab, toff, tbits, slot};
     return RTR_OK;
@@ -859,7 +859,7 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const PriorityRows&
     RTR_CUDA_TRY(cudaMemcpyAsync(&want, lpos + m2, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     RTR_CUDA_TRY(cudaMemcpyAsync(nb2, d_nbig, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     RTR_CUDA_TRY(cudaStreamSynchronize(s));
-    g->launches += 2;
+    g->launches += 1 + take_primitive_launches();
     const unsigned nbig = nb2[0], nhuge = nb2[1];  // big[0, nhuge) take a block, the rest a warp
     int32_t* big = nullptr;
     if (nbig > 0) {
@@ -896,7 +896,7 @@ int count_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, const PriorityRows&
         }
         k_seg_slots<<<grid_for(1ll << 40, 256, 4), 256, 0, s>>>(g->offsets, lpos, nullptr, big, nhuge, segoff,
                                                                 segslot);
-        g->launches += 3;
+        g->launches += 2 + take_primitive_launches();
     }
     // the lists: all of them when they fit in the free HBM (less 1 GiB), else windows of whole
     // rows; a graph-owned buffer, reused by later counts of the graph

@@ -154,6 +154,7 @@ PinnedRing g_ring;
 int parse_escape_device(rtr_graph* g, Scratch& sc, const char* h_text, FILE* f, int64_t len, const char* what,
                         int64_t* n_out, int64_t* m_out, int64_t** du_out, int64_t** dv_out)
 {
+    take_primitive_launches();  // what a call that failed left uncounted is not this one's
     cudaStream_t s = g->stream;
     char* text = (char*)sc.get((size_t)len + kTile + 16);
     if (!text) {
@@ -228,6 +229,7 @@ int parse_escape_device(rtr_graph* g, Scratch& sc, const char* h_text, FILE* f, 
     }
     k_nl_count<<<(unsigned)tiles, kBlock, 0, s>>>(text, len, tile_cnt);
     RTR_TRY(exclusive_scan_i64(tile_cnt, tile_off, tiles, tile_off + tiles, ltmp, s));
+    g->launches += 1 + take_primitive_launches();
     int64_t nnl = 0;
     RTR_CUDA_TRY(cudaMemcpyAsync(&nnl, tile_off + tiles, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     RTR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -255,7 +257,7 @@ int parse_escape_device(rtr_graph* g, Scratch& sc, const char* h_text, FILE* f, 
         k_lines<<<grid_for(L, kBlock), kBlock, 0, s>>>(text, len, nlpos, nnl, L, is_data, va, vb, first);
         RTR_TRY(exclusive_scan_u32(is_data, rank, L, ndata, utmp, s));
     }
-    g->launches += 6;
+    g->launches += (nnl ? 1 : 0) + (L ? 1 : 0) + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     unsigned long long fl[2];
     uint32_t D = 0;
@@ -299,7 +301,7 @@ int parse_escape_device(rtr_graph* g, Scratch& sc, const char* h_text, FILE* f, 
         return RTR_ERR_CUDA;
     }
     if (m) k_scatter<<<grid_for(L, kBlock), kBlock, 0, s>>>(is_data, rank, va, vb, L, m, du, dv);
-    g->launches += 1;
+    g->launches += m ? 1 : 0;
     RTR_CUDA_TRY(cudaGetLastError());
     *n_out = n;
     *m_out = m;

@@ -376,6 +376,7 @@ __global__ void k_scores(const uint8_t* __restrict__ moved, const uint32_t* __re
 
 int expand_clusters(rtr_graph* g, int64_t threshold)
 {
+    take_primitive_launches();  // what a call that failed left uncounted is not this one's
     if (g->stage < 4) {
         set_error("expand called before extraction");
         return RTR_ERR_STATE;
@@ -435,7 +436,7 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
     RTR_CUDA_TRY(cudaMemsetAsync(d_cnt, 0, sizeof(uint32_t) * 4, s));
     k_singleton_flags<<<gk, kBlock, 0, s>>>(g->cl_off, ncl, flag);
     RTR_TRY(exclusive_scan_u32(flag, fpos, ncl, d_cnt, utmp, s));
-    g->launches += 4;
+    g->launches += 1 + take_primitive_launches();
     uint32_t S32 = 0;
     RTR_CUDA_TRY(cudaMemcpyAsync(&S32, d_cnt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     RTR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -458,7 +459,7 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
         k_singleton_list<<<gk, kBlock, 0, s>>>(flag, fpos, ncl, g->cl_off, g->cl_vert, g->offsets, s_cluster,
                                                s_vertex, vs, s_tab);
         RTR_TRY(exclusive_scan_i64(s_tab, s_toff, S, s_toff + S, ltmp, s));
-        g->launches += 4;
+        g->launches += 1 + take_primitive_launches();
     }
     int64_t tab_total = 0;
     if (S > 0) {
@@ -498,7 +499,7 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
     k_caps<<<gk, kBlock, 0, s>>>(g->cl_off, ncl, inbound, sequential ? 1 : 0, ncap, bcap);
     RTR_TRY(exclusive_scan_i64(ncap, noff, ncl, noff + ncl, ltmp, s));
     RTR_TRY(exclusive_scan_i64(bcap, boff, ncl, boff + ncl, ltmp, s));
-    g->launches += 9;
+    g->launches += (S > 0 ? 2 : 1) + take_primitive_launches();
     int64_t caps[2] = {0, 0};
     RTR_CUDA_TRY(cudaMemcpyAsync(&caps[0], noff + ncl, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     RTR_CUDA_TRY(cudaMemcpyAsync(&caps[1], boff + ncl, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
@@ -523,7 +524,7 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
 
     if (sequential) {
         if (S > 0) k_apply_sequential<<<1, 1, 0, s>>>(st, s_cluster, S, vs, s_best, moved, err);
-        g->launches += 1;
+        g->launches += S > 0 ? 1 : 0;
     } else if (S > 0) {
         uint64_t* mk = (uint64_t*)sc.get(sizeof(uint64_t) * (S + 1));
         uint64_t* malt = (uint64_t*)sc.get(sizeof(uint64_t) * (S + 1));
@@ -568,7 +569,7 @@ int expand_clusters(rtr_graph* g, int64_t threshold)
     k_u8_to_u32<<<gn, kBlock, 0, s>>>(moved, n, m32);
     RTR_TRY(exclusive_scan_u32(m32, mpos, n, d_cnt + 2, utmp, s));
     k_scores<<<gn, kBlock, 0, s>>>(moved, mpos, n, vs, s_score, g->x_scv, g->x_scx);
-    g->launches += 12;
+    g->launches += 6 + take_primitive_launches();
     RTR_CUDA_TRY(cudaGetLastError());
     uint32_t nsc = 0;
     unsigned long long errw = 0;

@@ -1090,6 +1090,7 @@ struct SideJoin {
 
 int extract_clusters(rtr_graph* g)
 {
+    take_primitive_launches();  // what a call that failed left uncounted is not this one's
     if (g->stage < 3) {
         set_error("extract called before the clean");
         return RTR_ERR_STATE;

@@ -324,6 +324,7 @@ int finish_csr(rtr_graph* g, unsigned long long* h_ctr)
 
 int build_csr(rtr_graph* g, const int64_t* d_u, const int64_t* d_v, int64_t m, bool simplify)
 {
+    take_primitive_launches();  // what a call that failed left uncounted is not this one's
     cudaStream_t s = g->stream;
     const int64_t n = g->n;
     if (n <= 0 || n >= (int64_t)INT32_MAX || m < 0 || 2 * m >= (int64_t)INT32_MAX) {
@@ -399,6 +400,7 @@ int build_csr(rtr_graph* g, const int64_t* d_u, const int64_t* d_v, int64_t m, b
 
 int build_csr_from_host_csr(rtr_graph* g, const int64_t* h_offsets, const int64_t* h_nbors)
 {
+    take_primitive_launches();  // what a call that failed left uncounted is not this one's
     cudaStream_t s = g->stream;
     const int64_t n = g->n;
     const int64_t m2 = h_offsets[n];

@@ -479,16 +479,21 @@ __global__ void k_nuc_labels(const int32_t* __restrict__ vert, int64_t cnt, cons
         out[p] = inv[vert[p]];
 }
 
+// The relabelled graph, whose launches are its owner's.
 struct GraphGuard {
+    rtr_graph* owner;
     rtr_graph* g = nullptr;
     ~GraphGuard()
     {
-        if (g) rtr_graph_destroy(g);
+        if (!g) return;
+        owner->launches += g->launches;
+        rtr_graph_destroy(g);
     }
 };
 
 int nucleus_run(rtr_graph* g)
 {
+    take_primitive_launches();  // what a call that failed left uncounted is not this one's
     const int64_t n = g->n, m = g->m;
     cudaStream_t s = g->stream;
     g->nuc_done = false;
@@ -505,7 +510,7 @@ int nucleus_run(rtr_graph* g)
     const int B = bits_for((uint64_t)(n - 1));
     const uint64_t mask = (1ull << B) - 1;
     Scratch isc(g);
-    GraphGuard rel;
+    GraphGuard rel{g};
     int32_t* inv = (int32_t*)isc.get(sizeof(int32_t) * (n + 1));
     {
         Scratch sc(g);
@@ -697,6 +702,7 @@ int nucleus_run(rtr_graph* g)
         RTR_CUDA_TRY(cudaMemsetAsync(d_tot, 0, sizeof(int64_t) * 2, rs));
         if (ncl > 0) {
             k_nuc_children<<<gk, kBlock, 0, rs>>>(la, ncl, cl, brings);
+            g->launches += 1;
             RTR_TRY(exclusive_scan_i64(brings, bat, ncl, d_tot, ltmp, rs));
         }
         unsigned born = 0;
@@ -741,7 +747,7 @@ int nucleus_run(rtr_graph* g)
         }
         k_nuc_members<<<gq, kBlock, 0, rs>>>(ms, cnt, mflag, mpos, next + 7, ncl, B, vn, cl, vert);
         k_nuc_sizes<<<grid_for(born, kBlock), kBlock, 0, rs>>>(ncl, ncl + born, cl);
-        g->launches += 9 + take_primitive_launches();
+        g->launches += 8 + take_primitive_launches();
         RTR_CUDA_TRY(cudaGetLastError());
         ncl += born;
         vn += distinct;
