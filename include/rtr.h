@@ -157,10 +157,11 @@ int rtr_set_count_window(rtr_graph* g, int64_t max_entries);
  * triangle-carrying edges) with at least min_seeds seeds and triangle lists of
  * at most max_mean_list entries on average are replayed by one thread block
  * each, a window of the next pops at a time -- perVertex is folded afterwards in
- * the reference's pop order -- and the other units one warp per unit.  Until it
- * is called the library picks by its own rule, under which every unit that
- * meets the reported 2048 and 8 takes the windows, and others may.  Results are
- * the same bits for every setting.  No counterpart in the reference. */
+ * the reference's pop order -- and the other units one warp per unit.  By default
+ * the library picks by its own rule, under which every unit that meets the
+ * reported 2048 and 8 takes the windows, and others may; setting those two values
+ * returns to it.  Results are the same bits for every setting.  No counterpart in
+ * the reference. */
 int rtr_set_clean_split(rtr_graph* g, int64_t min_seeds, double max_mean_list);
 int rtr_get_clean_split(const rtr_graph* g, int64_t* min_seeds, double* max_mean_list);
 

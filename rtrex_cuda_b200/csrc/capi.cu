@@ -529,7 +529,8 @@ int rtr_set_clean_split(rtr_graph* g, int64_t min_seeds, double max_mean_list)
     }
     g->clean_round_min = min_seeds;
     g->clean_round_list = max_mean_list;
-    g->clean_auto = false;
+    // the values reported by default stand for the library's rule
+    g->clean_auto = min_seeds == kCleanRoundMin && max_mean_list == kCleanRoundList;
     return RTR_OK;
 }
 

@@ -61,6 +61,10 @@ constexpr uint32_t SS_S = 1u << 30;
 constexpr uint32_t SS_N = 2u << 30;
 constexpr uint32_t SS_CODE = 3u << 30;
 
+// What rtr_get_clean_split reports by default.
+constexpr int64_t kCleanRoundMin = 2048;
+constexpr double kCleanRoundList = 8.0;
+
 // Error codes returned through the C ABI are the rtr_status values of rtr.h.
 
 // Device-side error word bits (written by kernels, read by the host).

@@ -104,10 +104,10 @@ struct rtr_graph {
     bool lists = false;  // the last count kept the triangle lists (the clean needs them)
     // clean units with at least this many seeds and triangle lists of at most
     // this mean length take the window replay (one thread block each); the
-    // others one warp per unit.  Until the caller sets them (clean_auto) the
-    // clean picks the window replay by its own rule, a superset of these.
-    int64_t clean_round_min = 2048;
-    double clean_round_list = 8.0;
+    // others one warp per unit.  Until the caller sets other values (clean_auto)
+    // the clean picks the window replay by its own rule, a superset of these.
+    int64_t clean_round_min = rtr::kCleanRoundMin;
+    double clean_round_list = rtr::kCleanRoundList;
     bool clean_auto = true;
     // bounds of the clean's device-side checks, lowered only to test their reports:
     // try_wait rounds of a window's first wait (0: the full limit), unit stack entries (-1: as sized)

@@ -67,3 +67,21 @@ def test_units_replay_without_the_log(name, split):
             peaks.append(_peak(g))
     full, none, less, most = peaks
     assert none == less < full == most  # the log is taken whole or not at all
+
+
+def test_setting_the_reported_split_changes_nothing():
+    """rtr_set_clean_split of what rtr_get_clean_split reports leaves the library's own rule in force."""
+    n, u, v = _graph("wide")
+    seen = []
+    for split in (None, "reported", (2048, 8.5), "back"):
+        with rtr.Graph.from_edges(n, u, v) as g:
+            if split == "back":
+                g.set_clean_split(1, 1e30)
+                g.set_clean_split(2048, 8.0)
+            elif split:
+                g.set_clean_split(*(g.clean_split() if split == "reported" else split))
+            g.count()
+            g.clean(0.3)
+            seen.append((g.clean_split(), _peak(g)))
+    assert seen[0] == seen[1] == seen[3]
+    assert seen[2][1] < seen[0][1]  # that unit's lists are longer, it replays one warp
