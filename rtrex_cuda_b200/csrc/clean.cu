@@ -504,18 +504,21 @@ __device__ __forceinline__ void pop_begin(const StackEntry& c, PopCtx& p)
 }
 
 // The popped edge's own state, loaded by every lane from warp-uniform addresses
-// (broadcast loads, no shuffles): the record's last word (list length |
-// support word), its weight and its endpoints' weights.  Issued in the first
-// round trip.
+// (broadcast loads, no shuffles): its weight, its support word and its endpoints'
+// weights.  Issued in the first round trip.  The list length between weight and
+// support is left out (the stack entry has it): with it the three become one
+// 16-byte load, of words that the pop before may just have stored in 8 and 4
+// bytes, and cascades take a tenth longer (a triangular lattice of 29,601 edges
+// 24.9 against 22.4 ms, a 57,800-edge block model 1.67 against 1.54).
 struct OwnState {
-    unsigned long long w;  // cnt | ss << 32
     double pe, pu, pv;
+    uint32_t ss;
 };
 
 __device__ __forceinline__ void pop_own_loads(const CleanArgs& a, const StackEntry& c, OwnState& o)
 {
     const EdgeRec* r = a.rec + c.e;
-    o.w = *reinterpret_cast<const unsigned long long*>(&r->cnt);
+    o.ss = r->ss;
     o.pe = r->pe;
     o.pu = a.pv[c.first];
     o.pv = a.pv[c.second];
@@ -526,7 +529,7 @@ __device__ __forceinline__ bool pop_own_state(const CleanArgs& a, const StackEnt
                                               uint32_t& s_e, PopCtx& p, unsigned long long* diag)
 {
     const int lane = threadIdx.x & 31;
-    s_e = (uint32_t)(o.w >> 32) & SS_SUP;
+    s_e = o.ss & SS_SUP;
     p.acc_e = o.pe;
     p.acc_u = o.pu;
     p.acc_v = o.pv;
