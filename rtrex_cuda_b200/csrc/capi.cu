@@ -448,8 +448,8 @@ int rtr_graph_destroy(rtr_graph* g)
     for (int k = 0; k < 2 * rtr_graph::kTimers; ++k)
         if (g->kev[k]) cudaEventDestroy(g->kev[k]);
     if (g->own_stream && g->stream) cudaStreamDestroy(g->stream);
-    if (g->side) cudaStreamDestroy(g->side);
-    if (g->side2) cudaStreamDestroy(g->side2);
+    for (cudaStream_t st : {g->side, g->side2, g->side3, g->side4})
+        if (st) cudaStreamDestroy(st);
     delete[] g->batch_vbase;
     delete g;
     return RTR_OK;

@@ -185,9 +185,6 @@ __global__ void k_unit_desc(const uint64_t* __restrict__ keys, int64_t ns, int r
     unit_desc(keys, ns, rbits, head, hpos, ecount, units, cap);
 }
 
-// How a unit is replayed.
-enum UnitClass : uint32_t { UNIT_WIDE = 0, UNIT_NARROW = 1, UNIT_WARP = 2 };
-
 struct UnitRule {
     int64_t min_seeds;  // window replay from this many seeds ...
     double max_list;    // ... and up to this mean triangle-list length
@@ -205,6 +202,11 @@ constexpr int64_t kAutoSeeds = 512;
 // it 8 items packed into 256 threads: 15.4 against 20.4 ms on the co-purchase
 // graph (mean list 3), 150 against 116 ms on the 203,311-edge R-MAT (mean 31).
 constexpr double kNarrowList = 8.0;
+// Units with fewer seeds than this share of their edges also pop one by one where
+// windows commit too little (clean_rounds.cu).  Above it the windows alone were
+// always better on 28 graphs of 0.05 <= eps <= 0.5 (0.79 of one warp's time and less,
+// but 0.99 and 0.94 on two; below it up to 1.65), and watching costs 2 to 3%.
+constexpr double kFewSeeds = 0.6;
 
 // Unit bounds and classes, and the triangles of the window-replayed units.
 __device__ __forceinline__ void unit_class(UnitDesc* units, int64_t nu, int64_t ns, const uint32_t* ecount, const unsigned long long* tsum, UnitRule rule, uint32_t* cls, unsigned long long* ntri, unsigned* ncls)
@@ -215,7 +217,10 @@ __device__ __forceinline__ void unit_class(UnitDesc* units, int64_t nu, int64_t 
         const int64_t r = units[u].root;
         const double lists = (double)tsum[r], edges = (double)ecount[r];
         const bool rounds = end - units[u].seed_begin >= rule.min_seeds && lists <= rule.max_list * edges;
-        const uint32_t c = !rounds ? UNIT_WARP : lists > rule.wide_list * edges ? UNIT_WIDE : UNIT_NARROW;
+        const bool few = (double)(end - units[u].seed_begin) < kFewSeeds * edges;
+        const uint32_t c = !rounds                           ? UNIT_WARP
+                           : lists > rule.wide_list * edges ? (few ? UNIT_WIDE_FEW : UNIT_WIDE)
+                                                            : (few ? UNIT_NARROW_FEW : UNIT_NARROW);
         cls[u] = c;
         if (rounds) {
             atomicAdd(&ncls[c], 1u);
@@ -240,8 +245,8 @@ __device__ __forceinline__ void unit_finish(UnitDesc* units, const int64_t* cap,
         units[u].edges = cap[u];
         units[u].stack_cap = (stack_limit >= 0 && cap[u] > stack_limit) ? stack_limit : cap[u];
         const uint64_t work = (uint64_t)(units[u].seed_end - units[u].seed_begin);
-        const uint64_t w = work < 0x3fffffffull ? work : 0x3fffffffull;
-        order_keys[u] = ((uint64_t)cls[u] << 62) | ((0x3fffffffull - w) << 32) | (uint64_t)u;
+        const uint64_t w = work < 0x1fffffffull ? work : 0x1fffffffull;
+        order_keys[u] = ((uint64_t)cls[u] << 61) | ((0x1fffffffull - w) << 32) | (uint64_t)u;
     }
 }
 
@@ -867,7 +872,8 @@ int initial_clean(rtr_graph* g, double eps)
         if (const int rc = read_words(g, tot, d_tot, sizeof tot)) return rc;
         if (small) nu = (uint32_t)tot[4];
         const unsigned* nc = (const unsigned*)(tot + 2);
-        int64_t nwide = nc[UNIT_WIDE], nnarrow = nc[UNIT_NARROW];
+        int64_t kinds[UNIT_KINDS] = {nc[UNIT_WIDE], nc[UNIT_WIDE_FEW], nc[UNIT_NARROW], nc[UNIT_NARROW_FEW], 0};
+        int64_t nbig = kinds[UNIT_WIDE] + kinds[UNIT_WIDE_FEW] + kinds[UNIT_NARROW] + kinds[UNIT_NARROW_FEW];
         StackEntry* stacks = (StackEntry*)sc.get(sizeof(StackEntry) * (tot[0] + 1));
         if (!stacks) {
             set_error("device allocation failed (clean stacks)");
@@ -877,39 +883,33 @@ int initial_clean(rtr_graph* g, double eps)
         // unit replays one warp each.  Freed after the side streams are waited for.
         std::unique_ptr<Scratch> log(new Scratch(g));
         RoundReplay rr;
-        if (nwide + nnarrow > 0 && !clean_rounds_reserve(g, *log, tot[0], tot[1], &rr)) {
+        if (nbig > 0 && !clean_rounds_reserve(g, *log, tot[0], tot[1], &rr)) {
             log.reset();
-            nwide = nnarrow = 0;
+            nbig = 0;
+            std::fill(kinds, kinds + UNIT_WARP, 0);
         }
-        const int64_t nbig = nwide + nnarrow;
+        kinds[UNIT_WARP] = (int64_t)nu - nbig;
         ktime_begin(g, KT_CLEAN_UNITS);
         // The units order[0, nbig) take the window replay, the others replay one warp
-        // per unit; each of the three kinds that exists takes a stream of its own, the
+        // per unit; each of the kinds that exists takes a stream of its own, the
         // first the graph's (a side stream costs 0.1 ms to make and to destroy, a third
         // of what a graph of 1,000 edges spends in this stage).
-        SideWait side_wait, side_wait2;  // an early return waits for the side streams before scratch is freed
-        const bool has_small = nbig < (int64_t)nu;
-        cudaStream_t wide_st = s, narrow_st = s;
-        if (nwide > 0 && has_small) {
-            if (!g->side) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking));
-            wide_st = side_wait.st = g->side;
+        SideWait side_wait[UNIT_WARP];  // an early return waits for the side streams before scratch is freed
+        cudaStream_t* const spare[UNIT_WARP] = {&g->side, &g->side2, &g->side3, &g->side4};
+        cudaStream_t st[UNIT_KINDS] = {s, s, s, s, s};
+        int used = kinds[UNIT_WARP] > 0 ? 1 : 0;  // the warp replay's is the graph's
+        for (int k = 0; k < UNIT_WARP; ++k) {
+            if (kinds[k] == 0 || used++ == 0) continue;
+            cudaStream_t& side = *spare[used - 2];
+            if (!side) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+            st[k] = side_wait[k].st = side;
         }
-        if (nnarrow > 0 && (nwide > 0 || has_small)) {
-            cudaStream_t& st = wide_st == s ? g->side : g->side2;
-            if (!st) RTR_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-            narrow_st = side_wait2.st = st;
-        }
-        if (nbig > 0) {
-            const int rc = clean_rounds_launch(g, wide_st, narrow_st, rec, seeds, units, order, nwide, nnarrow, stacks,
-                                               &rr);
-            if (rc) return rc;
-        }
-        if (has_small) {
+        if (nbig > 0) RTR_TRY(clean_rounds_launch(g, st, rec, seeds, units, order, kinds, stacks, &rr));
+        if (kinds[UNIT_WARP] > 0) {
             CleanArgs ca{g->tl, rec, g->pv, 1 / (double)n, seeds,
                          g->clean_wait_first > 0 ? (long)g->clean_wait_first : kWaitLimit, g->clean_stack_limit};
             // one warp per unit, persistent over the unit list (largest units first)
-            const int64_t nsmall = (int64_t)nu - nbig;
-            int blocks = (int)std::min<int64_t>((nsmall + kCleanWarps - 1) / kCleanWarps,
+            int blocks = (int)std::min<int64_t>((kinds[UNIT_WARP] + kCleanWarps - 1) / kCleanWarps,
                                                 (int64_t)grid_for(1 << 30, kCleanBlock, 8));
             blocks = std::max(blocks, 1);
             const size_t smem = sizeof(WarpSmem) * kCleanWarps;
@@ -920,11 +920,11 @@ int initial_clean(rtr_graph* g, double eps)
             RTR_CUDA_TRY(cudaGetLastError());
         }
         if (nbig > 0) {
-            for (cudaStream_t st : {wide_st, narrow_st}) {
-                if (st == s) continue;
+            for (int k = 0; k < UNIT_WARP; ++k) {
+                if (st[k] == s) continue;
                 cudaEvent_t joined;
                 RTR_CUDA_TRY(cudaEventCreateWithFlags(&joined, cudaEventDisableTiming));
-                cudaEventRecord(joined, st);
+                cudaEventRecord(joined, st[k]);
                 cudaStreamWaitEvent(s, joined, 0);
                 cudaEventDestroy(joined);
             }

@@ -26,6 +26,11 @@
 //     in the reference's push order (triangle order, (lower,w) before
 //     (higher,w)).
 //
+// Where nearly every pop pushes, a window commits one or two items and costs as
+// much as a full one.  Units of few seeds for their edges, whose pops are mostly
+// pushed ones, therefore take a form (kOne) that watches the pops a round commits
+// and, while they are few, lets the first warp pop items one by one.
+//
 // So the committed pops come in exactly the reference's order.  Each is logged
 // with its number of live triangles, and a byte per list entry says which of
 // them the pop removed.  After the replay the popped edges' own perEdge and the
@@ -99,6 +104,7 @@ struct WinSmem {
     int wlive[NW];
     int cut[2];                                 // where the window ends, by round parity (see below)
     int npush;
+    int2 single;                                // where a run of single pops left the stack's top, and its pops
 };
 
 struct RoundArgs {
@@ -130,6 +136,20 @@ __device__ __forceinline__ void load_state(const EdgeRec* p, EdgeRec& r)
 // A cut value: the window ends with item `last`, which pushes (2 * last) or
 // after which the later items may not be taken (2 * last + 1).
 __device__ __forceinline__ int cut_after(int last) { return 2 * (last > 0 ? last : 0) + 1; }
+
+// Pops one by one (kOne): after kTries rounds that committed fewer than kWorth pops
+// each on average (a round takes ~4,000 cycles, a warp's pop ~2,000), the first
+// warp takes the next kSingleFirst pops, twice as many each time the windows are
+// found wanting again, kSingleMost at most.  Rounds that a list of more than
+// kSingleList entries ends or fills say nothing: such an item is the block's.
+// Windows alone / with single pops / one warp per unit, ms: triangular lattice
+// (186,501 edges, 996 seeds) 216 / 121 / 142, Delaunay mesh (149,970) 138 / 91 / 102,
+// points in the plane of mean degree 20 (98,385, eps 0.5) 66 / 46 / 64, in space of
+// 25 (112,529, eps 0.3) 71 / 50 / 61; where windows do well it costs 2 to 3%.
+constexpr int kTries = 16;
+constexpr int kWorth = 2;
+constexpr int kSingleFirst = 64, kSingleMost = 4096;
+constexpr int kSingleList = 64;
 
 // The first 16 entries of a list that a later round reads: into L1 as soon as an
 // edge is seen to fall (its push is likely the next round's first item), into L2
@@ -208,7 +228,76 @@ __device__ __forceinline__ double fold_lower(const WinSmem<NW, G, W>& S, int slo
     return x;
 }
 
-template <int NW, int G, int W>
+struct SinglePops {
+    int top, done;
+    unsigned long long removed;
+};
+
+// The first warp's pops, at most n, from the ring positions [bot, top).  Out of
+// line: the rounds' own code then stays as it is without it.
+template <int R>
+__device__ __noinline__ SinglePops pop_singles(const TriEntry* tl, EdgeRec* rec, PopLog* plog, uint8_t* live8,
+                                               StackEntry* ring, int top, int bot, int n)
+{
+    constexpr int M = R - 1;
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    int done = 0;
+    unsigned long long removed = 0;
+    while (done < n && top > bot) {
+        const StackEntry c = ring[(top - 1) & M];
+        if (c.cnt > kSingleList || top - 1 - bot + 2 * c.cnt > R) break;
+        __syncwarp();  // c is read before a push takes its place
+        const PairSide ps = pair_side(c);
+        TriEntry t{};
+        if (lane < c.cnt) t = ld_entry(tl + c.t0 + lane);
+        const uint32_t s_e = rec[c.e].ss & SS_SUP;
+        top -= 1;
+        for (int base = 0; base < c.cnt && s_e > 0; base += 32) {
+            const bool valid = base + lane < c.cnt;
+            if (base > 0 && valid) t = ld_entry(tl + c.t0 + base + lane);
+            EdgeRec r1{}, r2{};
+            r1.ss = r2.ss = SS_N;
+            const int32_t rlw = ps.lower_is_a ? t.raz : t.rbz;
+            const int32_t rhw = ps.lower_is_a ? t.rbz : t.raz;
+            if (valid) {
+                r1 = rec[rlw];
+                r2 = rec[rhw];
+            }
+            const uint32_t c1 = r1.ss & SS_CODE, c2 = r2.ss & SS_CODE;
+            bool f1 = false, f2 = false;
+            if (valid && c1 != SS_N && c2 != SS_N) {
+                r1.pe -= t.wgt;
+                r2.pe -= t.wgt;
+                f1 = c1 != SS_S && r1.pe < r1.thr;
+                f2 = c2 != SS_S && r2.pe < r2.thr;
+                r1.ss = ((r1.ss & SS_SUP) - 1u) | (f1 ? SS_S : c1);
+                r2.ss = ((r2.ss & SS_SUP) - 1u) | (f2 ? SS_S : c2);
+                store_state(rec + rlw, r1);
+                store_state(rec + rhw, r2);
+                live8[c.t0 + base + lane] = 1;
+                if (f1) touch_list(tl + r1.t0, (int32_t)r1.cnt);
+                if (f2) touch_list(tl + r2.t0, (int32_t)r2.cnt);
+            }
+            const unsigned b1 = __ballot_sync(kFull, f1), b2 = __ballot_sync(kFull, f2);
+            const int q = top + __popc(b1 & lt) + __popc(b2 & lt);
+            if (f1) ring[q & M] = StackEntry{rlw, ps.lower, t.z, ps.dlow, t.dz, (int32_t)r1.cnt, r1.t0};
+            if (f2)
+                ring[(q + (f1 ? 1 : 0)) & M] = StackEntry{rhw, ps.higher, t.z, ps.dhigh, t.dz, (int32_t)r2.cnt, r2.t0};
+            top += __popc(b1) + __popc(b2);
+        }
+        if (lane == 0) {
+            rec[c.e].ss = SS_N;  // every live triangle of it is gone
+            plog[done] = PopLog{c.e, (int32_t)s_e, c.t0};
+        }
+        removed += s_e;
+        __syncwarp();
+        ++done;
+    }
+    return SinglePops{top, done, removed};
+}
+
+template <int NW, int G, int W, bool kOne>
 __global__ void __launch_bounds__(32 * NW) k_clean_rounds(RoundArgs a)
 {
     using C = Cfg<NW, G, W>;
@@ -238,6 +327,8 @@ __global__ void __launch_bounds__(32 * NW) k_clean_rounds(RoundArgs a)
     unsigned long long removed = 0;  // of this thread's items
     int par = 0;
     bool fail = false;
+    int single = 0, hold = kSingleFirst;  // pops to take one by one; how many the next time
+    int tried = 0, taken = 0;             // window rounds since the last decision, and their pops
     __syncthreads();
     // the oldest `s` ring entries to the global region
     auto spill = [&](int s) {
@@ -298,6 +389,25 @@ __global__ void __launch_bounds__(32 * NW) k_clean_rounds(RoundArgs a)
         if (avail > C::kRing - 2 * T) {  // room for a round's pushes
             spill(avail - (C::kRing - 2 * T) + C::kRing / 4);
             if (fail) break;
+        }
+        // ---- one by one, by the first warp
+        if (kOne && single > 0) {
+            if (wid == 0) {
+                const int64_t left = ud.edges - npop;
+                const SinglePops p = pop_singles<C::kRing>(a.tl, a.rec, plog + npop, a.live8, S.ring, top, bot,
+                                                           left < single ? (int)left : single);
+                if (lane == 0) {
+                    S.single = make_int2(p.top, p.done);
+                    removed += p.removed;
+                }
+            }
+            __syncthreads();
+            const int2 s = S.single;
+            __syncthreads();  // read before the first warp writes it again
+            top = s.x;
+            npop += s.y;
+            single -= s.y;
+            if (s.y > 0) continue;  // else the next item's list is the block's
         }
         // ---- the window: this thread's item and list entry
         int ni = avail < W ? avail : W;
@@ -515,7 +625,7 @@ __global__ void __launch_bounds__(32 * NW) k_clean_rounds(RoundArgs a)
                 removed += left;
             }
         }
-        int npush = 0;
+        int npush = 0, last_cnt = 0;
         if (pushed) {
             // its pushes in the reference's order, from ring position top - (last + 1)
             const bool mine = live && item == last;
@@ -523,8 +633,10 @@ __global__ void __launch_bounds__(32 * NW) k_clean_rounds(RoundArgs a)
             npush = __popc(b1) + __popc(b2);
             int base = 0, w0 = last * G >> 5, w1 = w0;
             if (G == 0) {
-                w0 = __shfl_sync(kFull, i0, last) >> 5;
-                w1 = (__shfl_sync(kFull, i1, last) - 1) >> 5;
+                const int e0 = __shfl_sync(kFull, i0, last), e1 = __shfl_sync(kFull, i1, last);
+                w0 = e0 >> 5;
+                w1 = (e1 - 1) >> 5;
+                last_cnt = e1 - e0;
             }
             if (w0 != w1) {  // the item spans warps
                 if (lane == 0) S.wpush[wid] = npush;
@@ -552,6 +664,19 @@ __global__ void __launch_bounds__(32 * NW) k_clean_rounds(RoundArgs a)
         npop += last + 1;
         top += npush - (last + 1);
         par ^= 1;
+        if (kOne && (pushed ? last_cnt <= kSingleList : last + 1 >= kWorth)) {
+            taken += last + 1;
+            ++tried;
+        }
+        if (kOne && tried == kTries) {
+            if (taken < kWorth * kTries) {
+                single = hold;
+                hold = hold < kSingleMost ? 2 * hold : hold;
+            } else {
+                hold = kSingleFirst;
+            }
+            tried = taken = 0;
+        }
     }
     if (removed) atomicAdd(a.total, (unsigned long long)(-(long long)removed));
 }
@@ -682,12 +807,14 @@ __global__ void __launch_bounds__(128) k_fold_long_runs(const longlong2* __restr
     }
 }
 
-template <int NW, int G, int W>
-int launch_rounds(rtr_graph* g, RoundArgs ra, int64_t units, cudaStream_t st)
+template <int NW, int G, int W, bool kOne>
+int launch_rounds(rtr_graph* g, const RoundArgs& ra, int64_t units, cudaStream_t st)
 {
+    if (units == 0) return RTR_OK;
     const size_t smem = sizeof(WinSmem<NW, G, W>);
-    RTR_CUDA_TRY(cudaFuncSetAttribute(k_clean_rounds<NW, G, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_clean_rounds<NW, G, W><<<(unsigned)units, 32 * NW, smem, st>>>(ra);
+    RTR_CUDA_TRY(cudaFuncSetAttribute(k_clean_rounds<NW, G, W, kOne>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+    k_clean_rounds<NW, G, W, kOne><<<(unsigned)units, 32 * NW, smem, st>>>(ra);
     g->launches += 1;
     RTR_CUDA_TRY(cudaGetLastError());
     return RTR_OK;
@@ -743,35 +870,34 @@ bool clean_rounds_reserve(rtr_graph* g, Scratch& sc, int64_t stack_entries, int6
     return true;
 }
 
-int clean_rounds_launch(rtr_graph* g, cudaStream_t wide_st, cudaStream_t narrow_st, EdgeRec* rec,
-                        const StackEntry* seeds, const UnitDesc* units, const uint64_t* order, int64_t nwide,
-                        int64_t nnarrow, StackEntry* stacks, RoundReplay* rr)
+int clean_rounds_launch(rtr_graph* g, const cudaStream_t* st, EdgeRec* rec, const StackEntry* seeds,
+                        const UnitDesc* units, const uint64_t* order, const int64_t* kinds, StackEntry* stacks,
+                        RoundReplay* rr)
 {
     rr->rec = rec;
     cudaStream_t s = g->stream;
     RTR_CUDA_TRY(cudaMemsetAsync(rr->plog, 0xff, sizeof(PopLog) * ((size_t)rr->pops_cap + 1), s));
     RTR_CUDA_TRY(cudaMemsetAsync(rr->live8, 0, (size_t)g->tl_len + 16, s));
     // the replays on side streams run after everything above
-    if (wide_st != s || narrow_st != s) {
-        cudaEvent_t ready;
-        RTR_CUDA_TRY(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
-        cudaEventRecord(ready, s);
-        for (cudaStream_t st : {wide_st, narrow_st})
-            if (st != s) cudaStreamWaitEvent(st, ready, 0);
-        cudaEventDestroy(ready);
+    cudaEvent_t ready = nullptr;
+    for (int k = 0; k < UNIT_WARP; ++k) {
+        if (kinds[k] == 0 || st[k] == s) continue;
+        if (!ready) {
+            RTR_CUDA_TRY(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+            cudaEventRecord(ready, s);
+        }
+        cudaStreamWaitEvent(st[k], ready, 0);
     }
+    if (ready) cudaEventDestroy(ready);
     RoundArgs ra{g->tl,    rec,       1 / (double)g->n,         seeds,  units,     order, stacks,
                  rr->plog, rr->live8, (unsigned*)(g->ctr + 1), g->ctr, g->ctr + 2};
-    if (nwide > 0) {
-        const int rc = launch_rounds<8, 0, 8>(g, ra, nwide, wide_st);
-        if (rc) return rc;
-    }
-    ra.order = order + nwide;
-    if (nnarrow > 0) {
-        const int rc = launch_rounds<8, 16, 16>(g, ra, nnarrow, narrow_st);
-        if (rc) return rc;
-    }
-    return RTR_OK;
+    RTR_TRY((launch_rounds<8, 0, 8, false>(g, ra, kinds[UNIT_WIDE], st[UNIT_WIDE])));
+    ra.order += kinds[UNIT_WIDE];
+    RTR_TRY((launch_rounds<8, 0, 8, true>(g, ra, kinds[UNIT_WIDE_FEW], st[UNIT_WIDE_FEW])));
+    ra.order += kinds[UNIT_WIDE_FEW];
+    RTR_TRY((launch_rounds<8, 16, 16, false>(g, ra, kinds[UNIT_NARROW], st[UNIT_NARROW])));
+    ra.order += kinds[UNIT_NARROW];
+    return launch_rounds<8, 16, 16, true>(g, ra, kinds[UNIT_NARROW_FEW], st[UNIT_NARROW_FEW]);
 }
 
 int clean_rounds_finish(rtr_graph* g, RoundReplay* rr)

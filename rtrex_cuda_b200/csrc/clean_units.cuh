@@ -69,12 +69,16 @@ struct alignas(16) PopLog {
     int64_t at;  // its triangle list
 };
 
-// Window replay (clean_rounds.cu) of the units order[0, nwide) (long triangle
-// lists) and order[nwide, nwide + nnarrow) (short ones): one thread block per
-// unit on the given streams, concurrently with whatever the caller launches on
-// the graph's stream; the popped edges' perEdge and the per-vertex weights of
-// those units are folded in afterwards, in the reference's order, by
-// clean_rounds_finish on the graph's stream (after both streams are joined).
+// How a unit is replayed, in the schedule's order: in windows of long or of short
+// triangle lists, each for units of many seeds and of few, or by one warp.
+enum UnitClass : uint32_t { UNIT_WIDE = 0, UNIT_WIDE_FEW, UNIT_NARROW, UNIT_NARROW_FEW, UNIT_WARP, UNIT_KINDS };
+
+// Window replay (clean_rounds.cu) of the units at the front of `order`, kinds[k] of
+// each kind in turn: one thread block per unit on the kind's stream,
+// concurrently with whatever the caller launches on the graph's stream; the
+// popped edges' perEdge and the per-vertex weights of those units are folded in
+// afterwards, in the reference's order, by clean_rounds_finish on the graph's
+// stream (after the others are joined).
 struct RoundReplay {
     EdgeRec* rec = nullptr;
     int64_t pops_cap = 0, logs_cap = 0;
@@ -94,9 +98,9 @@ struct RoundReplay {
 // units then replay one warp each, which needs none of it (the lists are kept
 // without regard to the log, so no graph loses its clean to it).
 bool clean_rounds_reserve(rtr_graph* g, Scratch& sc, int64_t stack_entries, int64_t log_entries, RoundReplay* rr);
-int clean_rounds_launch(rtr_graph* g, cudaStream_t wide_st, cudaStream_t narrow_st, EdgeRec* rec,
-                        const StackEntry* seeds, const UnitDesc* units, const uint64_t* order, int64_t nwide,
-                        int64_t nnarrow, StackEntry* stacks, RoundReplay* rr);
+int clean_rounds_launch(rtr_graph* g, const cudaStream_t* st, EdgeRec* rec, const StackEntry* seeds,
+                        const UnitDesc* units, const uint64_t* order, const int64_t* kinds, StackEntry* stacks,
+                        RoundReplay* rr);
 int clean_rounds_finish(rtr_graph* g, RoundReplay* rr);
 
 }  // namespace rtr

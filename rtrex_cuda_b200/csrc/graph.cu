@@ -143,8 +143,8 @@ size_t free_device_bytes(rtr_graph* g, bool trim)
 {
     if (trim) {
         cudaStreamSynchronize(g->stream);
-        if (g->side) cudaStreamSynchronize(g->side);
-        if (g->side2) cudaStreamSynchronize(g->side2);
+        for (cudaStream_t st : {g->side, g->side2, g->side3, g->side4})
+            if (st) cudaStreamSynchronize(st);
         cudaMemPool_t pool;
         if (cudaDeviceGetDefaultMemPool(&pool, g->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
     }

@@ -117,8 +117,8 @@ struct rtr_graph {
     // extraction: components of at least this many vertices are replayed by a
     // whole thread block (the two-hop scan's pairs worked out ahead), the others by a warp
     int64_t extract_big = 512;
-    cudaStream_t side = nullptr;  // second and third streams of the graph (created on first use)
-    cudaStream_t side2 = nullptr;
+    // further streams of the graph (created on first use)
+    cudaStream_t side = nullptr, side2 = nullptr, side3 = nullptr, side4 = nullptr;
 
     // stage timings from CUDA events (ms)
     float ms_build = 0, ms_count = 0, ms_clean = 0, ms_extract = 0, ms_decompose = 0, ms_expand = 0;
