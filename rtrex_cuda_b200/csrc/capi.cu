@@ -191,9 +191,9 @@ const char* rtr_version(void) { return "rtrex-b200 0.1 (sm_100a)"; }
 
 const char* rtr_last_error(void) { return last_error(); }
 
-// Edge arrays -> device CSR; `prepare` (g, scratch, edges) may rewrite the copied edges first.
 }  // extern "C"
 
+// Edge arrays -> device CSR; `prepare` (g, scratch, edges) may rewrite the copied edges first.
 template <typename F>
 static int create_from_edges(const int64_t* src, const int64_t* dst, int64_t m, int64_t n, int device, int flags,
                              rtr_graph** out, F&& prepare)

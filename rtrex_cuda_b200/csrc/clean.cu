@@ -166,7 +166,8 @@ __global__ void k_unit_heads(const uint64_t* __restrict__ keys, int64_t ns, int 
     unit_heads(keys, ns, rbits, head);
 }
 
-__device__ __forceinline__ void unit_desc(const uint64_t* keys, int64_t ns, int rbits, const uint32_t* head, const uint32_t* hpos, const uint32_t* ecount, UnitDesc* units, int64_t* cap)
+__device__ __forceinline__ void unit_desc(const uint64_t* keys, int64_t ns, int rbits, const uint32_t* head,
+                                          const uint32_t* hpos, const uint32_t* ecount, UnitDesc* units, int64_t* cap)
 {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < ns; j += (int64_t)gridDim.x * blockDim.x) {
         if (!head[j]) continue;
@@ -209,7 +210,9 @@ constexpr double kNarrowList = 8.0;
 constexpr double kFewSeeds = 0.6;
 
 // Unit bounds and classes, and the triangles of the window-replayed units.
-__device__ __forceinline__ void unit_class(UnitDesc* units, int64_t nu, int64_t ns, const uint32_t* ecount, const unsigned long long* tsum, UnitRule rule, uint32_t* cls, unsigned long long* ntri, unsigned* ncls)
+__device__ __forceinline__ void unit_class(UnitDesc* units, int64_t nu, int64_t ns, const uint32_t* ecount,
+                                           const unsigned long long* tsum, UnitRule rule, uint32_t* cls,
+                                           unsigned long long* ntri, unsigned* ncls)
 {
     for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < nu; u += (int64_t)gridDim.x * blockDim.x) {
         const int64_t end = (u + 1 < nu) ? units[u + 1].seed_begin : ns;
@@ -238,7 +241,8 @@ __global__ void k_unit_class(UnitDesc* __restrict__ units, int64_t nu, int64_t n
 
 // The schedule: the units' classes in turn, within each the units with the
 // most seeds first.
-__device__ __forceinline__ void unit_finish(UnitDesc* units, const int64_t* cap, const int64_t* capoff, int64_t nu, const uint32_t* cls, uint64_t* order_keys, int64_t stack_limit)
+__device__ __forceinline__ void unit_finish(UnitDesc* units, const int64_t* cap, const int64_t* capoff, int64_t nu,
+                                            const uint32_t* cls, uint64_t* order_keys, int64_t stack_limit)
 {
     for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < nu; u += (int64_t)gridDim.x * blockDim.x) {
         units[u].stack_base = capoff[u];
@@ -258,7 +262,9 @@ __global__ void k_unit_finish(UnitDesc* __restrict__ units, const int64_t* __res
 }
 
 // Seed descriptors, sorted seed j (unit-major, slot order within a unit).
-__device__ __forceinline__ void seed_info(const uint64_t* keys, int64_t ns, uint64_t rmask, const int32_t* fwd, const int32_t* esrc, const int32_t* nb, const int32_t* deg, const EdgeRec* rec, StackEntry* info)
+__device__ __forceinline__ void seed_info(const uint64_t* keys, int64_t ns, uint64_t rmask, const int32_t* fwd,
+                                          const int32_t* esrc, const int32_t* nb, const int32_t* deg,
+                                          const EdgeRec* rec, StackEntry* info)
 {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < ns; j += (int64_t)gridDim.x * blockDim.x) {
         const int32_t k = (int32_t)(keys[j] & rmask);

@@ -60,7 +60,8 @@ __global__ void k_iota_key_deg(const int32_t* __restrict__ deg, int64_t n, int B
     iota_key_deg(deg, n, B, keys);
 }
 
-__device__ __forceinline__ void set_rank(const uint64_t* sorted, int64_t n, uint64_t mask, int32_t* rank, int32_t* by_rank)
+__device__ __forceinline__ void set_rank(const uint64_t* sorted, int64_t n, uint64_t mask, int32_t* rank,
+                                         int32_t* by_rank)
 {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
         const int32_t v = (int32_t)(sorted[j] & mask);
@@ -120,7 +121,8 @@ __global__ void k_comp_keys(const int32_t* __restrict__ root, const int32_t* __r
     comp_keys(root, rank, n, R, keys);
 }
 
-__device__ __forceinline__ void comp_heads(const uint64_t* keys, int64_t n, int R, const int32_t* by_rank, uint32_t* head, int32_t* vlist)
+__device__ __forceinline__ void comp_heads(const uint64_t* keys, int64_t n, int R, const int32_t* by_rank,
+                                           uint32_t* head, int32_t* vlist)
 {
     const uint64_t mask = (1ull << R) - 1;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
@@ -143,7 +145,8 @@ struct CompDesc {
     int64_t scap;
 };
 
-__device__ __forceinline__ void comp_begin(const uint64_t* keys, int64_t n, int R, const uint32_t* head, const uint32_t* hpos, CompDesc* comps)
+__device__ __forceinline__ void comp_begin(const uint64_t* keys, int64_t n, int R, const uint32_t* head,
+                                           const uint32_t* hpos, CompDesc* comps)
 {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x)
         if (head[j]) comps[hpos[j]].vbegin = j;
@@ -155,7 +158,8 @@ __global__ void k_comp_begin(const uint64_t* __restrict__ keys, int64_t n, int R
     comp_begin(keys, n, R, head, hpos, comps);
 }
 
-__device__ __forceinline__ void comp_sizes(CompDesc* comps, int64_t nc, int64_t n, const uint64_t* keys, int R, const uint32_t* acount, int64_t* bneed, int64_t* sneed)
+__device__ __forceinline__ void comp_sizes(CompDesc* comps, int64_t nc, int64_t n, const uint64_t* keys, int R,
+                                           const uint32_t* acount, int64_t* bneed, int64_t* sneed)
 {
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
         const int64_t b = comps[c].vbegin;
@@ -173,7 +177,8 @@ __global__ void k_comp_sizes(CompDesc* __restrict__ comps, int64_t nc, int64_t n
     comp_sizes(comps, nc, n, keys, R, acount, bneed, sneed);
 }
 
-__device__ __forceinline__ void comp_finish(CompDesc* comps, int64_t nc, const int64_t* boff, const int64_t* soff, const int64_t* sneed, uint64_t* order_keys, int64_t big_thr)
+__device__ __forceinline__ void comp_finish(CompDesc* comps, int64_t nc, const int64_t* boff, const int64_t* soff,
+                                            const int64_t* sneed, uint64_t* order_keys, int64_t big_thr)
 {
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
         comps[c].bbase = boff[c];
@@ -196,7 +201,8 @@ __global__ void k_comp_finish(CompDesc* __restrict__ comps, int64_t nc, const in
 }
 
 // Components of at least `thr` vertices (the block kernel's) and the largest vertex count among them.
-__device__ __forceinline__ void big_count(const CompDesc* comps, int64_t nc, int64_t thr, unsigned* nbig, unsigned long long* maxv)
+__device__ __forceinline__ void big_count(const CompDesc* comps, int64_t nc, int64_t thr, unsigned* nbig,
+                                          unsigned long long* maxv)
 {
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x)
         if (comps[c].vcount >= thr) {
@@ -935,7 +941,8 @@ __global__ void __launch_bounds__(kBigBlock) k_extract_big(ExtractArgs a, const 
     }
 }
 
-__device__ __forceinline__ void cluster_keys(const CompDesc* comps, int64_t nc, const int32_t* ncl, const int64_t* cpos, const int32_t* hdr_seed, const int32_t* rank, int B, uint64_t* keys)
+__device__ __forceinline__ void cluster_keys(const CompDesc* comps, int64_t nc, const int32_t* ncl, const int64_t* cpos,
+                                             const int32_t* hdr_seed, const int32_t* rank, int B, uint64_t* keys)
 {
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
         const int64_t vb = comps[c].vbegin;
@@ -951,7 +958,9 @@ __global__ void k_cluster_keys(const CompDesc* __restrict__ comps, int64_t nc, c
     cluster_keys(comps, nc, ncl, cpos, hdr_seed, rank, B, keys);
 }
 
-__device__ __forceinline__ void cluster_gather(const uint64_t* sorted, int64_t ncl, uint64_t mask, const int32_t* hdr_seed, const int32_t* hdr_size, int32_t* cl_seed, int64_t* size64)
+__device__ __forceinline__ void cluster_gather(const uint64_t* sorted, int64_t ncl, uint64_t mask,
+                                               const int32_t* hdr_seed, const int32_t* hdr_size, int32_t* cl_seed,
+                                               int64_t* size64)
 {
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ncl; g += (int64_t)gridDim.x * blockDim.x) {
         const int64_t h = (int64_t)(sorted[g] & mask);
@@ -967,7 +976,9 @@ __global__ void k_cluster_gather(const uint64_t* __restrict__ sorted, int64_t nc
     cluster_gather(sorted, ncl, mask, hdr_seed, hdr_size, cl_seed, size64);
 }
 
-__device__ __forceinline__ void cluster_members(const uint64_t* sorted, int64_t ncl, int64_t n, uint64_t mask, const int64_t* hdr_start, const int64_t* cl_off, const int32_t* out_vert, int32_t* cl_vert, int32_t* cluster_of)
+__device__ __forceinline__ void cluster_members(const uint64_t* sorted, int64_t ncl, int64_t n, uint64_t mask,
+                                                const int64_t* hdr_start, const int64_t* cl_off,
+                                                const int32_t* out_vert, int32_t* cl_vert, int32_t* cluster_of)
 {
     if (cl_off[ncl] != n) return;  // reported by the host
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ncl; g += (int64_t)gridDim.x * blockDim.x) {

@@ -201,7 +201,6 @@ __global__ void __launch_bounds__(kBlock) k_radix_pass(const uint64_t* __restric
     constexpr S kMask = ((S)1 << kShift) - 1;
     __shared__ uint64_t s_key[kPassTile];
     __shared__ uint32_t s_cnt[kWarps][kBins + 1];
-    __shared__ uint32_t s_excl[kBins];
     __shared__ int64_t s_base[kBins];
     __shared__ uint32_t s_warp[kBins / 32];
     __shared__ unsigned long long s_warp64[kBins / 32];
@@ -236,7 +235,6 @@ __global__ void __launch_bounds__(kBlock) k_radix_pass(const uint64_t* __restric
     volatile S* st = status + t;
     if (tile > 0) st[tile * kBins] = ((S)1 << kShift) | (S)sum;
     const uint32_t excl = bins_exclusive_scan(sum, s_warp);
-    s_excl[t] = excl;
     // where the digit's keys begin
     unsigned long long h = hist[t], hx = h;
 #pragma unroll
