@@ -779,15 +779,17 @@ int fold_priority_rows(rtr_graph* g, Scratch& sc, const RowSets& rs, PriorityRow
     RTR_CUDA_TRY(cudaMemcpyAsync(&entries, lpos + S, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     if (const int rc = read_words(g, &nseg, segoff + k, sizeof(int64_t))) return rc;
     g->launches += 2 + take_primitive_launches();
-    // a graph-owned buffer (reused by later counts) of at most an eighth of the free memory, beside
-    // which any other row's list (a term is an edge: at most m) and its count's scratch still fit
+    // a graph-owned buffer of at most an eighth of the free memory, beside which any other row's list
+    // (a term is an edge: at most m) and its count's scratch still fit; later counts reuse it, with
+    // the other rows' lists that the graph then holds too
     const int64_t bytes = (int64_t)sizeof(int32_t) * (entries + 1);
-    const int64_t avail = (int64_t)device_avail_bytes(g) + g->rows_ahead_cap;
     const int64_t rest = kListsMargin + (int64_t)sizeof(int32_t) * (g->m + 1) + 64 * g->n + (16ll << 20);
-    if ((g->rows_ahead_cap < bytes && bytes > avail / 8) ||
-        std::max(bytes, g->rows_ahead_cap) + rest > avail + g->rows_lists_cap) {
-        release_owned(g, &g->rows_ahead, &g->rows_ahead_cap);
-        return RTR_OK;
+    if (g->rows_ahead_cap < bytes) {
+        const int64_t avail = (int64_t)device_avail_bytes(g) + g->rows_ahead_cap;
+        if (bytes > avail / 8 || bytes + rest > avail + g->rows_lists_cap) {
+            release_owned(g, &g->rows_ahead, &g->rows_ahead_cap);
+            return RTR_OK;
+        }
     }
     int32_t* lists = (int32_t*)grow_owned(g, &g->rows_ahead, &g->rows_ahead_cap, bytes);
     int32_t* segslot = lists ? (int32_t*)sc.get(sizeof(int32_t) * (size_t)(nseg + 1)) : nullptr;

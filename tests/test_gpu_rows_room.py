@@ -34,10 +34,14 @@ def _count(edges, device, window):
         return g.weights()[1], g.count_windows()[0]
 
 
-def test_what_fits_without_rows_ahead_fits_with_them():
+def _edges():
     n, u, v = _hubs(CASES["40"], 5)
     a, b = np.meshgrid(np.arange(512), np.arange(1024))
-    edges = n + 1536, np.concatenate([u, n + a.ravel()]), np.concatenate([v, n + 512 + b.ravel()])
+    return n + 1536, np.concatenate([u, n + a.ravel()]), np.concatenate([v, n + 512 + b.ravel()])
+
+
+def test_what_fits_without_rows_ahead_fits_with_them():
+    edges = _edges()
     with rtr.Graph.from_edges(*edges) as g:
         built, _ = _memory(g)
         g.set_count_mode(2)
@@ -55,3 +59,17 @@ def test_what_fits_without_rows_ahead_fits_with_them():
             assert (helpers.bits(ahead[0]) == helpers.bits(want)).all()
         fitted.append(alone is not None)
     assert not fitted[0] and fitted[-1]  # the sizes span the line
+
+
+def test_held_buffers_do_for_later_counts():
+    """A graph that was counted with rows ahead is counted again when nothing more is available."""
+    with rtr.Graph.from_edges(*_edges()) as g:
+        g.set_count_mode(2)
+        g.count()
+        want = g.weights()[1]
+        held, _ = _memory(g)
+        for device in (0, 1, 1, 0):
+            g.set_device_limits(graph_bytes=device)
+            g.count()
+            assert (helpers.bits(g.weights()[1]) == helpers.bits(want)).all()
+            assert _memory(g)[0] == held
