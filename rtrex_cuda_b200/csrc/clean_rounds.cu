@@ -43,11 +43,11 @@
 // table, fold, commit; 4 barriers) of ~4,000 cycles, of which the memory is a
 // fifth and the rest instruction latency, and every item that pushes ends a
 // round.  On the 926,000-edge co-purchase graph (B200, eps 0.3) the giant
-// unit's 41,000 pops take 7,100 rounds, 14.4 ms; reserving cells and letting
-// only conflict-free items commit (with the sequence as a linked list, ranked
-// afterwards) took 25.0 ms, one warp per unit 38.5 ms.  On the 203,311-edge R-MAT
-// graph (mean list 31) 162,000 pops take 39,600 rounds, 111 ms against 235 ms one
-// warp per unit.  Measured and slower: a warp replaying single items from lists
+// unit's 41,800 pops take 7,340 rounds (5,440 ended by a push), 14.4 ms; reserving
+// cells and letting only conflict-free items commit (with the sequence as a linked
+// list, ranked afterwards) took 25.0 ms, one warp per unit 38.5 ms.  On the
+// 203,311-edge R-MAT graph (mean list 31) 162,000 pops take 40,700 rounds (25,700
+// ended by a push), 111 ms against 235 ms one warp per unit.  Measured and slower: a warp replaying single items from lists
 // brought into L1 by helper warps (19.7 / 203 ms), one thread per edge folding all
 // items' subtractions (18.9 / 148 ms), one warp walking the window's items in
 // shared memory after a parallel load (27.5 / 139 ms).
