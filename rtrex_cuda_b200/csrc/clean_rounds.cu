@@ -47,10 +47,11 @@
 // cells and letting only conflict-free items commit (with the sequence as a linked
 // list, ranked afterwards) took 25.0 ms, one warp per unit 38.5 ms.  On the
 // 203,311-edge R-MAT graph (mean list 31) 162,000 pops take 40,700 rounds (25,700
-// ended by a push), 111 ms against 235 ms one warp per unit.  Measured and slower: a warp replaying single items from lists
-// brought into L1 by helper warps (19.7 / 203 ms), one thread per edge folding all
-// items' subtractions (18.9 / 148 ms), one warp walking the window's items in
-// shared memory after a parallel load (27.5 / 139 ms).
+// ended by a push), 111 ms against 235 ms one warp per unit.  Measured and slower:
+// a warp replaying single items from lists brought into L1 by helper warps (19.7 /
+// 203 ms), one thread per edge folding all items' subtractions (18.9 / 148 ms), one
+// warp walking the window's items in shared memory after a parallel load (27.5 /
+// 139 ms).
 //
 // An item whose list does not fit is popped alone, its entries taken one block
 // width at a time.
